@@ -20,6 +20,7 @@
 #include <cuda_runtime.h>
 #include <cstdlib>
 #include <cstring>
+#include <numeric>
 #include "afc_async.cuh"
 #include "afc_engine.cuh"
 #include "afc_internal.h"
@@ -1185,6 +1186,13 @@ bool tma_plan(const StageList& sl, int ld, long long lanes, const LaneMap& im, c
     while (lanes_pref <= 0 && tp.L > Lmin &&
            3 * (size_t)tp.L * (size_t)std::max<long long>(ld, rows) * csz + 64 > 110 * 1024)
       tp.L /= 2;
+    // every box starts on 128 bytes of shared memory: its rows come in
+    // multiples of 128 bytes (rows of 64 bytes: an even count, ...; at most 256
+    // rows either way, and the last box still starts inside the axis)
+    if (tp.nbx > 1) {
+      const int m = 128 / std::gcd(128, (int)(tp.L * csz));
+      tp.bn = (tp.bn + m - 1) / m * m;
+    }
     tp.kb = (es + tp.L - 1) / tp.L;
   }
   tp.ld = ld;
