@@ -297,9 +297,18 @@ static bool gpu_radices_uncached(int64_t n, std::vector<int>& rad) {
   return (int)rad.size() <= kMaxStages;
 }
 
+static int env_int(const char* name, int dflt) {
+  const char* v = getenv(name);
+  return v && *v ? atoi(v) : dflt;
+}
+
 struct LenPlan {
   StageList sl{};
   void* tw = nullptr;
+  // stage twiddles of the compile-time engine (powers of two 64 .. 4096;
+  // AFC_FX=0 at plan creation keeps the general engine), behind tw's entries in
+  // the same allocation; null when the length has no compile-time build
+  void* fx_tw = nullptr;
   int P = 0, ld = 0;
   int64_t n = 0;
 };
@@ -360,8 +369,17 @@ static afc_status build_lenplan(int64_t n, bool dbl, LenPlan& lp, cudaStream_t s
     if (Ns > 1) off += Ns * (rad[s] - 1);
     Ns *= rad[s];
   }
-  AFC_CUDA(dev_alloc(&lp.tw, (size_t)std::max(off, 1) * csz), "twiddle table");
+  StageList fx{};
+  const bool has_fx = env_int("AFC_FX", 1) != 0 && fx_stage_list(n, fx);
+  const size_t fx_off = ((size_t)std::max(off, 1) * csz + 255) / 256 * 256;
+  size_t fx_cnt = 0;  // entries of the last stage end the table
+  if (has_fx) fx_cnt = (size_t)fx.st[fx.nst - 1].twoff + (size_t)(fx.st[fx.nst - 1].R - 1) * fx.st[fx.nst - 1].Ns;
+  AFC_CUDA(dev_alloc(&lp.tw, fx_off + fx_cnt * csz), "twiddle table");
   if (off > 0) AFC_CUDA(gen_stage_twiddles_dev(lp.tw, lp.sl, dbl, st), "twiddle generation");
+  if (has_fx) {
+    lp.fx_tw = static_cast<char*>(lp.tw) + fx_off;
+    AFC_CUDA(gen_stage_twiddles_dev(lp.fx_tw, fx, dbl, st), "twiddle generation");
+  }
   return AFC_OK;
 }
 
@@ -373,6 +391,8 @@ struct AxisPlan {
   int64_t N1 = 0, N2 = 0, twB = 1;
   void* tw_hi = nullptr;
   void* tw_lo = nullptr;
+  void* fx_a = nullptr;              // FOURSTEP of compile-time lengths: step twiddle factors (fx_b inside fx_a's
+  void* fx_b = nullptr;              // allocation)
   int64_t M = 0;                     // convolution length
   bool conv_smem = true;
   void* chirp = nullptr;
@@ -385,7 +405,7 @@ struct AxisPlan {
   std::unique_ptr<AxisPlan> sub;     // four-step plan of length M (large Bluestein)
   int tuned_P = 0, tuned_L = 0;      // autotuned tile shape (batch plans)
   ~AxisPlan() {
-    void* ptrs[] = {lp.tw, lp1.tw, lp2.tw, tw_hi, tw_lo, chirp, spec_f, spec_i, spec_rf, spec_ri, gather, scatter};
+    void* ptrs[] = {lp.tw, lp1.tw, lp2.tw, tw_hi, tw_lo, fx_a, chirp, spec_f, spec_i, spec_rf, spec_ri, gather, scatter};
     for (void* p : ptrs)
       if (p) cudaFree(p);
   }
@@ -407,11 +427,6 @@ static unsigned* device_err_word() {
   cudaMemset(p, 0, sizeof(unsigned));
   g_err_words[dev] = p;
   return p;
-}
-
-static int env_int(const char* name, int dflt) {
-  const char* v = getenv(name);
-  return v && *v ? atoi(v) : dflt;
 }
 
 static afc_status build_fourstep(int64_t n, bool dbl, AxisPlan& ap, cudaStream_t st) {
@@ -442,6 +457,12 @@ static afc_status build_fourstep(int64_t n, bool dbl, AxisPlan& ap, cudaStream_t
   AFC_CUDA(dev_alloc(&ap.tw_hi, (size_t)nhi * csz), "four-step twiddles");
   AFC_CUDA(gen_roots_dev(ap.tw_lo, B, 1, n, dbl, st), "four-step twiddles");
   AFC_CUDA(gen_roots_dev(ap.tw_hi, nhi, B, n, dbl, st), "four-step twiddles");
+  if (ap.lp1.fx_tw) {
+    const size_t na = (size_t)(ap.N1 / 16) * ap.N2, nb = (size_t)16 * ap.N2;
+    AFC_CUDA(dev_alloc(&ap.fx_a, (na + nb) * csz), "step twiddles");
+    ap.fx_b = static_cast<char*>(ap.fx_a) + na * csz;
+    AFC_CUDA(gen_fx_step_dev(ap.fx_a, ap.fx_b, ap.N1, ap.N2, dbl, st), "step twiddles");
+  }
   return AFC_OK;
 }
 
@@ -551,7 +572,28 @@ static void record(LaunchDesc d, int kind, bool inv) {
   tl_rec->launches.push_back(RecLaunch{d, kind, inv});
 }
 
+// Puts a descriptor on the compile-time engine when its length and operators
+// have a build; the descriptor is unchanged otherwise.  The engine does its lane
+// arithmetic in 32 bits.
+static bool fx_take(LaunchDesc& d, const LenPlan& lp, int form, int mode, bool dbl) {
+  const long long lim = 1ll << 31;
+  if (!lp.fx_tw || tl_rec || d.lanes <= 0 || d.lanes >= lim - 4096) return false;
+  if (d.im.d1 >= lim || d.im.d2 >= lim || d.om.d1 >= lim || d.om.d2 >= lim) return false;
+  if (d.col_div >= lim || d.col_mod >= lim || d.nlen >= lim || d.nlen_out >= lim || d.jmul * lp.n >= 2 * lim)
+    return false;
+  if (form != FX_COLS && d.im.es != 1) return false;
+  if (form == FX_ROWS && d.om.es != 1) return false;
+  LaunchDesc f = d;
+  f.fx_tw = lp.fx_tw;
+  f.fx_form = form;
+  f.fx_mode = mode;
+  if (!(dbl ? fx_ready_f64(f) : fx_ready_f32(f))) return false;
+  d = f;
+  return true;
+}
+
 static cudaError_t do_lanes(const LaunchDesc& d, bool dbl, bool inv, cudaStream_t st) {
+  if (d.fx_form >= 0) return dbl ? launch_fx_f64(d, st) : launch_fx_f32(d, st);
   if (tl_rec) {
     record(d, 0, inv);
     return cudaSuccess;
@@ -559,6 +601,7 @@ static cudaError_t do_lanes(const LaunchDesc& d, bool dbl, bool inv, cudaStream_
   return launch_lanes(d, dbl, inv, st);
 }
 static cudaError_t do_conv(const LaunchDesc& d, bool dbl, bool inv, cudaStream_t st) {
+  if (d.fx_form >= 0) return dbl ? launch_fx_f64(d, st) : launch_fx_f32(d, st);
   if (tl_rec) {
     record(d, 1, inv);
     return cudaSuccess;
@@ -594,6 +637,13 @@ static cudaError_t exec_fourstep(const AxisPlan& ap, bool dbl, bool inv, const A
   a.stage_in = a.im.es != 1 || !plain_in(a.in_op);
   a.stage_out = true;
   a.L = choose_L(ap.lp1, a.lanes, a.stage_in, a.stage_out, csz);
+  if (ap.fx_a) {
+    LaunchDesc f = a;
+    f.out_op = OUT_STEP;
+    f.fx_a = ap.fx_a;
+    f.fx_b = ap.fx_b;
+    if (fx_take(f, ap.lp1, FX_COLS, inv ? FX_INV : FX_FWD, dbl)) a = f;
+  }
   cudaError_t e = do_lanes(a, dbl, inv, st);
   if (e != cudaSuccess) return e;
   LaunchDesc b;
@@ -617,6 +667,7 @@ static cudaError_t exec_fourstep(const AxisPlan& ap, bool dbl, bool inv, const A
   b.stage_out = b.om.es != 1 || !plain_out(b.out_op);
   if (ap.lp2.sl.nst <= 1) b.stage_out = true;
   b.L = choose_L(ap.lp2, b.lanes, b.stage_in, b.stage_out, csz);
+  fx_take(b, ap.lp2, FX_ROWS_T, inv ? FX_INV : FX_FWD, dbl);
   return do_lanes(b, dbl, inv, st);
 }
 
@@ -625,8 +676,16 @@ static cudaError_t exec_fourstep(const AxisPlan& ap, bool dbl, bool inv, const A
 // call as exec_axis makes, so the pass then takes exactly that path.
 static long long mirror_cols(const AxisPlan& ap, bool dbl, const AxisIO& io) {
   static const int tma_on = env_int("AFC_TMA", 1), tma_lanes = env_int("AFC_TMA_LANES", 0);
-  if (!io.mirror || ap.algo != ALGO_SMEM || tl_rec || !tma_on || io.lanes <= 0) return 0;
+  if (!io.mirror || ap.algo != ALGO_SMEM || tl_rec || io.lanes <= 0) return 0;
   if (io.in_op != IN_C || io.out_op != OUT_C) return 0;
+  const long long es = io.im.es;
+  if (ap.lp.fx_tw && io.im.d2 == es && io.im.s0 == ap.n * es && io.im.s2 == 1 && io.im.d1 == 1 && !io.im.off &&
+      io.lanes % es == 0 && io.lanes < (1ll << 31) - 4096) {
+    const int L = fx_col_lanes(ap.n, dbl);
+    const long long H = L ? (es / 2 / L + 1) * L : 0;
+    if (L) return H < es ? H : 0;
+  }
+  if (!tma_on) return 0;
   unsigned* err = device_err_word();
   TmaPlan tp;
   if (!err || !tma_plan(ap.lp.sl, ap.lp.ld, io.lanes, io.im, io.om, io.in, io.out, dbl, tma_lanes, tp, false, false,
@@ -655,6 +714,31 @@ static cudaError_t exec_axis(const AxisPlan& ap, bool dbl, bool inv, const AxisI
       d.pair_w = io.pair_w;
       const bool rin = io.in_op == IN_R && io.out_op == OUT_C, rout = io.in_op == IN_C && io.out_op == OUT_RE;
       static const int tma_on = env_int("AFC_TMA", 1), tma_lanes = env_int("AFC_TMA_LANES", 0);
+      // Powers of two 64 .. 4096 (strided: 64 .. 1024) run on the compile-time
+      // engine, the rest on the TMA kernel.  Measured on B200, 2^24 points per
+      // pass: contiguous complex64 64 / 512 / 1024 / 4096 points 77 / 98 / 96 /
+      // 69 us on the TMA kernel against 51 / 45 / 47 / 53 us, complex128 205 /
+      // 147 / 144 / 152 against 83 / 83 / 89 / 111 us (6.2 TB/s); columns of
+      // 1024 and 256 points complex64 119 and 52 against 81 and 49 us,
+      // complex128 165 and 98 against 126 and 87 us.  The TMA tile spends a
+      // barrier and a shared-memory round trip on each side of the stages and
+      // keeps one tile per CTA in flight; here a dozen CTAs per SM load, compute
+      // and store independently.
+      if (!tl_rec && ap.lp.fx_tw) {
+        LaunchDesc f = d;
+        if (io.im.es == 1 && io.om.es == 1) {
+          f.store_cols = io.out_op == OUT_TRUNC ? (int)io.nlen : (int)io.store_cols;
+          if (fx_take(f, ap.lp, FX_ROWS, inv ? FX_INV : FX_FWD, dbl)) return do_lanes(f, dbl, inv, st);
+        } else if (io.im.es != 1) {
+          const long long H = io.need_mirror ? mirror_cols(ap, dbl, io) : 0;
+          if (H > 0) {  // lanes 0 .. H - 1 of each outer index, the rest mirrored
+            f.im.d2 = f.om.d2 = H;
+            f.lanes = io.lanes / io.im.es * H;
+            f.hm_cmax = (int)(io.im.es - H);
+          }
+          if (fx_take(f, ap.lp, FX_COLS, inv ? FX_INV : FX_FWD, dbl)) return do_lanes(f, dbl, inv, st);
+        }
+      }
       if (!tl_rec && ((io.in_op == IN_C && io.out_op == OUT_C) || rin || rout) && tma_on) {
         TmaPlan tp;
         unsigned* err = device_err_word();
@@ -718,6 +802,7 @@ static cudaError_t exec_axis(const AxisPlan& ap, bool dbl, bool inv, const AxisI
         d.gather = ap.gather;
         d.scatter = ap.scatter;
         d.L = choose_L(ap.lp, io.lanes, true, true, csz, 2 * csz, 2);
+        if (!rader) fx_take(d, ap.lp, FX_ROWS, FX_CONV, dbl);
         return do_conv(d, dbl, inv, st);
       }
       // Bluestein with a four-step convolution of length M = N1 x N2, three
@@ -758,6 +843,55 @@ static cudaError_t exec_axis(const AxisPlan& ap, bool dbl, bool inv, const AxisI
       a.stage_in = true;
       a.stage_out = true;
       a.L = choose_L(mp.lp1, a.lanes, a.stage_in, a.stage_out, csz);
+      // compile-time lengths: both step twiddles sit in the column passes
+      // (pass 1's store, the conjugate on pass 3's load), so the row pass is a
+      // plain convolution tile.  The three passes change engine together.
+      const bool fx_out = io.out_op == OUT_C || io.out_op == OUT_RE;
+      if (mp.fx_a && fx_out) {
+        LaunchDesc fa = a;
+        fa.out_op = OUT_STEP;
+        fa.fx_a = mp.fx_a;
+        fa.fx_b = mp.fx_b;
+        LaunchDesc fb;
+        fill_common(fb, mp.lp2);
+        fb.lanes = io.lanes * N1;
+        fb.im = LaneMap{N1, d2, d2 * M, N2, M, 1, nullptr};
+        fb.om = fb.im;
+        fb.in = w1;
+        fb.out = w2;
+        fb.in_op = IN_C;
+        fb.out_op = OUT_C;
+        fb.spec = inv ? ap.spec_ri : ap.spec_rf;
+        fb.spec_ld = N2;
+        fb.col_div = d2;
+        fb.col_mod = N1;
+        LaunchDesc fc;
+        fill_common(fc, mp.lp1);
+        fc.lanes = io.lanes * N2;
+        fc.im = LaneMap{N2, d2, d2 * M, 1, M, N2, nullptr};
+        fc.om = io.om.off ? LaneMap{1, N2, 0, 0, io.om.es, N2 * io.om.es, io.om.off}
+                          : LaneMap{N2, io.om.d2, io.om.s0, io.om.es, io.om.s2, N2 * io.om.es, nullptr};
+        fc.in = w2;
+        fc.out = io.out;
+        fc.in_op = IN_STEP;
+        fc.fx_a = mp.fx_a;
+        fc.fx_b = mp.fx_b;
+        fc.out_op = real_out ? OUT_CHIRP_RE : OUT_CHIRP;
+        fc.scale = io.scale;
+        fc.jmul = N2;
+        fc.col_div = d2;
+        fc.col_mod = N2;
+        fc.nlen = ap.n;
+        fc.chirp = ap.chirp;
+        fc.chirp_conj = inv ? 1 : 0;
+        if (fx_take(fa, mp.lp1, FX_COLS, FX_FWD, dbl) && fx_take(fb, mp.lp2, FX_ROWS, FX_CONV, dbl) &&
+            fx_take(fc, mp.lp1, FX_COLS, FX_INV, dbl)) {
+          cudaError_t fe = do_lanes(fa, dbl, false, st);
+          if (fe == cudaSuccess) fe = do_conv(fb, dbl, false, st);
+          if (fe == cudaSuccess) fe = do_lanes(fc, dbl, true, st);
+          return fe;
+        }
+      }
       cudaError_t e = do_lanes(a, dbl, false, st);
       if (e != cudaSuccess) return e;
       LaunchDesc b;
@@ -2097,7 +2231,8 @@ afc_status afc_stft_forward(afc_plan plan, const void* signal, int64_t signal_le
   d.stage_in = true;
   d.stage_out = ap.lp.sl.nst <= 1;
   d.L = choose_L(ap.lp, d.lanes, d.stage_in, d.stage_out, csz);
-  cudaError_t e = launch_lanes(d, plan->dbl, false, static_cast<cudaStream_t>(stream));
+  fx_take(d, ap.lp, FX_ROWS, FX_FWD, plan->dbl);
+  cudaError_t e = do_lanes(d, plan->dbl, false, static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return cuda_fail(e, "stft forward");
   return AFC_OK;
 }
@@ -2322,6 +2457,7 @@ afc_status afc_czt_execute(afc_czt_plan plan, const void* in, void* out, int64_t
   d.spec = plan->spec;
   d.scale = 1.0;
   d.L = choose_L(plan->lp, batch, true, true, csz, 2 * csz + 3 * sizeof(long long), 2);
+  fx_take(d, plan->lp, FX_ROWS, FX_CONV, plan->dbl);
   cudaError_t e = do_conv(d, plan->dbl, false, static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return cuda_fail(e, "czt execute");
   return AFC_OK;
@@ -2402,6 +2538,7 @@ afc_status afc_hilbert_analytic(afc_hilbert_plan plan, const void* signal, void*
   d.spec = plan->mask;
   d.scale = 1.0;
   d.L = choose_L(plan->lp, batch, true, true, csz, 2 * csz + 3 * sizeof(long long), 2);
+  fx_take(d, plan->lp, FX_ROWS, FX_CONV, plan->dbl);
   cudaError_t e = do_conv(d, plan->dbl, false, st);
   if (e != cudaSuccess) return cuda_fail(e, "analytic signal");
   return AFC_OK;

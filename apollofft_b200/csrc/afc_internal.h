@@ -8,11 +8,23 @@
 
 namespace afc {
 
-enum InOpKind { IN_C = 0, IN_R = 1, IN_HERM = 2, IN_CHIRP = 3, IN_CHIRP_R = 4, IN_GATHER = 5, IN_GATHER_R = 6, IN_FRAME = 7 };
+enum InOpKind {
+  IN_C = 0, IN_R = 1, IN_HERM = 2, IN_CHIRP = 3, IN_CHIRP_R = 4, IN_GATHER = 5, IN_GATHER_R = 6, IN_FRAME = 7,
+  IN_STEP = 8  // compile-time engine: times the conjugate step twiddle
+};
 enum OutOpKind {
   OUT_C = 0, OUT_RE = 1, OUT_TRUNC = 2, OUT_TW = 3, OUT_MUL = 4, OUT_CHIRP = 5, OUT_CHIRP_RE = 6,
-  OUT_SCATTER = 7, OUT_SCATTER_RE = 8
+  OUT_SCATTER = 7, OUT_SCATTER_RE = 8,
+  OUT_STEP = 9  // compile-time engine: times the step twiddle (conj if tw_conj)
 };
+
+// Tile forms and modes of the compile-time power-of-two engine (afc_fx.cuh).
+enum FxForm {
+  FX_ROWS = 0,    // lane-major load and store (contiguous lanes)
+  FX_COLS = 1,    // lane-minor load and store (strided lanes, rows of L elements)
+  FX_ROWS_T = 2,  // lane-major load, lane-minor store (rows stored as columns)
+};
+enum FxMode { FX_FWD = 0, FX_INV = 1, FX_CONV = 2 };
 
 // Everything one launch of the lanes / conv kernels needs (type-erased).
 struct LaunchDesc {
@@ -45,6 +57,15 @@ struct LaunchDesc {
   long long nlen_out = 0;          // OUT_CHIRP: outputs kept (j < nlen_out) when > 0, else nlen
   const void* window = nullptr;  // IN_FRAME: analysis window (real, frame length)
   long long frame_off = 0;       // IN_FRAME: frames start at lane base - frame_off
+  // compile-time power-of-two engine (afc_fx.cuh): its stage twiddles, the two
+  // factors of the step twiddle W_M^{col i} = a[t cm + col] b[q cm + col]
+  // (i = t + P q, cm = col_mod columns), the tile form and mode (-1: general engine)
+  const void* fx_tw = nullptr;
+  const void* fx_a = nullptr;
+  const void* fx_b = nullptr;
+  int fx_form = -1, fx_mode = 0;
+  int store_cols = 0;  // rows: > 0 keeps the first store_cols points of each lane
+  int hm_cmax = 0;     // columns of a Hermitian pass: columns 1 .. hm_cmax are also stored mirrored
 };
 
 // A tile of the persistent batch kernel: descriptor index, kind (0 forward lanes
@@ -217,6 +238,19 @@ size_t tc_fft_smem(int n);
 cudaError_t kernel_smem_grant(const void* kern, size_t smem);
 int kernel_ctas_per_sm(const void* kern, int threads, size_t smem);
 cudaError_t launch_lanes(const LaunchDesc& d, bool dbl, bool inv, cudaStream_t st);
+// Compile-time power-of-two kernels: whether one serves a descriptor whose
+// fx_form / fx_mode / operators are set, and its launch.
+bool fx_ready_f32(const LaunchDesc& d);
+bool fx_ready_f64(const LaunchDesc& d);
+cudaError_t launch_fx_f32(const LaunchDesc& d, cudaStream_t st);
+cudaError_t launch_fx_f64(const LaunchDesc& d, cudaStream_t st);
+// Lanes per tile of the compile-time columns (0: no build).
+int fx_col_lanes(long long n, bool dbl);
+// Stage list of the compile-time engine for n = 64 .. 4096 (a power of two).
+bool fx_stage_list(long long n, StageList& sl);
+// Step twiddle factors of N1-point columns over N2 columns (M = N1 N2):
+// a[t N2 + c] = W_M^{c t}, t < N1 / 16; b[q N2 + c] = W_M^{c q N1 / 16}, q < 16.
+cudaError_t gen_fx_step_dev(void* a, void* b, long long N1, long long N2, bool dbl, cudaStream_t st);
 size_t kargs_size(bool dbl);
 void kargs_pack(const LaunchDesc& d, bool dbl, void* dst);
 // Threads of a persistent batch CTA (a tile uses at most this many).
