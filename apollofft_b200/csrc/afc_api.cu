@@ -625,6 +625,8 @@ static cudaError_t exec_fourstep(const AxisPlan& ap, bool dbl, bool inv, const A
   a.in = io.in;
   a.out = ws;
   a.in_op = io.in_op;
+  a.herm_n = io.herm_n;
+  a.pair_w = io.pair_w;
   a.out_op = OUT_TW;
   a.jmul = N2;
   a.col_div = d2;

@@ -65,14 +65,16 @@ __device__ __forceinline__ typename CT<T>::type gload(const KArgs<T>& a, long lo
     case IN_HERM: {  // half spectrum (n/2+1 bins) expanded by Hermitian symmetry
       const C* p = static_cast<const C*>(a.in);
       const long long n = a.herm_n;
+      const long long j = (long long)i * a.jmul + col;  // index in the full spectrum
       C v;
-      if (2LL * i <= n) {
+      if (2 * j <= n) {
         v = p[base + (long long)i * a.im.es];
-      } else {
-        v = p[base + (n - i) * a.im.es];
+      } else {  // a two-pass column starts col elements into the lane
+        const long long es = a.im.es / a.jmul;
+        v = p[base + (n - j - col) * es];
         v.y = -v.y;
       }
-      if (i > 0 && 2LL * i != n) v = cscale(v, a.pair_w);
+      if (j > 0 && 2 * j != n) v = cscale(v, a.pair_w);
       return v;
     }
     case IN_CHIRP:

@@ -74,7 +74,8 @@ def test_columns(afc, cuda, precision, kind, dims):
 
 @pytest.mark.parametrize("precision", ["f64", "f32"])
 @pytest.mark.parametrize("dims,kind", [((8192,), "c2c"), ((16384,), "r2c_full"), ((65536,), "c2c"), ((1 << 20,), "c2c"),
-                                       ((16384, 3), "c2c"), ((3, 32768), "r2c_full"), ((24576,), "c2c")])
+                                       ((16384, 3), "c2c"), ((3, 32768), "r2c_full"), ((24576,), "c2c"),
+                                       ((32768,), "r2c_half")])
 def test_two_pass_lengths(afc, cuda, precision, dims, kind):
     check(afc, cuda, dims, 3, precision, kind)
 
