@@ -457,7 +457,7 @@ static afc_status build_fourstep(int64_t n, bool dbl, AxisPlan& ap, cudaStream_t
   AFC_CUDA(dev_alloc(&ap.tw_hi, (size_t)nhi * csz), "four-step twiddles");
   AFC_CUDA(gen_roots_dev(ap.tw_lo, B, 1, n, dbl, st), "four-step twiddles");
   AFC_CUDA(gen_roots_dev(ap.tw_hi, nhi, B, n, dbl, st), "four-step twiddles");
-  if (ap.lp1.fx_tw) {
+  if (ap.lp1.fx_tw && ap.N1 % 16 == 0) {  // a power of two
     const size_t na = (size_t)(ap.N1 / 16) * ap.N2, nb = (size_t)16 * ap.N2;
     AFC_CUDA(dev_alloc(&ap.fx_a, (na + nb) * csz), "step twiddles");
     ap.fx_b = static_cast<char*>(ap.fx_a) + na * csz;
@@ -547,6 +547,7 @@ struct RecLaunch {
 };
 struct Recorder {
   std::vector<RecLaunch> launches;
+  bool fx = false;  // launches may go to the compile-time engine
   int max_threads = kBatchThreads;
 };
 static thread_local Recorder* tl_rec = nullptr;
@@ -566,6 +567,10 @@ static void record(LaunchDesc d, int kind, bool inv) {
   untag(out, d.out_sel);
   d.in = in;
   d.out = const_cast<void*>(out);
+  if (d.fx_form >= 0) {
+    tl_rec->launches.push_back(RecLaunch{d, kind, inv});
+    return;
+  }
   const int mt = tl_rec->max_threads;
   while (d.L > 1 && d.L * d.P > mt) d.L = d.L > 1 ? d.L / 2 : 1;
   if (d.L * d.P > mt) d.P = std::max(1, mt / d.L);
@@ -577,7 +582,7 @@ static void record(LaunchDesc d, int kind, bool inv) {
 // arithmetic in 32 bits.
 static bool fx_take(LaunchDesc& d, const LenPlan& lp, int form, int mode, bool dbl) {
   const long long lim = 1ll << 31;
-  if (!lp.fx_tw || tl_rec || d.lanes <= 0 || d.lanes >= lim - 4096) return false;
+  if (!lp.fx_tw || (tl_rec && !tl_rec->fx) || d.lanes <= 0 || d.lanes >= lim - 4096) return false;
   if (d.im.d1 >= lim || d.im.d2 >= lim || d.om.d1 >= lim || d.om.d2 >= lim) return false;
   if (d.col_div >= lim || d.col_mod >= lim || d.nlen >= lim || d.nlen_out >= lim || d.jmul * lp.n >= 2 * lim)
     return false;
@@ -588,24 +593,25 @@ static bool fx_take(LaunchDesc& d, const LenPlan& lp, int form, int mode, bool d
   f.fx_form = form;
   f.fx_mode = mode;
   if (!(dbl ? fx_ready_f64(f) : fx_ready_f32(f))) return false;
+  if (tl_rec && (dbl ? fx_batch_kind_f64(f) : fx_batch_kind_f32(f)) < 0) return false;
   d = f;
   return true;
 }
 
 static cudaError_t do_lanes(const LaunchDesc& d, bool dbl, bool inv, cudaStream_t st) {
-  if (d.fx_form >= 0) return dbl ? launch_fx_f64(d, st) : launch_fx_f32(d, st);
   if (tl_rec) {
     record(d, 0, inv);
     return cudaSuccess;
   }
+  if (d.fx_form >= 0) return dbl ? launch_fx_f64(d, st) : launch_fx_f32(d, st);
   return launch_lanes(d, dbl, inv, st);
 }
 static cudaError_t do_conv(const LaunchDesc& d, bool dbl, bool inv, cudaStream_t st) {
-  if (d.fx_form >= 0) return dbl ? launch_fx_f64(d, st) : launch_fx_f32(d, st);
   if (tl_rec) {
     record(d, 1, inv);
     return cudaSuccess;
   }
+  if (d.fx_form >= 0) return dbl ? launch_fx_f64(d, st) : launch_fx_f32(d, st);
   return launch_conv(d, dbl, st);
 }
 
@@ -726,7 +732,7 @@ static cudaError_t exec_axis(const AxisPlan& ap, bool dbl, bool inv, const AxisI
       // barrier and a shared-memory round trip on each side of the stages and
       // keeps one tile per CTA in flight; here a dozen CTAs per SM load, compute
       // and store independently.
-      if (!tl_rec && ap.lp.fx_tw) {
+      if ((!tl_rec || tl_rec->fx) && ap.lp.fx_tw) {
         LaunchDesc f = d;
         if (io.im.es == 1 && io.om.es == 1) {
           f.store_cols = io.out_op == OUT_TRUNC ? (int)io.nlen : (int)io.store_cols;
@@ -860,7 +866,7 @@ static cudaError_t exec_axis(const AxisPlan& ap, bool dbl, bool inv, const AxisI
         fb.im = LaneMap{N1, d2, d2 * M, N2, M, 1, nullptr};
         fb.om = fb.im;
         fb.in = w1;
-        fb.out = w2;
+        fb.out = w1;  // a row tile reads all of its rows before it stores them
         fb.in_op = IN_C;
         fb.out_op = OUT_C;
         fb.spec = inv ? ap.spec_ri : ap.spec_rf;
@@ -873,7 +879,7 @@ static cudaError_t exec_axis(const AxisPlan& ap, bool dbl, bool inv, const AxisI
         fc.im = LaneMap{N2, d2, d2 * M, 1, M, N2, nullptr};
         fc.om = io.om.off ? LaneMap{1, N2, 0, 0, io.om.es, N2 * io.om.es, io.om.off}
                           : LaneMap{N2, io.om.d2, io.om.s0, io.om.es, io.om.s2, N2 * io.om.es, nullptr};
-        fc.in = w2;
+        fc.in = w1;
         fc.out = io.out;
         fc.in_op = IN_STEP;
         fc.fx_a = mp.fx_a;
@@ -1006,12 +1012,23 @@ static int plan_stages_uncached(int64_t m, size_t csz) {
   return best;
 }
 
+// Whether a Bluestein convolution of M points runs on the compile-time engine.
+static bool fx_conv_length(int64_t M) {
+  return env_int("AFC_FX", 1) != 0 && (M & (M - 1)) == 0 && M >= 64 && M <= (1 << 20);
+}
+
 // Convolution length for Rader / Bluestein: the length >= need with the least
 // work (length x stages) among the next power of two and the 7-smooth lengths
 // below it (Bluestein's convolution is exact for any length >= 2n - 1).
-static int64_t conv_length(int64_t need, size_t csz) {
+static int64_t conv_length(int64_t need, size_t csz, bool bluestein) {
   int64_t p2 = 1;
   while (p2 < need) p2 <<= 1;
+  // Bluestein convolutions of 64 .. 2^20 points run on the compile-time engine
+  // at powers of two, three to four times as fast per point as a 7-smooth length
+  // on the general one (complex64, 2^22 convolution points: 50 against 183 us
+  // in one tile, 78 against 280 us in three passes), so a smooth length at
+  // least half as long never pays
+  if (bluestein && fx_conv_length(p2)) return p2;
   int64_t best = p2;
   static const int mode = env_int("AFC_CONV_LEN", 0);  // 0 cost model, 1 powers of two only
   if (mode == 1) return p2;
@@ -1047,7 +1064,7 @@ static afc_status build_axis(int64_t n, bool dbl, AxisPlan& ap, cudaStream_t st)
     // convolution of length p-1, exact or zero-padded to a power of two.
     const int64_t L = n - 1;
     int64_t M = L;
-    if (!plannable(L, csz)) M = conv_length(2 * L - 1, csz);
+    if (!plannable(L, csz)) M = conv_length(2 * L - 1, csz, false);
     if (!plannable(M, csz))
       return fail(AFC_ERR_UNSUPPORTED, "no Rader plan for %lld", (long long)n);
     ap.algo = ALGO_RADER;
@@ -1077,7 +1094,7 @@ static afc_status build_axis(int64_t n, bool dbl, AxisPlan& ap, cudaStream_t st)
     return s;
   }
   // Bluestein chirp-z with a convolution of length M >= 2n-1.
-  const int64_t M = conv_length(2 * n - 1, csz);
+  const int64_t M = conv_length(2 * n - 1, csz, true);
   ap.algo = ALGO_BLUESTEIN;
   ap.M = M;
   AFC_CUDA(dev_alloc(&ap.chirp, (size_t)n * csz), "chirp");
@@ -1087,7 +1104,9 @@ static afc_status build_axis(int64_t n, bool dbl, AxisPlan& ap, cudaStream_t st)
   AFC_CUDA(gen_bluestein_b_dev(ap.spec_f, ap.chirp, n, M, false, dbl, st), "Bluestein kernel");
   AFC_CUDA(gen_bluestein_b_dev(ap.spec_i, ap.chirp, n, M, true, dbl, st), "Bluestein kernel");
   afc_status s;
-  if (plannable(M, csz)) {
+  // one tile up to 4096 points, else (8192 complex64 would still fit the
+  // general engine's tile) the three compile-time passes
+  if (plannable(M, csz) && !(M > 4096 && fx_conv_length(M))) {
     ap.conv_smem = true;
     s = build_lenplan(M, dbl, ap.lp, st);
     if (s != AFC_OK) return s;
@@ -1792,6 +1811,15 @@ struct afc_batch_plan_s {
     int grid = 0;
   };
   std::vector<Phase> phases[2];
+  // compile-time tiles, per direction: one launch before the phases
+  struct FxList {
+    void* descs = nullptr;
+    afc::FxBatchItem* items = nullptr;
+    int nitems = 0;
+    int* ctr = nullptr;  // claim counter, then one counter per transform of several passes
+    int nctr = 0;
+  };
+  FxList fx[2];
   int* counters = nullptr;  // one per phase and direction
   afc::Fence fence;         // last use of ws / counters on the GPU
   // CUDA graph of the persistent phases, keyed by (in, out, direction)
@@ -1808,6 +1836,11 @@ struct afc_batch_plan_s {
         if (ph.items) cudaFree(ph.items);
       }
     if (counters) cudaFree(counters);
+    for (auto& f : fx) {
+      if (f.descs) cudaFree(f.descs);
+      if (f.items) cudaFree(f.items);
+      if (f.ctr) cudaFree(f.ctr);
+    }
   }
 };
 
@@ -1852,7 +1885,19 @@ static cudaError_t run_batch_persistent(afc_batch_plan_s& bp, const void* in, vo
   auto& ph = bp.phases[inv ? 1 : 0];
   const size_t np = ph.size();
   int* ctr = bp.counters + (inv ? 8 : 0);
-  cudaError_t e = cudaMemsetAsync(ctr, 0, np * sizeof(int), st);
+  cudaError_t e = cudaSuccess;
+  const auto& fx = bp.fx[inv ? 1 : 0];
+  if (fx.nitems > 0) {
+    unsigned* err = device_err_word();
+    if (!err) return cudaErrorMemoryAllocation;
+    e = cudaMemsetAsync(fx.ctr, 0, fx.nctr * sizeof(int), st);
+    if (e != cudaSuccess) return e;
+    e = bp.dbl ? launch_fx_batch_f64(fx.descs, fx.items, fx.nitems, fx.ctr, in, out, bp.ws, err, inv, st)
+               : launch_fx_batch_f32(fx.descs, fx.items, fx.nitems, fx.ctr, in, out, bp.ws, err, inv, st);
+    if (e != cudaSuccess) return e;
+  }
+  if (np == 0) return e;
+  e = cudaMemsetAsync(ctr, 0, np * sizeof(int), st);
   if (e != cudaSuccess) return e;
   for (size_t k = 0; k < np; ++k) {
     e = launch_batch(ph[k].descs, ph[k].items, ph[k].nitems, ctr + k, ph[k].smem, ph[k].grid, in, out, bp.ws, bp.dbl,
@@ -1871,7 +1916,7 @@ static std::map<std::pair<int64_t, int>, std::pair<int, int>> g_tune;
 
 static void tune_group(BatchGroup& g, bool dbl, void* scratch, cudaStream_t st) {
   AxisPlan& ap = *g.ap;
-  if (ap.algo != ALGO_SMEM) return;
+  if (ap.algo != ALGO_SMEM || ap.lp.fx_tw) return;  // compile-time lengths have one shape
   const auto key = std::make_pair(g.n, dbl ? 1 : 0);
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
@@ -1944,6 +1989,84 @@ static void tune_group(BatchGroup& g, bool dbl, void* scratch, cudaStream_t st) 
   g_tune[key] = std::make_pair(bestP, bestL);
 }
 
+// The tile list of the compile-time batch kernel.  Transforms of several passes
+// come first, largest first, pass k of a transform about k kLag tiles after its
+// first one: far enough that the tiles in flight rarely wait, close enough that
+// the intermediates stay in L2.  Single-tile transforms fill the drain.
+struct FxAcc {
+  static constexpr double kLag = 1800;  // three to four tiles for each CTA in flight
+  struct Multi {
+    long long tiles;  // all passes of one transform
+    std::vector<FxBatchItem> items;
+    std::vector<int> pass;  // pass of each item
+  };
+  std::vector<unsigned char> descs;
+  std::vector<Multi> multi;
+  std::vector<std::pair<double, FxBatchItem>> single;  // cost, tile
+  int ndesc = 0, ndep = 0;
+
+  void add(const std::vector<RecLaunch>& launches, long long lanes, bool dbl) {
+    const size_t ksz = kargs_size(dbl);
+    std::vector<Multi> grp(launches.size() > 1 ? lanes : 0);
+    for (auto& m : grp) m.tiles = 0;
+    for (size_t k = 0; k < launches.size(); ++k) {
+      const LaunchDesc& d = launches[k].d;
+      const int di = ndesc++;
+      descs.resize((size_t)ndesc * ksz);
+      kargs_pack(d, dbl, descs.data() + (size_t)di * ksz);
+      const int kind = dbl ? fx_batch_kind_f64(d) : fx_batch_kind_f32(d);
+      const long long L = 4096 / d.sl.n, tiles = (d.lanes + L - 1) / L;
+      if (launches.size() == 1) {
+        const double c = d.sl.nst * (d.fx_mode == FX_CONV ? 2.0 : 1.0);
+        for (long long t = 0; t < tiles; ++t)
+          single.emplace_back(c, FxBatchItem{di, kind, (unsigned)(t * L), 0, 0, {}});
+        continue;
+      }
+      // pass k of lane i covers sub-lanes [i per, (i + 1) per), a multiple of L
+      const long long per = d.lanes / lanes;
+      for (long long i = 0; i < lanes; ++i) {
+        Multi& m = grp[i];
+        const long long before = m.tiles;
+        for (long long q = i * per; q < (i + 1) * per; q += L) {
+          m.items.push_back(FxBatchItem{di, kind, (unsigned)q, (int)(1 + ndep + i), (int)before, {}});
+          m.pass.push_back((int)k);
+          ++m.tiles;
+        }
+      }
+    }
+    if (!grp.empty()) ndep += (int)lanes;
+    for (auto& m : grp) multi.push_back(std::move(m));
+  }
+
+  afc_status finish(afc_batch_plan_s::FxList& out, bool dbl, cudaStream_t st) {
+    std::stable_sort(multi.begin(), multi.end(), [](const Multi& a, const Multi& b) { return a.tiles > b.tiles; });
+    std::stable_sort(single.begin(), single.end(), [](auto& a, auto& b) { return a.first > b.first; });
+    std::vector<std::pair<double, FxBatchItem>> all;
+    double at = 0;
+    for (const auto& m : multi) {
+      for (size_t j = 0; j < m.items.size(); ++j) all.emplace_back(at + m.pass[j] * kLag, m.items[j]);
+      at += (double)m.tiles;
+    }
+    const double span = multi.empty() ? 1.0 : 2 * kLag;
+    for (size_t j = 0; j < single.size(); ++j)
+      all.emplace_back(at + span * (double)j / (double)single.size(), single[j].second);
+    std::stable_sort(all.begin(), all.end(), [](auto& a, auto& b) { return a.first < b.first; });
+    if (all.empty()) return AFC_OK;
+    std::vector<FxBatchItem> items;
+    for (auto& p : all) items.push_back(p.second);
+    out.nitems = (int)items.size();
+    out.nctr = 1 + ndep;
+    AFC_CUDA(dev_alloc(&out.descs, descs.size()), "batch descriptors");
+    AFC_CUDA(dev_alloc((void**)&out.items, items.size() * sizeof(FxBatchItem)), "batch items");
+    AFC_CUDA(dev_alloc((void**)&out.ctr, out.nctr * sizeof(int)), "batch counters");
+    AFC_CUDA(cudaMemcpyAsync(out.descs, descs.data(), descs.size(), cudaMemcpyHostToDevice, st), "batch descriptors");
+    AFC_CUDA(cudaMemcpyAsync(out.items, items.data(), items.size() * sizeof(FxBatchItem), cudaMemcpyHostToDevice, st),
+             "batch items");
+    AFC_CUDA(cudaStreamSynchronize(st), "batch items");  // the vectors leave
+    return AFC_OK;
+  }
+};
+
 // Records every group's launches for one direction and turns them into the
 // phase lists of the persistent kernel (launch k of a group runs in phase k).
 static afc_status build_phases(afc_batch_plan_s& bp, bool inv, cudaStream_t st) {
@@ -1956,8 +2079,10 @@ static afc_status build_phases(afc_batch_plan_s& bp, bool inv, cudaStream_t st) 
     size_t smem = 0;
   };
   std::vector<PhaseAcc> acc;
+  FxAcc fxa;
   for (auto& g : bp.groups) {
     Recorder rec;
+    rec.fx = true;
     tl_rec = &rec;
     AxisIO io;
     io.in = tag_ptr(1, 0);
@@ -1984,6 +2109,20 @@ static afc_status build_phases(afc_batch_plan_s& bp, bool inv, cudaStream_t st) 
     } else {
       e = exec_axis(*g->ap, bp.dbl, inv, io, tag_ptr(3, g->ws_off), st);
     }
+    // a group goes to the compile-time list only as a whole: its passes are
+    // ordered there by its own counters
+    if (e == cudaSuccess && std::all_of(rec.launches.begin(), rec.launches.end(),
+                                        [](const RecLaunch& r) { return r.d.fx_form >= 0; })) {
+      tl_rec = nullptr;
+      fxa.add(rec.launches, g->lanes, bp.dbl);
+      continue;
+    }
+    if (e == cudaSuccess && std::any_of(rec.launches.begin(), rec.launches.end(),
+                                        [](const RecLaunch& r) { return r.d.fx_form >= 0; })) {
+      rec.launches.clear();
+      rec.fx = false;
+      e = exec_axis(*g->ap, bp.dbl, inv, io, tag_ptr(3, g->ws_off), st);
+    }
     tl_rec = nullptr;
     if (e != cudaSuccess) return cuda_fail(e, "batch record");
     for (size_t k = 0; k < rec.launches.size(); ++k) {
@@ -2002,6 +2141,10 @@ static afc_status build_phases(afc_batch_plan_s& bp, bool inv, cudaStream_t st) 
         pa.cost.push_back(c);
       }
     }
+  }
+  {
+    afc_status fs = fxa.finish(bp.fx[inv ? 1 : 0], bp.dbl, st);
+    if (fs != AFC_OK) return fs;
   }
   if (acc.size() > 8) return fail(AFC_ERR_UNSUPPORTED, "batch plan needs %zu phases (max 8)", acc.size());
   int sms = 148;

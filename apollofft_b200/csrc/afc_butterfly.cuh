@@ -119,6 +119,31 @@ template <bool INV> struct DFT<16, INV> {
   }
 };
 
+// 16-point butterfly of v[0..7], the upper half zero on input: the inner DFT4
+// over (v[a], v[a + 4], 0, 0) needs one addition per output instead of two.
+template <bool INV, class C> __device__ __forceinline__ void dft16_half(C* v) {
+  C z[4][4];
+#pragma unroll
+  for (int a = 0; a < 4; ++a) {
+    const C s = v[a], d = v[a + 4], r = rot90<INV>(d);
+    z[a][0] = cadd(s, d);
+    z[a][1] = cadd(s, r);
+    z[a][2] = csub(s, d);
+    z[a][3] = csub(s, r);
+  }
+#pragma unroll
+  for (int a = 1; a < 4; ++a)
+#pragma unroll
+    for (int c = 1; c < 4; ++c) z[a][c] = w16mul<INV>(z[a][c], a * c);
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    C col[4] = {z[0][c], z[1][c], z[2][c], z[3][c]};
+    DFT<4, INV>::run(col);
+#pragma unroll
+    for (int d = 0; d < 4; ++d) v[c + 4 * d] = col[d];
+  }
+}
+
 template <int R> struct OddRoots;
 template <> struct OddRoots<3> {
   __host__ __device__ __forceinline__ static constexpr double c(int e) {

@@ -9,13 +9,15 @@
 namespace afc {
 
 // CTAs per SM a kernel is built for.  16 points are 32 (complex64) or 64
-// (complex128) registers; three 256-thread CTAs leave 80 registers, two 128.
-template <class T> constexpr int fx_min_ctas(int threads) {
+// (complex128) registers; 768 threads leave 80 registers, 512 leave 128.  The
+// odd lengths hold at most 10 points: 1024 threads of 64 registers.
+template <class T, int N> constexpr int fx_min_ctas(int threads) {
+  if (!fx_pow2(N)) return (sizeof(T) == 4 ? 1024 : 512) / ((threads + 31) / 32 * 32);
   return threads > 256 ? 1 : (sizeof(T) == 4 ? 3 : 2) * (256 / threads);
 }
 
-template <class T, int N, int FORM, int MODE, int IN, int OUT>
-__global__ void __launch_bounds__(FxTile<T, N, FORM>::threads, fx_min_ctas<T>(FxTile<T, N, FORM>::threads))
+template <class T, int N, int FORM, int MODE, int IN, int OUT, bool HALF>
+__global__ void __launch_bounds__(FxTile<T, N, FORM>::threads, fx_min_ctas<T, N>(FxTile<T, N, FORM>::threads))
     fx_kernel(const __grid_constant__ KArgs<T> a) {
   extern __shared__ __align__(16) unsigned char smraw[];
   constexpr int L = FxTile<T, N, FORM>::L;
@@ -23,7 +25,8 @@ __global__ void __launch_bounds__(FxTile<T, N, FORM>::threads, fx_min_ctas<T>(Fx
   // the previous launch drains; nothing is read before that one has completed
   griddep_wait();
   griddep_launch_dependents();
-  fx_tile<T, N, L, FORM, MODE, IN, OUT>(a, blockIdx.x * (unsigned)L, reinterpret_cast<typename CT<T>::type*>(smraw));
+  fx_tile<T, N, L, FORM, MODE, IN, OUT, HALF>(a, a.in, a.out, blockIdx.x * (unsigned)L,
+                                       reinterpret_cast<typename CT<T>::type*>(smraw));
 }
 
 struct FxEntry {
@@ -31,25 +34,30 @@ struct FxEntry {
   int L = 0, threads = 0;
   size_t smem = 0;
 };
-template <class T, int N, int FORM, int MODE, int IN, int OUT> static FxEntry fx_entry() {
+template <class T, int N, int FORM, int MODE, int IN, int OUT, bool HALF> static FxEntry fx_entry() {
   using Tl = FxTile<T, N, FORM>;
-  return FxEntry{reinterpret_cast<const void*>(&fx_kernel<T, N, FORM, MODE, IN, OUT>), Tl::L, Tl::threads, Tl::smem};
+  return FxEntry{reinterpret_cast<const void*>(&fx_kernel<T, N, FORM, MODE, IN, OUT, HALF>), Tl::L, Tl::threads, Tl::smem};
 }
 
 // Lane-minor forms stop at 1024 points: rows of 64 bytes at 2048 would need a
 // CTA of 1024 threads (64 registers each).
-template <class T, int FORM, int MODE, int IN, int OUT> static FxEntry fx_by_length(long long n) {
+template <class T, int FORM, int MODE, int IN, int OUT, bool HALF = false> static FxEntry fx_by_length(long long n) {
   switch (n) {
-    case 64: return fx_entry<T, 64, FORM, MODE, IN, OUT>();
-    case 128: return fx_entry<T, 128, FORM, MODE, IN, OUT>();
-    case 256: return fx_entry<T, 256, FORM, MODE, IN, OUT>();
-    case 512: return fx_entry<T, 512, FORM, MODE, IN, OUT>();
-    case 1024: return fx_entry<T, 1024, FORM, MODE, IN, OUT>();
+    case 64: return fx_entry<T, 64, FORM, MODE, IN, OUT, HALF>();
+    case 128: return fx_entry<T, 128, FORM, MODE, IN, OUT, HALF>();
+    case 256: return fx_entry<T, 256, FORM, MODE, IN, OUT, HALF>();
+    case 512: return fx_entry<T, 512, FORM, MODE, IN, OUT, HALF>();
+    case 1024: return fx_entry<T, 1024, FORM, MODE, IN, OUT, HALF>();
     default: break;
   }
   if constexpr (FORM == FX_ROWS) {
-    if (n == 2048) return fx_entry<T, 2048, FORM, MODE, IN, OUT>();
-    if (n == 4096) return fx_entry<T, 4096, FORM, MODE, IN, OUT>();
+    if (n == 2048) return fx_entry<T, 2048, FORM, MODE, IN, OUT, HALF>();
+    if (n == 4096) return fx_entry<T, 4096, FORM, MODE, IN, OUT, HALF>();
+  }
+  if constexpr (FORM != FX_ROWS_T && MODE != FX_CONV && IN == IN_C && OUT == OUT_C) {
+    if (n == 243) return fx_entry<T, 243, FORM, MODE, IN, OUT, HALF>();
+    if (n == 250) return fx_entry<T, 250, FORM, MODE, IN, OUT, HALF>();
+    if (n == 343) return fx_entry<T, 343, FORM, MODE, IN, OUT, HALF>();
   }
   return FxEntry{};
 }
@@ -63,11 +71,15 @@ template <class T> static FxEntry fx_lookup(const LaunchDesc& d) {
   }
   const bool chin = d.in_op == IN_CHIRP || d.in_op == IN_CHIRP_R;
   const bool chout = d.out_op == OUT_CHIRP || d.out_op == OUT_CHIRP_RE;
+  // chirped points j = i jmul + col below n jmul / 2 lie in the lower half of every lane
+  const bool half = 2 * std::max(d.nlen, d.nlen_out) <= n * d.jmul;
   switch (d.fx_form) {
     case FX_ROWS:
       if (d.fx_mode == FX_CONV) {
         if (cin && cout) return fx_by_length<T, FX_ROWS, FX_CONV, IN_C, OUT_C>(n);
-        if (chin && chout) return fx_by_length<T, FX_ROWS, FX_CONV, IN_CHIRP, OUT_CHIRP>(n);
+        if (chin && chout)  // half: Bluestein always, a CZT when both of its lengths are at most n / 2
+          return half ? fx_by_length<T, FX_ROWS, FX_CONV, IN_CHIRP, OUT_CHIRP, true>(n)
+                      : fx_by_length<T, FX_ROWS, FX_CONV, IN_CHIRP, OUT_CHIRP>(n);
       } else if (cin && cout) {
         return d.fx_mode == FX_FWD ? fx_by_length<T, FX_ROWS, FX_FWD, IN_C, OUT_C>(n)
                                    : fx_by_length<T, FX_ROWS, FX_INV, IN_C, OUT_C>(n);
@@ -83,10 +95,10 @@ template <class T> static FxEntry fx_lookup(const LaunchDesc& d) {
         return fx_by_length<T, FX_COLS, FX_FWD, IN_C, OUT_STEP>(n);
       if (d.fx_mode == FX_INV && cin && d.out_op == OUT_STEP)
         return fx_by_length<T, FX_COLS, FX_INV, IN_C, OUT_STEP>(n);
-      if (d.fx_mode == FX_FWD && chin && d.out_op == OUT_STEP)
-        return fx_by_length<T, FX_COLS, FX_FWD, IN_CHIRP, OUT_STEP>(n);
-      if (d.fx_mode == FX_INV && d.in_op == IN_STEP && chout)
-        return fx_by_length<T, FX_COLS, FX_INV, IN_STEP, OUT_CHIRP>(n);
+      if (d.fx_mode == FX_FWD && chin && d.out_op == OUT_STEP && half)
+        return fx_by_length<T, FX_COLS, FX_FWD, IN_CHIRP, OUT_STEP, true>(n);
+      if (d.fx_mode == FX_INV && d.in_op == IN_STEP && chout && half)
+        return fx_by_length<T, FX_COLS, FX_INV, IN_STEP, OUT_CHIRP, true>(n);
       break;
     case FX_ROWS_T:
       if (d.fx_mode == FX_FWD && cin && cout) return fx_by_length<T, FX_ROWS_T, FX_FWD, IN_C, OUT_C>(n);
@@ -128,6 +140,163 @@ template <class T> static cudaError_t launch_fx_t(const LaunchDesc& d, cudaStrea
   ce = cudaLaunchKernelExC(&cfg, e.k, args);
   count_launch(1);
   return ce;
+}
+
+// ───────────────────────── persistent batch kernel ─────────────────────────
+// Every compile-time tile of an uneven batch in one launch.  A tile is 4096
+// points (256 threads) of any length and form; CTAs claim tiles in list order
+// from an atomic counter.  A transform of several passes (two-pass lengths,
+// large Bluestein) orders them by a counter of its own: each finished tile adds
+// one, and a tile of a later pass waits until every tile of the passes before
+// it is done.  Waiting is safe without co-residency: a tile waits only for tiles
+// earlier in the list, those were claimed earlier by CTAs that are running, and
+// the lowest unfinished tile never waits for an unfinished one.  Waits are
+// bounded: on timeout the CTA sets the error word and leaves.
+//
+// One launch instead of one per pass keeps a transform's intermediate in L2
+// (the list runs its passes a few hundred tiles apart) and leaves one tail.  The
+// next tile's claim and list entry are fetched while the current tile runs.
+
+constexpr int kFxBatchThreads = 256;
+
+template <class T, int N, int FORM, int MODE, int IN, int OUT>
+__device__ __forceinline__ void fx_batch_tile(const KArgs<T>& a, const void* in, void* out, unsigned q0,
+                                              unsigned char* sm) {
+  fx_tile<T, N, 4096 / N, FORM, MODE, IN, OUT, IN == IN_CHIRP || OUT == OUT_CHIRP>(a, in, out, q0, reinterpret_cast<typename CT<T>::type*>(sm));
+}
+
+template <class T, bool INV>
+__global__ void __launch_bounds__(kFxBatchThreads, sizeof(T) == 4 ? 3 : 2)
+    fx_batch_kernel(const KArgs<T>* __restrict__ descs, const FxBatchItem* __restrict__ items, int nitems, int* ctr,
+                    const void* in_base, void* out_base, void* ws_base, unsigned* err) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  __shared__ __align__(16) FxBatchItem s_item[2];
+  __shared__ int s_idx[2];
+  const int tid = threadIdx.x;
+  constexpr int DIR = INV ? FX_INV : FX_FWD;
+  // nothing of the loop but one claim lives in registers while a tile runs: the
+  // current list entry is [p], the next one arrives in [p ^ 1] meanwhile
+  if (tid == 0) {
+    s_idx[0] = atomicAdd(ctr, 1);
+    s_idx[1] = atomicAdd(ctr, 1);
+    s_item[0] = items[min(s_idx[0], nitems - 1)];
+  }
+  __syncthreads();
+  for (int p = 0; s_idx[p] < nitems; p ^= 1) {
+    const FxBatchItem& bi = s_item[p];
+    int nx = 0;
+    if (tid == 0) {
+      const FxBatchItem* src = items + min(s_idx[p ^ 1], nitems - 1);
+      const unsigned dst = smem_u32(&s_item[p ^ 1]);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src) : "memory");
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst + 16), "l"(reinterpret_cast<const char*>(src) + 16) : "memory");
+      nx = atomicAdd(ctr, 1);
+    }
+    if (bi.wait > 0) {  // the passes before this one, of the same transform
+      bool ok = true;
+      if (tid == 0) {
+        const volatile int* c = ctr + bi.dep;
+        int k = 0;
+        while (*c < bi.wait && k < (1 << 22)) {
+          __nanosleep(64);
+          ++k;
+        }
+        ok = *c >= bi.wait;
+        __threadfence();
+      }
+      if (__syncthreads_or(!ok)) {
+        if (tid == 0) atomicExch(err, 1u);
+        return;
+      }
+    }
+    const KArgs<T>& a = descs[bi.desc];
+    const char* bases[4] = {nullptr, static_cast<const char*>(in_base), static_cast<const char*>(out_base),
+                            static_cast<const char*>(ws_base)};
+    const void* in = (a.in_sel == 1 ? bases[1] : a.in_sel == 2 ? bases[2] : bases[3]) + (size_t)a.in;
+    void* out = const_cast<char*>((a.out_sel == 2 ? bases[2] : a.out_sel == 1 ? bases[1] : bases[3]) + (size_t)a.out);
+    const unsigned q0 = bi.q0;
+#define AFC_FXB(OP, LG, FORM, MODE, IN, OUT) \
+  case OP * 8 + LG - 6: fx_batch_tile<T, (1 << LG), FORM, MODE, IN, OUT>(a, in, out, q0, smraw); break;
+#define AFC_FXB5(OP, FORM, MODE, IN, OUT)                                                                     \
+  AFC_FXB(OP, 6, FORM, MODE, IN, OUT) AFC_FXB(OP, 7, FORM, MODE, IN, OUT) AFC_FXB(OP, 8, FORM, MODE, IN, OUT) \
+  AFC_FXB(OP, 9, FORM, MODE, IN, OUT) AFC_FXB(OP, 10, FORM, MODE, IN, OUT)
+#define AFC_FXB7(OP, FORM, MODE, IN, OUT) \
+  AFC_FXB5(OP, FORM, MODE, IN, OUT) AFC_FXB(OP, 11, FORM, MODE, IN, OUT) AFC_FXB(OP, 12, FORM, MODE, IN, OUT)
+    switch (bi.kind) {
+      AFC_FXB7(FXB_ROWS, FX_ROWS, DIR, IN_C, OUT_C)
+      AFC_FXB5(FXB_COLS, FX_COLS, DIR, IN_C, OUT_STEP)
+      AFC_FXB5(FXB_ROWS_T, FX_ROWS_T, DIR, IN_C, OUT_C)
+      AFC_FXB7(FXB_CONV, FX_ROWS, FX_CONV, IN_CHIRP, OUT_CHIRP)
+      AFC_FXB5(FXB_CHIRP_COLS, FX_COLS, FX_FWD, IN_CHIRP, OUT_STEP)
+      AFC_FXB5(FXB_CONV_ROWS, FX_ROWS, FX_CONV, IN_C, OUT_C)
+      AFC_FXB5(FXB_COLS_CHIRP, FX_COLS, FX_INV, IN_STEP, OUT_CHIRP)
+      default: break;
+    }
+#undef AFC_FXB7
+#undef AFC_FXB5
+#undef AFC_FXB
+    __syncthreads();  // the tile's stores are issued, its shared memory is free
+    if (tid == 0) {
+      if (bi.dep > 0) {
+        __threadfence();
+        atomicAdd(ctr + bi.dep, 1);
+      }
+      asm volatile("cp.async.wait_all;\n" ::: "memory");
+      s_idx[p] = nx;
+    }
+    __syncthreads();
+  }
+}
+
+// Tile kind of a descriptor in the batch kernel, -1 when it has none.
+template <class T> static int fx_batch_kind_t(const LaunchDesc& d) {
+  if (!fx_lookup<T>(d).k || d.store_cols || d.hm_cmax) return -1;
+  if ((d.in_op != IN_C && d.in_op != IN_CHIRP && d.in_op != IN_STEP) ||
+      (d.out_op != OUT_C && d.out_op != OUT_CHIRP && d.out_op != OUT_STEP))
+    return -1;
+  int lg = 0;
+  while ((1 << lg) < d.sl.n) ++lg;
+  if ((1 << lg) != d.sl.n) return -1;
+  int op;
+  if (d.fx_form == FX_ROWS) op = d.fx_mode != FX_CONV ? FXB_ROWS : d.in_op == IN_CHIRP ? FXB_CONV : FXB_CONV_ROWS;
+  else if (d.fx_form == FX_ROWS_T) op = FXB_ROWS_T;
+  else if (d.out_op == OUT_STEP) op = d.in_op == IN_CHIRP ? FXB_CHIRP_COLS : FXB_COLS;
+  else if (d.in_op == IN_STEP) op = FXB_COLS_CHIRP;
+  else return -1;
+  if (d.out_op == OUT_CHIRP || d.in_op == IN_CHIRP)  // chirp tiles of the batch kernel are half
+    if (2 * std::max(d.nlen, d.nlen_out) > (long long)d.sl.n * d.jmul) return -1;
+  if (lg > 10 && op != FXB_ROWS && op != FXB_CONV) return -1;
+  return op * 8 + lg - 6;
+}
+
+template <class T> constexpr size_t fx_batch_smem() {
+  using C = typename CT<T>::type;
+  size_t m = 0;
+  const int ns[7] = {64, 128, 256, 512, 1024, 2048, 4096};
+  for (int n : ns)
+    for (int lm = 0; lm < (n <= 1024 ? 2 : 1); ++lm) {
+      const size_t b = (size_t)(4096 / n) * fx_ld(n, 4096 / n, lm != 0, (int)sizeof(C)) * sizeof(C);
+      if (b > m) m = b;
+    }
+  return m;
+}
+
+template <class T>
+static cudaError_t launch_fx_batch_t(const void* descs, const FxBatchItem* items, int nitems, int* ctr, const void* in,
+                                     void* out, void* ws, unsigned* err, bool inv, cudaStream_t st) {
+  auto k = inv ? fx_batch_kernel<T, true> : fx_batch_kernel<T, false>;
+  const size_t smem = fx_batch_smem<T>();
+  cudaError_t e = kernel_smem_grant(reinterpret_cast<const void*>(k), smem);
+  if (e != cudaSuccess) return e;
+  int sms = 148, dev = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  long long grid = (long long)sms * kernel_ctas_per_sm(reinterpret_cast<const void*>(k), kFxBatchThreads, smem);
+  if (grid > nitems) grid = nitems;
+  k<<<(unsigned)grid, kFxBatchThreads, smem, st>>>(static_cast<const KArgs<T>*>(descs), items, nitems, ctr, in, out, ws,
+                                                   err);
+  count_launch(1);
+  return cudaGetLastError();
 }
 
 }  // namespace afc

@@ -76,6 +76,28 @@ struct BatchItem {
   long long q0;
 };
 
+// Tile kinds of the compile-time batch kernel (times 8, plus log2 n - 6).
+enum FxBatchOp {
+  FXB_ROWS = 0,        // contiguous lanes
+  FXB_COLS = 1,        // two-pass length, columns with the step twiddle
+  FXB_ROWS_T = 2,      // two-pass length, rows stored as columns
+  FXB_CONV = 3,        // Bluestein convolution in one tile
+  FXB_CHIRP_COLS = 4,  // large Bluestein: chirp, columns, step twiddle
+  FXB_CONV_ROWS = 5,   //   rows times the spectrum
+  FXB_COLS_CHIRP = 6,  //   conjugate step twiddle, inverse columns, chirp
+};
+// A tile of the compile-time batch kernel: descriptor, kind, first lane, and
+// for transforms of several passes the transform's counter (index behind the
+// claim counter, 0: none) and how many of its tiles must be done first.
+struct FxBatchItem {
+  int desc;
+  int kind;
+  unsigned q0;
+  int dep;
+  int wait;
+  int pad[3];  // 32 bytes: two 16-byte asynchronous copies
+};
+
 // dynamic shared memory of lanes_kernel: L lanes x buffers x ld + 3 L lane descriptors
 inline size_t lanes_smem_bytes(const LaunchDesc& d, size_t csz) {
   const int nbuf = engine_buffers(d.sl.nst, d.stage_in, d.stage_out);
@@ -244,9 +266,15 @@ bool fx_ready_f32(const LaunchDesc& d);
 bool fx_ready_f64(const LaunchDesc& d);
 cudaError_t launch_fx_f32(const LaunchDesc& d, cudaStream_t st);
 cudaError_t launch_fx_f64(const LaunchDesc& d, cudaStream_t st);
+int fx_batch_kind_f32(const LaunchDesc& d);
+int fx_batch_kind_f64(const LaunchDesc& d);
+cudaError_t launch_fx_batch_f32(const void* descs, const FxBatchItem* items, int nitems, int* ctr, const void* in,
+                                void* out, void* ws, unsigned* err, bool inv, cudaStream_t st);
+cudaError_t launch_fx_batch_f64(const void* descs, const FxBatchItem* items, int nitems, int* ctr, const void* in,
+                                void* out, void* ws, unsigned* err, bool inv, cudaStream_t st);
 // Lanes per tile of the compile-time columns (0: no build).
 int fx_col_lanes(long long n, bool dbl);
-// Stage list of the compile-time engine for n = 64 .. 4096 (a power of two).
+// Stage list of the compile-time engine: powers of two 64 .. 4096, and 243, 250, 343.
 bool fx_stage_list(long long n, StageList& sl);
 // Step twiddle factors of N1-point columns over N2 columns (M = N1 N2):
 // a[t N2 + c] = W_M^{c t}, t < N1 / 16; b[q N2 + c] = W_M^{c q N1 / 16}, q < 16.

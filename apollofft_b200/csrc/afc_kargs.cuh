@@ -49,6 +49,9 @@ template <class T> struct KArgs {
   const C* fx_tw;          // compile-time engine: stage twiddles and step twiddle factors
   const C* fx_a;
   const C* fx_b;
+  // log2 of im.d2, om.d2, col_div and col_mod when all four are powers of two
+  // (two-pass lengths on contiguous lanes), else fx_sh[0] = -1
+  int fx_sh[4];
   int store_cols;          // compile-time rows: > 0 keeps the first store_cols points
   int hm_cmax;             // compile-time columns: columns 1 .. hm_cmax are also stored mirrored
 };
@@ -207,6 +210,14 @@ template <class T> inline KArgs<T> to_kargs(const LaunchDesc& d) {
   a.fx_tw = static_cast<const C*>(d.fx_tw);
   a.fx_a = static_cast<const C*>(d.fx_a);
   a.fx_b = static_cast<const C*>(d.fx_b);
+  const long long pw[4] = {a.im.d2, a.om.d2, a.col_div, a.col_mod};
+  for (int i = 0; i < 4; ++i) {
+    int sh = 0;
+    while ((1ll << sh) < pw[i]) ++sh;
+    a.fx_sh[i] = sh;
+  }
+  for (int i = 0; i < 4; ++i)
+    if ((1ll << a.fx_sh[i]) != pw[i]) a.fx_sh[0] = -1;
   a.store_cols = d.store_cols;
   a.hm_cmax = d.hm_cmax;
   a.in_sel = d.in_sel;

@@ -774,6 +774,9 @@ bool fx_stage_list(long long n, StageList& sl) {
     case 1024: fx_list<1024>(sl); return true;
     case 2048: fx_list<2048>(sl); return true;
     case 4096: fx_list<4096>(sl); return true;
+    case 243: fx_list<243>(sl); return true;
+    case 250: fx_list<250>(sl); return true;
+    case 343: fx_list<343>(sl); return true;
     default: return false;
   }
 }
@@ -785,6 +788,9 @@ int fx_col_lanes(long long n, bool dbl) {
     case 256: return dbl ? FxTile<double, 256, FX_COLS>::L : FxTile<float, 256, FX_COLS>::L;
     case 512: return dbl ? FxTile<double, 512, FX_COLS>::L : FxTile<float, 512, FX_COLS>::L;
     case 1024: return dbl ? FxTile<double, 1024, FX_COLS>::L : FxTile<float, 1024, FX_COLS>::L;
+    case 243: return dbl ? FxTile<double, 243, FX_COLS>::L : FxTile<float, 243, FX_COLS>::L;
+    case 250: return dbl ? FxTile<double, 250, FX_COLS>::L : FxTile<float, 250, FX_COLS>::L;
+    case 343: return dbl ? FxTile<double, 343, FX_COLS>::L : FxTile<float, 343, FX_COLS>::L;
     default: return 0;
   }
 }

@@ -57,7 +57,8 @@ def check(afc, cuda, dims, batch, precision, kind):
 
 @pytest.mark.parametrize("precision", ["f64", "f32"])
 @pytest.mark.parametrize("kind", ["c2c", "r2c_full", "r2c_half"])
-@pytest.mark.parametrize("n,batch", [(64, 1), (64, 33), (128, 17), (256, 9), (512, 5), (1024, 3), (2048, 3), (4096, 2)])
+@pytest.mark.parametrize("n,batch", [(64, 1), (64, 33), (128, 17), (256, 9), (512, 5), (1024, 3), (2048, 3), (4096, 2),
+                                     (243, 10), (250, 1), (343, 11)])
 def test_rows(afc, cuda, precision, kind, n, batch):
     check(afc, cuda, (n,), batch, precision, kind)
 
@@ -65,7 +66,8 @@ def test_rows(afc, cuda, precision, kind, n, batch):
 @pytest.mark.parametrize("precision", ["f64", "f32"])
 @pytest.mark.parametrize("kind", ["c2c", "r2c_full", "r2c_half"])
 @pytest.mark.parametrize("dims", [(64, 1), (64, 2), (64, 3), (128, 7), (256, 18), (512, 33), (1024, 20), (1024, 130),
-                                  (64, 256), (3, 128, 10), (256, 3, 9), (128, 64, 66)])
+                                  (64, 256), (3, 128, 10), (256, 3, 9), (128, 64, 66), (243, 17), (250, 343), (343, 40),
+                                  (5, 250, 9)])
 def test_columns(afc, cuda, precision, kind, dims):
     if kind == "r2c_half" and dims[-1] < 2:
         pytest.skip("a half spectrum needs two points")
@@ -122,3 +124,29 @@ def test_caller_operations(afc, cuda, precision, n):
     czt = z.astype(np.complex128) @ np.exp(-0.3j * np.arange(nin)[:, None] - 0.7j / m * jk)
     # the chirps W^(j^2 / 2) carry the rounding of phases up to j^2 / 2
     assert rel(got, czt) < (2e-11 if precision == "f64" else 2e-5)
+
+
+@pytest.mark.parametrize("precision", ["f64", "f32"])
+@pytest.mark.parametrize("lengths", [
+    [8192],                                                       # one transform of two passes
+    [65521, 64, 8192, 10007, 1031, 100, 4096, 8192, 16384, 4099],  # every tile kind, general lengths beside them
+    [10007] * 5 + [64] * 130 + [128] * 3 + [2048] * 2,             # lanes that leave remainders in a tile
+    [100, 210, 997],                                              # nothing for the compile-time engine
+])
+def test_uneven_batches(afc, cuda, precision, lengths):
+    import torch
+    rng = np.random.default_rng(len(lengths))
+    plan = afc.BatchPlan(lengths, precision=precision)
+    cdt = np.complex128 if precision == "f64" else np.complex64
+    x = (rng.standard_normal(plan.total) + 1j * rng.standard_normal(plan.total)).astype(cdt)
+    t = torch.from_numpy(x).to(cuda)
+    for inverse in (False, True):
+        f = np.fft.ifft if inverse else np.fft.fft
+        ref = np.concatenate([f(x[o:o + n].astype(np.complex128)) for o, n in zip(plan.offsets, plan.lengths)])
+        for mode in (0, 0, 1, 2):  # mode 0 twice: direct, then its graph
+            out = plan.execute(t, inverse=inverse, mode=mode).cpu().numpy()
+            for o, n in zip(plan.offsets, plan.lengths):
+                assert rel(out[o:o + n], ref[o:o + n]) < TOL[precision], (mode, int(n))
+    z = t.clone()
+    plan.execute(z, out=z, mode=2)
+    assert torch.equal(z, plan.execute(t, mode=2))
