@@ -7,6 +7,7 @@ from __future__ import annotations
 import os
 import subprocess
 import sys
+from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
@@ -35,14 +36,17 @@ def build(force: bool = False, verbose: bool = False) -> str:
     if not force and not _stale():
         return LIB
     os.makedirs(OUT_DIR, exist_ok=True)
-    objs = []
-    for src in SOURCES:
-        obj = os.path.join(OUT_DIR, src.replace(".cu", ".o"))
+    objs = [os.path.join(OUT_DIR, src.replace(".cu", ".o")) for src in SOURCES]
+
+    def compile_one(src: str, obj: str) -> None:
         cmd = [NVCC, *FLAGS, "-dc", "-c", os.path.join(CSRC, src), "-o", obj]
         if verbose:
-            print(" ".join(cmd))
+            print(" ".join(cmd), flush=True)
         subprocess.run(cmd, check=True)
-        objs.append(obj)
+
+    # the sources are independent until the device link: a minute or two each, side by side
+    with ThreadPoolExecutor(max_workers=max(1, min(len(SOURCES), os.cpu_count() or 1))) as pool:
+        list(pool.map(compile_one, SOURCES, objs))
     link = [NVCC, "-gencode", "arch=compute_100a,code=sm_100a", "-shared", "-ccbin", "/usr/bin/g++",
             *objs, "-o", LIB, "-lcudart"]
     if verbose:

@@ -396,22 +396,50 @@ struct AxisPlan {
   int64_t M = 0;                     // convolution length
   bool conv_smem = true;
   void* chirp = nullptr;
-  void* spec_f = nullptr;
+  void* spec_f = nullptr;            // kernel spectra of both directions (one allocation, spec_i behind spec_f)
   void* spec_i = nullptr;
-  void* spec_rf = nullptr;           // large Bluestein: spectra in row-major [k1][k2] order
+  void* spec_rf = nullptr;           // large Bluestein: the same in row-major [k1][k2] order
   void* spec_ri = nullptr;
   int* gather = nullptr;
   int* scatter = nullptr;
-  std::unique_ptr<AxisPlan> sub;     // four-step plan of length M (large Bluestein)
+  std::shared_ptr<AxisPlan> sub;     // four-step plan of length M (large Bluestein), shared within a batch plan
   int tuned_P = 0, tuned_L = 0;      // autotuned tile shape (batch plans)
   ~AxisPlan() {
-    void* ptrs[] = {lp.tw, lp1.tw, lp2.tw, tw_hi, tw_lo, fx_a, chirp, spec_f, spec_i, spec_rf, spec_ri, gather, scatter};
+    void* ptrs[] = {lp.tw, lp1.tw, lp2.tw, tw_hi, tw_lo, fx_a, chirp, spec_f, spec_rf, gather, scatter};
     for (void* p : ptrs)
       if (p) cudaFree(p);
   }
 };
 
 static afc_status build_axis(int64_t n, bool dbl, AxisPlan& ap, cudaStream_t st);
+
+// What the plans of one batch share while they are built: the two-pass plan of
+// each convolution length, and one scratch allocation for table FFTs (each was
+// allocated, waited for and freed per table).
+struct BuildShare {
+  std::map<int64_t, std::shared_ptr<AxisPlan>> sub;
+  void* scratch = nullptr;
+  size_t bytes = 0;
+  ~BuildShare() {
+    if (scratch) cudaFree(scratch);
+  }
+  // at least `need` bytes, or null; work already enqueued on the stream has
+  // finished with the old block before it is freed (cudaFree waits)
+  void* get(size_t need) {
+    if (need <= bytes) return scratch;
+    if (scratch) cudaFree(scratch);
+    scratch = nullptr;
+    bytes = 0;
+    if (dev_alloc(&scratch, need) != cudaSuccess) {
+      cudaGetLastError();
+      scratch = nullptr;
+      return nullptr;
+    }
+    bytes = need;
+    return scratch;
+  }
+};
+static thread_local BuildShare* tl_share = nullptr;
 
 // One device word per device that bounded waits in the kernels set on timeout.
 static std::mutex g_err_mu;
@@ -966,11 +994,16 @@ static afc_status fft_table(const AxisPlan& mp, bool dbl, void* buf, cudaStream_
   io.im = LaneMap{1, 1, mp.n, 0, 0, 1, nullptr};
   io.om = io.im;
   void* ws = nullptr;
-  size_t wsb = axis_ws_bytes(mp, 1, csz);
-  if (wsb) AFC_CUDA(dev_alloc(&ws, wsb), "table workspace");
+  const size_t wsb = axis_ws_bytes(mp, 1, csz);
+  // within a batch plan's build the scratch is kept and the stream orders its uses
+  const bool own = !tl_share;
+  if (wsb) {
+    if (own) AFC_CUDA(dev_alloc(&ws, wsb), "table workspace");
+    else if (!(ws = tl_share->get(wsb))) return fail(AFC_ERR_OUT_OF_MEMORY, "table workspace: out of memory");
+  }
   cudaError_t e = exec_axis(mp, dbl, false, io, ws, st);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  if (ws) cudaFree(ws);
+  if (e == cudaSuccess && own) e = cudaStreamSynchronize(st);
+  if (ws && own) cudaFree(ws);
   if (e != cudaSuccess) return cuda_fail(e, "table FFT");
   return AFC_OK;
 }
@@ -1080,8 +1113,8 @@ static afc_status build_axis(int64_t n, bool dbl, AxisPlan& ap, cudaStream_t st)
     AFC_CUDA(dev_alloc((void**)&ap.scatter, L * sizeof(int)), "Rader maps");
     AFC_CUDA(cudaMemcpyAsync(ap.gather, gat.data(), L * sizeof(int), cudaMemcpyHostToDevice, st), "Rader maps");
     AFC_CUDA(cudaMemcpyAsync(ap.scatter, sca.data(), L * sizeof(int), cudaMemcpyHostToDevice, st), "Rader maps");
-    AFC_CUDA(dev_alloc(&ap.spec_f, (size_t)M * csz), "Rader spectrum");
-    AFC_CUDA(dev_alloc(&ap.spec_i, (size_t)M * csz), "Rader spectrum");
+    AFC_CUDA(dev_alloc(&ap.spec_f, 2 * (size_t)M * csz), "Rader spectrum");
+    ap.spec_i = static_cast<char*>(ap.spec_f) + (size_t)M * csz;
     AFC_CUDA(gen_rader_b_dev(ap.spec_f, ap.scatter, n, M, false, dbl, st), "Rader kernel");
     AFC_CUDA(gen_rader_b_dev(ap.spec_i, ap.scatter, n, M, true, dbl, st), "Rader kernel");
     AxisPlan mp;
@@ -1099,8 +1132,8 @@ static afc_status build_axis(int64_t n, bool dbl, AxisPlan& ap, cudaStream_t st)
   ap.M = M;
   AFC_CUDA(dev_alloc(&ap.chirp, (size_t)n * csz), "chirp");
   AFC_CUDA(gen_chirp_dev(ap.chirp, n, dbl, st), "chirp");
-  AFC_CUDA(dev_alloc(&ap.spec_f, (size_t)M * csz), "Bluestein spectrum");
-  AFC_CUDA(dev_alloc(&ap.spec_i, (size_t)M * csz), "Bluestein spectrum");
+  AFC_CUDA(dev_alloc(&ap.spec_f, 2 * (size_t)M * csz), "Bluestein spectrum");
+  ap.spec_i = static_cast<char*>(ap.spec_f) + (size_t)M * csz;
   AFC_CUDA(gen_bluestein_b_dev(ap.spec_f, ap.chirp, n, M, false, dbl, st), "Bluestein kernel");
   AFC_CUDA(gen_bluestein_b_dev(ap.spec_i, ap.chirp, n, M, true, dbl, st), "Bluestein kernel");
   afc_status s;
@@ -1120,16 +1153,21 @@ static afc_status build_axis(int64_t n, bool dbl, AxisPlan& ap, cudaStream_t st)
     return s;
   }
   ap.conv_smem = false;
-  ap.sub.reset(new AxisPlan());
-  ap.sub->n = M;
-  s = build_fourstep(M, dbl, *ap.sub, st);
-  if (s != AFC_OK) return s;
+  if (tl_share && tl_share->sub.count(M)) {
+    ap.sub = tl_share->sub[M];
+  } else {
+    ap.sub.reset(new AxisPlan());
+    ap.sub->n = M;
+    s = build_fourstep(M, dbl, *ap.sub, st);
+    if (s != AFC_OK) return s;
+    if (tl_share) tl_share->sub[M] = ap.sub;
+  }
   s = fft_table(*ap.sub, dbl, ap.spec_f, st);
   if (s == AFC_OK) s = fft_table(*ap.sub, dbl, ap.spec_i, st);
   if (s != AFC_OK) return s;
   // the fused middle pass reads each row k1 of the spectrum contiguously
-  AFC_CUDA(dev_alloc(&ap.spec_rf, (size_t)M * csz), "Bluestein spectrum");
-  AFC_CUDA(dev_alloc(&ap.spec_ri, (size_t)M * csz), "Bluestein spectrum");
+  AFC_CUDA(dev_alloc(&ap.spec_rf, 2 * (size_t)M * csz), "Bluestein spectrum");
+  ap.spec_ri = static_cast<char*>(ap.spec_rf) + (size_t)M * csz;  // same allocation
   AFC_CUDA(gen_row_spectrum_dev(ap.spec_rf, ap.spec_f, ap.sub->N1, ap.sub->N2, dbl, st), "Bluestein spectrum");
   AFC_CUDA(gen_row_spectrum_dev(ap.spec_ri, ap.spec_i, ap.sub->N1, ap.sub->N2, dbl, st), "Bluestein spectrum");
   return AFC_OK;
@@ -1784,7 +1822,8 @@ struct BatchGroup {
   int64_t n = 0;
   long long lanes = 0;
   std::unique_ptr<AxisPlan> ap;
-  long long* d_off = nullptr;  // device lane offsets (packed layout)
+  std::vector<long long> off;  // lane offsets (packed layout)
+  long long* d_off = nullptr;  // the same on the device
   size_t ws_off = 0;           // this group's workspace region (groups of a phase run concurrently)
   ~BatchGroup() {
     if (d_off) cudaFree(d_off);
@@ -1994,7 +2033,7 @@ static void tune_group(BatchGroup& g, bool dbl, void* scratch, cudaStream_t st) 
 // first one: far enough that the tiles in flight rarely wait, close enough that
 // the intermediates stay in L2.  Single-tile transforms fill the drain.
 struct FxAcc {
-  static constexpr double kLag = 1800;  // three to four tiles for each CTA in flight
+  static constexpr double kLag = 1800;  // three tiles for each CTA in flight (600 / 1800 / 4000: 1345 / 1287 / 1288 us)
   struct Multi {
     long long tiles;  // all passes of one transform
     std::vector<FxBatchItem> items;
@@ -2005,12 +2044,20 @@ struct FxAcc {
   std::vector<std::pair<double, FxBatchItem>> single;  // cost, tile
   int ndesc = 0, ndep = 0;
 
-  void add(const std::vector<RecLaunch>& launches, long long lanes, bool dbl) {
+  // off: the lanes' element offsets in the packed batch
+  void add(const std::vector<RecLaunch>& launches, const std::vector<long long>& off, bool dbl) {
     const size_t ksz = kargs_size(dbl);
+    const long long lanes = (long long)off.size(), csz = dbl ? 16 : 8;
     std::vector<Multi> grp(launches.size() > 1 ? lanes : 0);
     for (auto& m : grp) m.tiles = 0;
     for (size_t k = 0; k < launches.size(); ++k) {
-      const LaunchDesc& d = launches[k].d;
+      LaunchDesc d = launches[k].d;
+      // a pass of a long transform: the tile's entry carries its transform's
+      // offset instead of a table lookup per thread
+      const bool multi_pass = launches.size() > 1;
+      const bool ioff = multi_pass && d.im.off, ooff = multi_pass && d.om.off;
+      if (ioff) d.im.off = nullptr;
+      if (ooff) d.om.off = nullptr;
       const int di = ndesc++;
       descs.resize((size_t)ndesc * ksz);
       kargs_pack(d, dbl, descs.data() + (size_t)di * ksz);
@@ -2019,7 +2066,7 @@ struct FxAcc {
       if (launches.size() == 1) {
         const double c = d.sl.nst * (d.fx_mode == FX_CONV ? 2.0 : 1.0);
         for (long long t = 0; t < tiles; ++t)
-          single.emplace_back(c, FxBatchItem{di, kind, (unsigned)(t * L), 0, 0, {}});
+          single.emplace_back(c, FxBatchItem{di, kind, (unsigned)(t * L), 0, 0, 0, 0, {}});
         continue;
       }
       // pass k of lane i covers sub-lanes [i per, (i + 1) per), a multiple of L
@@ -2028,7 +2075,8 @@ struct FxAcc {
         Multi& m = grp[i];
         const long long before = m.tiles;
         for (long long q = i * per; q < (i + 1) * per; q += L) {
-          m.items.push_back(FxBatchItem{di, kind, (unsigned)q, (int)(1 + ndep + i), (int)before, {}});
+          m.items.push_back(FxBatchItem{di, kind, (unsigned)q, (int)(1 + ndep + i), (int)before,
+                                        ioff ? off[i] * csz : 0, ooff ? off[i] * csz : 0, {}});
           m.pass.push_back((int)k);
           ++m.tiles;
         }
@@ -2114,7 +2162,7 @@ static afc_status build_phases(afc_batch_plan_s& bp, bool inv, cudaStream_t st) 
     if (e == cudaSuccess && std::all_of(rec.launches.begin(), rec.launches.end(),
                                         [](const RecLaunch& r) { return r.d.fx_form >= 0; })) {
       tl_rec = nullptr;
-      fxa.add(rec.launches, g->lanes, bp.dbl);
+      fxa.add(rec.launches, g->off, bp.dbl);
       continue;
     }
     if (e == cudaSuccess && std::any_of(rec.launches.begin(), rec.launches.end(),
@@ -3288,11 +3336,14 @@ afc_status afc_batch_plan_create(afc_batch_plan* out, const int64_t* lengths, in
   afc_status s = AFC_OK;
   // single-CTA lengths of a batch keep several persistent CTAs per SM
   tl_smem_cap = batch_smem_cap(bp->dbl);
+  BuildShare share;
+  tl_share = &share;
   int64_t max_smem_len = 1;
   for (auto& kv : by_len) {
     std::unique_ptr<BatchGroup> grp(new BatchGroup());
     grp->n = kv.first;
     grp->lanes = (long long)kv.second.size();
+    grp->off = kv.second;
     grp->ap.reset(new AxisPlan());
     s = build_axis(kv.first, bp->dbl, *grp->ap, st);
     if (s != AFC_OK) break;
@@ -3305,6 +3356,7 @@ afc_status afc_batch_plan_create(afc_batch_plan* out, const int64_t* lengths, in
     bp->ws_bytes += (axis_ws_bytes(*grp->ap, grp->lanes, csz) + 255) / 256 * 256;
     bp->groups.push_back(std::move(grp));
   }
+  tl_share = nullptr;
   if (s == AFC_OK) {
     cudaError_t e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) s = cuda_fail(e, "batch plan build");

@@ -220,16 +220,14 @@ template <class T> __device__ __forceinline__ unsigned fx_col(const KArgs<T>& a,
 // HALF (chirp operators): the valid inputs and the kept outputs all lie in the
 // lower half of the lane, as in every Bluestein convolution (n <= M / 2), so
 // points q >= 8 are never loaded nor stored.
-// `in` / `out` are the launch's buffers (a batch resolves them per tile).  Plain
-// complex data are read through L2: each point is read once, and a batch tile
+// Plain complex data are read through L2: each point is read once, and a batch tile
 // may read what another CTA of the same launch wrote.
 // IN: IN_C (also IN_R, and IN_HERM on contiguous lanes), IN_FRAME, IN_CHIRP
 // (also IN_CHIRP_R), IN_STEP; OUT: OUT_C (also OUT_RE; on contiguous lanes
 // OUT_TRUNC and the first store_cols points; on strided lanes the mirrored
 // columns of a Hermitian pass), OUT_STEP, OUT_CHIRP (also OUT_CHIRP_RE).
 template <class T, int N, int L, int FORM, int MODE, int IN, int OUT, bool HALF = false>
-__device__ __forceinline__ void fx_tile(const KArgs<T>& a, const void* in, void* out, unsigned q0,
-                                        typename CT<T>::type* sm) {
+__device__ __forceinline__ void fx_tile(const KArgs<T>& a, unsigned q0, typename CT<T>::type* sm) {
   using C = typename CT<T>::type;
   using E = FxEng<T, N>;
   constexpr int P = E::P, EP = E::EP;
@@ -249,12 +247,12 @@ __device__ __forceinline__ void fx_tile(const KArgs<T>& a, const void* in, void*
     const long long es = FORM == FX_COLS ? a.im.es : 1;
     if constexpr (IN == IN_C) {
       if (a.in_op == IN_R) {
-        const T* p = static_cast<const T*>(in) + ib + tA * es;
+        const T* p = static_cast<const T*>(a.in) + ib + tA * es;
 #pragma unroll
         for (int q = 0; q < EP; ++q) v[q] = C{p[(long long)(P * q) * es], (T)0};
       } else if (FORM == FX_ROWS && a.in_op == IN_HERM) {
         // half spectrum (N / 2 + 1 bins) expanded by Hermitian symmetry
-        const C* p = static_cast<const C*>(in) + ib;
+        const C* p = static_cast<const C*>(a.in) + ib;
 #pragma unroll
         for (int q = 0; q < EP; ++q) {
           const int i = tA + P * q;
@@ -265,13 +263,13 @@ __device__ __forceinline__ void fx_tile(const KArgs<T>& a, const void* in, void*
           v[q] = x;
         }
       } else {
-        const C* p = static_cast<const C*>(in) + ib + tA * es;
+        const C* p = static_cast<const C*>(a.in) + ib + tA * es;
 #pragma unroll
         for (int q = 0; q < EP; ++q) v[q] = __ldcg(p + (long long)(P * q) * es);
       }
     } else if constexpr (IN == IN_FRAME) {
       const long long s = ib - a.frame_off + tA;
-      const T* p = static_cast<const T*>(in) + s;
+      const T* p = static_cast<const T*>(a.in) + s;
       const T* w = a.window + tA;
       if (s - tA >= 0 && s - tA + N <= a.nlen) {
 #pragma unroll
@@ -297,7 +295,7 @@ __device__ __forceinline__ void fx_tile(const KArgs<T>& a, const void* in, void*
         C x = C{(T)0, (T)0};
         if (j < nlen) {
           const long long o = o0 + (long long)(P * q) * es;
-          x = re ? C{static_cast<const T*>(in)[o], (T)0} : static_cast<const C*>(in)[o];
+          x = re ? C{static_cast<const T*>(a.in)[o], (T)0} : static_cast<const C*>(a.in)[o];
           const C c = __ldg(a.chirp + j);
           x = cj ? cmulc(x, c) : cmul(x, c);
         }
@@ -306,7 +304,7 @@ __device__ __forceinline__ void fx_tile(const KArgs<T>& a, const void* in, void*
     } else {  // IN_STEP: times the conjugate step twiddle of (column, tA + P q)
       const unsigned cm = (unsigned)a.col_mod;
       const unsigned col = fx_col(a, qA);
-      const C* p = static_cast<const C*>(in) + ib + tA * es;
+      const C* p = static_cast<const C*>(a.in) + ib + tA * es;
 #pragma unroll
       for (int q = 0; q < EP; ++q) v[q] = __ldcg(p + (long long)(P * q) * es);
       const C wa = __ldg(a.fx_a + (unsigned)tA * cm + col);
@@ -338,12 +336,12 @@ __device__ __forceinline__ void fx_tile(const KArgs<T>& a, const void* in, void*
   const T sc = a.scale;
   if constexpr (OUT == OUT_C) {
     if (a.out_op == OUT_RE) {
-      T* p = static_cast<T*>(out) + ob;
+      T* p = static_cast<T*>(a.out) + ob;
 #pragma unroll
       for (int q = 0; q < EP; ++q) p[(long long)(P * q) * es] = v[q].x * sc;
     } else if (FORM == FX_ROWS && a.store_cols > 0) {
       // the first store_cols points (OUT_TRUNC: a half spectrum, paired bins weighted)
-      C* p = static_cast<C*>(out) + ob;
+      C* p = static_cast<C*>(a.out) + ob;
       const T pw = a.out_op == OUT_TRUNC ? sc * a.pair_w : sc;
 #pragma unroll
       for (int q = 0; q < EP; ++q) {
@@ -351,7 +349,7 @@ __device__ __forceinline__ void fx_tile(const KArgs<T>& a, const void* in, void*
         if (i < a.store_cols) p[P * q] = cscale(v[q], i > 0 && 2 * i != N ? pw : sc);
       }
     } else {
-      C* p = static_cast<C*>(out) + ob;
+      C* p = static_cast<C*>(a.out) + ob;
 #pragma unroll
       for (int q = 0; q < EP; ++q) p[(long long)(P * q) * es] = cscale(v[q], sc);
       if (FORM == FX_COLS && a.hm_cmax > 0) {
@@ -359,7 +357,7 @@ __device__ __forceinline__ void fx_tile(const KArgs<T>& a, const void* in, void*
         // read backwards, Y[k][es - c] = conj(Y[(N - k) mod N][c])
         const int c = (int)(qB % (unsigned)a.om.d2);
         if (c >= 1 && c <= a.hm_cmax) {
-          C* m = static_cast<C*>(out) + fx_base(a.om, qB, a.fx_sh[0] >= 0 ? a.fx_sh[1] : -1) + a.om.es - 2 * c;
+          C* m = static_cast<C*>(a.out) + fx_base(a.om, qB, a.fx_sh[0] >= 0 ? a.fx_sh[1] : -1) + a.om.es - 2 * c;
 #pragma unroll
           for (int q = 0; q < EP; ++q) {
             const int k = tB + P * q;
@@ -373,7 +371,7 @@ __device__ __forceinline__ void fx_tile(const KArgs<T>& a, const void* in, void*
     const unsigned cm = (unsigned)a.col_mod;
     const unsigned col = fx_col(a, qB);
     const bool cj = a.tw_conj != 0;
-    C* p = static_cast<C*>(out) + ob;
+    C* p = static_cast<C*>(a.out) + ob;
     const C wa = __ldg(a.fx_a + (unsigned)tB * cm + col);
 #pragma unroll
     for (int q = 0; q < EP; ++q) {
@@ -394,8 +392,8 @@ __device__ __forceinline__ void fx_tile(const KArgs<T>& a, const void* in, void*
         const C c = __ldg(ch + j);
         const C y = cscale(cj ? cmulc(v[q], c) : cmul(v[q], c), sc);
         const long long o = ob + (long long)(P * q) * es;
-        if (re) static_cast<T*>(out)[o] = y.x;
-        else static_cast<C*>(out)[o] = y;
+        if (re) static_cast<T*>(a.out)[o] = y.x;
+        else static_cast<C*>(a.out)[o] = y;
       }
     }
   }
@@ -412,7 +410,7 @@ template <class T, int N, int FORM> struct FxTile {
   static constexpr bool P2 = fx_pow2(N);
   static constexpr int base = FORM == FX_ROWS && P2 ? 128 : 256;
   static constexpr int wide = sizeof(T) == 8 ? 8 : 16;  // 128-byte rows
-  static constexpr int minL = FORM == FX_ROWS ? 1 : P2 ? wide / 2 : wide * P <= 512 ? wide : 8;
+  static constexpr int minL = FORM == FX_ROWS ? 1 : P2 ? (N > 1024 ? wide / 4 : wide / 2) : wide * P <= 512 ? wide : 8;
   static constexpr int L = FORM != FX_ROWS && !P2 ? minL : base / P > minL ? base / P : minL;
   static constexpr int threads = L * P;
   static constexpr size_t smem =

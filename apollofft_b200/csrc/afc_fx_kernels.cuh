@@ -13,7 +13,8 @@ namespace afc {
 // odd lengths hold at most 10 points: 1024 threads of 64 registers.
 template <class T, int N> constexpr int fx_min_ctas(int threads) {
   if (!fx_pow2(N)) return (sizeof(T) == 4 ? 1024 : 512) / ((threads + 31) / 32 * 32);
-  return threads > 256 ? 1 : (sizeof(T) == 4 ? 3 : 2) * (256 / threads);
+  if (threads > 256) return sizeof(T) == 4 ? 2 : 1;
+  return (sizeof(T) == 4 ? 3 : 2) * (256 / threads);
 }
 
 template <class T, int N, int FORM, int MODE, int IN, int OUT, bool HALF>
@@ -25,7 +26,7 @@ __global__ void __launch_bounds__(FxTile<T, N, FORM>::threads, fx_min_ctas<T, N>
   // the previous launch drains; nothing is read before that one has completed
   griddep_wait();
   griddep_launch_dependents();
-  fx_tile<T, N, L, FORM, MODE, IN, OUT, HALF>(a, a.in, a.out, blockIdx.x * (unsigned)L,
+  fx_tile<T, N, L, FORM, MODE, IN, OUT, HALF>(a, blockIdx.x * (unsigned)L,
                                        reinterpret_cast<typename CT<T>::type*>(smraw));
 }
 
@@ -54,6 +55,8 @@ template <class T, int FORM, int MODE, int IN, int OUT, bool HALF = false> stati
     if (n == 2048) return fx_entry<T, 2048, FORM, MODE, IN, OUT, HALF>();
     if (n == 4096) return fx_entry<T, 4096, FORM, MODE, IN, OUT, HALF>();
   }
+  if constexpr (FORM == FX_COLS && IN == IN_C && OUT == OUT_C && sizeof(T) == 4)
+    if (n == 2048) return fx_entry<T, 2048, FORM, MODE, IN, OUT, HALF>();
   if constexpr (FORM != FX_ROWS_T && MODE != FX_CONV && IN == IN_C && OUT == OUT_C) {
     if (n == 243) return fx_entry<T, 243, FORM, MODE, IN, OUT, HALF>();
     if (n == 250) return fx_entry<T, 250, FORM, MODE, IN, OUT, HALF>();
@@ -160,69 +163,104 @@ template <class T> static cudaError_t launch_fx_t(const LaunchDesc& d, cudaStrea
 constexpr int kFxBatchThreads = 256;
 
 template <class T, int N, int FORM, int MODE, int IN, int OUT>
-__device__ __forceinline__ void fx_batch_tile(const KArgs<T>& a, const void* in, void* out, unsigned q0,
-                                              unsigned char* sm) {
-  fx_tile<T, N, 4096 / N, FORM, MODE, IN, OUT, IN == IN_CHIRP || OUT == OUT_CHIRP>(a, in, out, q0, reinterpret_cast<typename CT<T>::type*>(sm));
+__device__ __forceinline__ void fx_batch_tile(const KArgs<T>& a, unsigned q0, unsigned char* sm) {
+  fx_tile<T, N, 4096 / N, FORM, MODE, IN, OUT, IN == IN_CHIRP || OUT == OUT_CHIRP>(
+      a, q0, reinterpret_cast<typename CT<T>::type*>(sm));
 }
 
+__device__ __forceinline__ void fx_cp16(void* smem, const void* gmem) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(smem_u32(smem)), "l"(gmem) : "memory");
+}
+
+// Long lists (deep): the claims of a CTA run three tiles ahead; while tile i
+// runs, the descriptor of tile i + 1, the list entry of tile i + 2 and the claim
+// of tile i + 3 are on their way, so none of the three dependent fetches is
+// waited for.  Short lists claim one tile at a time, which balances them better.
+// Descriptors are read from shared memory, field by field where they are used
+// (read through a global pointer the compiler kept them in registers across the
+// tile and spilled 1.7 KB; now 64 bytes, and complex64 fits four CTAs per SM:
+// 4096 uneven transforms 1238 us at three, 1177 us at four).
 template <class T, bool INV>
-__global__ void __launch_bounds__(kFxBatchThreads, sizeof(T) == 4 ? 3 : 2)
+__global__ void __launch_bounds__(kFxBatchThreads, sizeof(T) == 4 ? 4 : 2)
     fx_batch_kernel(const KArgs<T>* __restrict__ descs, const FxBatchItem* __restrict__ items, int nitems, int* ctr,
-                    const void* in_base, void* out_base, void* ws_base, unsigned* err) {
+                    const void* in_base, void* out_base, void* ws_base, unsigned* err, int deep) {
   extern __shared__ __align__(16) unsigned char smraw[];
-  __shared__ __align__(16) FxBatchItem s_item[2];
-  __shared__ int s_idx[2];
+  __shared__ __align__(16) KArgs<T> s_ka[2];
+  __shared__ __align__(16) FxBatchItem s_item[3];
+  __shared__ int s_idx[3];
+  static_assert(sizeof(KArgs<T>) % 16 == 0 && sizeof(FxBatchItem) % 16 == 0, "copied 16 bytes at a time");
+  constexpr int KW = (int)sizeof(KArgs<T>) / 16, IW = (int)sizeof(FxBatchItem) / 16;
   const int tid = threadIdx.x;
   constexpr int DIR = INV ? FX_INV : FX_FWD;
-  // nothing of the loop but one claim lives in registers while a tile runs: the
-  // current list entry is [p], the next one arrives in [p ^ 1] meanwhile
+  auto copy_desc = [&](int slot, int item) {
+    const char* src = reinterpret_cast<const char*>(descs + s_item[item].desc);
+    if (tid < KW) fx_cp16(reinterpret_cast<char*>(&s_ka[slot]) + 16 * tid, src + 16 * tid);
+  };
+  // thread 0, once the copy has landed: buffer selectors become pointers
+  auto resolve = [&](int slot, int item) {
+    KArgs<T>& k = s_ka[slot];
+    char* bases[4] = {nullptr, (char*)in_base, (char*)out_base, (char*)ws_base};
+    k.in = bases[k.in_sel] + (size_t)k.in + s_item[item].in_off;
+    k.out = bases[k.out_sel] + (size_t)k.out + s_item[item].out_off;
+  };
   if (tid == 0) {
+    // one claim after the other: a CTA runs its claims in list order
     s_idx[0] = atomicAdd(ctr, 1);
-    s_idx[1] = atomicAdd(ctr, 1);
     s_item[0] = items[min(s_idx[0], nitems - 1)];
+    if (deep) {
+      s_idx[1] = atomicAdd(ctr, 1);
+      s_item[1] = items[min(s_idx[1], nitems - 1)];
+      s_idx[2] = atomicAdd(ctr, 1);
+    }
   }
   __syncthreads();
-  for (int p = 0; s_idx[p] < nitems; p ^= 1) {
-    const FxBatchItem& bi = s_item[p];
+  copy_desc(0, 0);
+  asm volatile("cp.async.wait_all;\n" ::: "memory");
+  __syncthreads();
+  if (tid == 0) resolve(0, 0);
+  __syncthreads();
+  for (int i = 0;; ++i) {
+    const int c0 = i % 3, c1 = (i + 1) % 3, c2 = (i + 2) % 3, ks = i & 1;
+    if (s_idx[c0] >= nitems) break;
     int nx = 0;
-    if (tid == 0) {
-      const FxBatchItem* src = items + min(s_idx[p ^ 1], nitems - 1);
-      const unsigned dst = smem_u32(&s_item[p ^ 1]);
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src) : "memory");
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst + 16), "l"(reinterpret_cast<const char*>(src) + 16) : "memory");
+    if (deep) copy_desc(ks ^ 1, c1);
+    if (deep && tid == 0) {
+      const char* src = reinterpret_cast<const char*>(items + min(s_idx[c2], nitems - 1));
+#pragma unroll
+      for (int w = 0; w < IW; ++w) fx_cp16(reinterpret_cast<char*>(&s_item[c2]) + 16 * w, src + 16 * w);
       nx = atomicAdd(ctr, 1);
     }
-    if (bi.wait > 0) {  // the passes before this one, of the same transform
+    if (s_item[c0].wait > 0) {  // the passes before this one, of the same transform
       bool ok = true;
       if (tid == 0) {
-        const volatile int* c = ctr + bi.dep;
+        const volatile int* c = ctr + s_item[c0].dep;
+        const int want = s_item[c0].wait;
         int k = 0;
-        while (*c < bi.wait && k < (1 << 22)) {
+        while (*c < want && k < (1 << 22)) {
           __nanosleep(64);
           ++k;
         }
-        ok = *c >= bi.wait;
+        ok = *c >= want;
         __threadfence();
       }
       if (__syncthreads_or(!ok)) {
-        if (tid == 0) atomicExch(err, 1u);
+        if (tid == 0) {
+          atomicExch(err, 1u);
+        }
+        asm volatile("cp.async.wait_all;\n" ::: "memory");
         return;
       }
     }
-    const KArgs<T>& a = descs[bi.desc];
-    const char* bases[4] = {nullptr, static_cast<const char*>(in_base), static_cast<const char*>(out_base),
-                            static_cast<const char*>(ws_base)};
-    const void* in = (a.in_sel == 1 ? bases[1] : a.in_sel == 2 ? bases[2] : bases[3]) + (size_t)a.in;
-    void* out = const_cast<char*>((a.out_sel == 2 ? bases[2] : a.out_sel == 1 ? bases[1] : bases[3]) + (size_t)a.out);
-    const unsigned q0 = bi.q0;
+    const KArgs<T>& a = s_ka[ks];
+    const unsigned q0 = s_item[c0].q0;
 #define AFC_FXB(OP, LG, FORM, MODE, IN, OUT) \
-  case OP * 8 + LG - 6: fx_batch_tile<T, (1 << LG), FORM, MODE, IN, OUT>(a, in, out, q0, smraw); break;
+  case OP * 8 + LG - 6: fx_batch_tile<T, (1 << LG), FORM, MODE, IN, OUT>(a, q0, smraw); break;
 #define AFC_FXB5(OP, FORM, MODE, IN, OUT)                                                                     \
   AFC_FXB(OP, 6, FORM, MODE, IN, OUT) AFC_FXB(OP, 7, FORM, MODE, IN, OUT) AFC_FXB(OP, 8, FORM, MODE, IN, OUT) \
   AFC_FXB(OP, 9, FORM, MODE, IN, OUT) AFC_FXB(OP, 10, FORM, MODE, IN, OUT)
 #define AFC_FXB7(OP, FORM, MODE, IN, OUT) \
   AFC_FXB5(OP, FORM, MODE, IN, OUT) AFC_FXB(OP, 11, FORM, MODE, IN, OUT) AFC_FXB(OP, 12, FORM, MODE, IN, OUT)
-    switch (bi.kind) {
+    switch (s_item[c0].kind) {
       AFC_FXB7(FXB_ROWS, FX_ROWS, DIR, IN_C, OUT_C)
       AFC_FXB5(FXB_COLS, FX_COLS, DIR, IN_C, OUT_STEP)
       AFC_FXB5(FXB_ROWS_T, FX_ROWS_T, DIR, IN_C, OUT_C)
@@ -235,16 +273,29 @@ __global__ void __launch_bounds__(kFxBatchThreads, sizeof(T) == 4 ? 3 : 2)
 #undef AFC_FXB7
 #undef AFC_FXB5
 #undef AFC_FXB
-    __syncthreads();  // the tile's stores are issued, its shared memory is free
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
+    __syncthreads();  // the tile's stores are issued, its shared memory is free, the copies have landed
     if (tid == 0) {
-      if (bi.dep > 0) {
+      if (s_item[c0].dep > 0) {
         __threadfence();
-        atomicAdd(ctr + bi.dep, 1);
+        atomicAdd(ctr + s_item[c0].dep, 1);
       }
-      asm volatile("cp.async.wait_all;\n" ::: "memory");
-      s_idx[p] = nx;
+      if (deep) {
+        s_idx[c0] = nx;  // tile i + 3
+        resolve(ks ^ 1, c1);
+      } else {
+        s_idx[c1] = atomicAdd(ctr, 1);
+        s_item[c1] = items[min(s_idx[c1], nitems - 1)];
+      }
     }
     __syncthreads();
+    if (!deep && s_idx[c1] < nitems) {
+      copy_desc(ks ^ 1, c1);
+      asm volatile("cp.async.wait_all;\n" ::: "memory");
+      __syncthreads();
+      if (tid == 0) resolve(ks ^ 1, c1);
+      __syncthreads();
+    }
   }
 }
 
@@ -292,9 +343,10 @@ static cudaError_t launch_fx_batch_t(const void* descs, const FxBatchItem* items
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   long long grid = (long long)sms * kernel_ctas_per_sm(reinterpret_cast<const void*>(k), kFxBatchThreads, smem);
+  const int deep = nitems >= 6 * grid;
   if (grid > nitems) grid = nitems;
   k<<<(unsigned)grid, kFxBatchThreads, smem, st>>>(static_cast<const KArgs<T>*>(descs), items, nitems, ctr, in, out, ws,
-                                                   err);
+                                                   err, deep);
   count_launch(1);
   return cudaGetLastError();
 }

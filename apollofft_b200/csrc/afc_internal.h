@@ -28,7 +28,7 @@ enum FxMode { FX_FWD = 0, FX_INV = 1, FX_CONV = 2 };
 
 // Everything one launch of the lanes / conv kernels needs (type-erased).
 struct LaunchDesc {
-  StageList sl;
+  StageList sl{};
   const void* tw = nullptr;
   long long lanes = 0;
   int L = 1, P = 1, ld = 1;
@@ -89,13 +89,14 @@ enum FxBatchOp {
 // A tile of the compile-time batch kernel: descriptor, kind, first lane, and
 // for transforms of several passes the transform's counter (index behind the
 // claim counter, 0: none) and how many of its tiles must be done first.
-struct FxBatchItem {
+struct alignas(16) FxBatchItem {
   int desc;
   int kind;
   unsigned q0;
   int dep;
   int wait;
-  int pad[3];  // 32 bytes: two 16-byte asynchronous copies
+  long long in_off, out_off;  // bytes added to the descriptor's buffers
+  int pad[2];                 // 48 bytes: three 16-byte asynchronous copies
 };
 
 // dynamic shared memory of lanes_kernel: L lanes x buffers x ld + 3 L lane descriptors

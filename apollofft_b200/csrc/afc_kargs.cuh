@@ -11,7 +11,7 @@ namespace afc {
 
 // ───────────────────────────── kernel arguments ─────────────────────────────
 
-template <class T> struct KArgs {
+template <class T> struct alignas(16) KArgs {
   using C = typename CT<T>::type;
   StageList sl;
   const C* tw;

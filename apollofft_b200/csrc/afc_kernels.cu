@@ -607,7 +607,8 @@ static std::map<std::pair<int, const void*>, size_t> g_kgrant;
 static std::map<std::tuple<int, const void*, int, size_t>, int> g_kper;
 
 cudaError_t kernel_smem_grant(const void* kern, size_t smem) {
-  if (smem <= 48 * 1024) return cudaSuccess;
+  // 48 KB without a grant, a kernel's static shared memory included
+  if (smem <= 40 * 1024) return cudaSuccess;
   int dev = 0;
   cudaGetDevice(&dev);
   const auto key = std::make_pair(dev, kern);
@@ -788,6 +789,7 @@ int fx_col_lanes(long long n, bool dbl) {
     case 256: return dbl ? FxTile<double, 256, FX_COLS>::L : FxTile<float, 256, FX_COLS>::L;
     case 512: return dbl ? FxTile<double, 512, FX_COLS>::L : FxTile<float, 512, FX_COLS>::L;
     case 1024: return dbl ? FxTile<double, 1024, FX_COLS>::L : FxTile<float, 1024, FX_COLS>::L;
+    case 2048: return dbl ? 0 : FxTile<float, 2048, FX_COLS>::L;
     case 243: return dbl ? FxTile<double, 243, FX_COLS>::L : FxTile<float, 243, FX_COLS>::L;
     case 250: return dbl ? FxTile<double, 250, FX_COLS>::L : FxTile<float, 250, FX_COLS>::L;
     case 343: return dbl ? FxTile<double, 343, FX_COLS>::L : FxTile<float, 343, FX_COLS>::L;

@@ -66,7 +66,7 @@ def test_rows(afc, cuda, precision, kind, n, batch):
 @pytest.mark.parametrize("precision", ["f64", "f32"])
 @pytest.mark.parametrize("kind", ["c2c", "r2c_full", "r2c_half"])
 @pytest.mark.parametrize("dims", [(64, 1), (64, 2), (64, 3), (128, 7), (256, 18), (512, 33), (1024, 20), (1024, 130),
-                                  (64, 256), (3, 128, 10), (256, 3, 9), (128, 64, 66), (243, 17), (250, 343), (343, 40),
+                                  (64, 256), (3, 128, 10), (256, 3, 9), (128, 64, 66), (243, 18), (250, 343), (343, 40),
                                   (5, 250, 9)])
 def test_columns(afc, cuda, precision, kind, dims):
     if kind == "r2c_half" and dims[-1] < 2:
