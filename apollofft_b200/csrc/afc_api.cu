@@ -361,11 +361,13 @@ static afc_status build_lenplan(int64_t n, bool dbl, LenPlan& lp, cudaStream_t s
   lp.ld = ld_for(n);
   lp.sl.n = (int)n;
   lp.sl.nst = (int)rad.size();
+  lp.sl.psh = (n & (n - 1)) ? 31 : 4;
   int Ns = 1, off = 0;
   for (size_t s = 0; s < rad.size(); ++s) {
     lp.sl.st[s].R = rad[s];
     lp.sl.st[s].Ns = Ns;
     lp.sl.st[s].twoff = off;
+    lp.sl.st[s].mg = Ns > 1 ? (unsigned)((((u64)1 << 32) + Ns - 1) / Ns) : 0u;
     if (Ns > 1) off += Ns * (rad[s] - 1);
     Ns *= rad[s];
   }

@@ -20,8 +20,7 @@
 // operators with index maps (chirps, gathers, twiddles, truncation) are staged
 // through shared memory by cooperative copies in the kernels.
 //
-// Shared index of element i: i + (i >> 4) (one pad element every 16 breaks the
-// stride-R bank conflicts of stage outputs).
+// Shared index of element i: i + (i >> psh), see StageList.
 #pragma once
 #include <cstdint>
 #include "afc_butterfly.cuh"
@@ -34,13 +33,36 @@ struct StageDesc {
   int R;
   int Ns;
   int twoff;  // offset (in complex elements) of this stage's twiddles, stored r-major: [(r-1) Ns + k]
+  unsigned mg;  // ceil(2^32 / Ns) for Ns > 1: j / Ns = umulhi(j, mg) while j Ns < 2^32
 };
 
 struct StageList {
   int n;
   int nst;
+  // shared index of element i: i + (i >> psh).  Powers of two: 4 (one pad
+  // element every 16 breaks the stride-R conflicts of stage outputs); other
+  // lengths start with an odd or composite radix whose outputs spread over the
+  // banks, and run unpadded (31: no element).
+  int psh;
   StageDesc st[kMaxStages];
 };
+
+// j mod Ns for a butterfly index j.
+__device__ __forceinline__ int stage_mod(int j, int Ns, unsigned mg) {
+  return Ns > 1 ? j - Ns * (int)__umulhi((unsigned)j, mg) : 0;
+}
+// Distance of r strides d in the shared layout.  For powers of two spad(i + r d)
+// splits into spad(i) + spad(r d) (i below d or both multiples of 16), and
+// unpadded lists are linear, so a butterfly's addresses are one base plus terms
+// that do not depend on the thread.
+template <bool PAD> __device__ __forceinline__ int stage_off(int r, int d) { return r * d + (PAD ? (r * d) >> 4 : 0); }
+template <bool PAD> __device__ __forceinline__ int stage_idx(int i) { return i + (PAD ? i >> 4 : 0); }
+// A stride the compiler cannot lift out of the butterfly loop: a thread runs one
+// or two butterflies per stage, and R lifted offsets cost R registers each way.
+__device__ __forceinline__ int stage_stride(int d) {
+  asm volatile("" : "+r"(d));
+  return d;
+}
 
 // Lane q -> base offset (in elements):  c = q % d2, b = (q / d2) % d1, a = q / (d1 d2),
 // base = a*s0 + b*s1 + c*s2.  Element i of the lane lives at base + i*es.
@@ -60,7 +82,7 @@ struct LaneMap {
   }
 };
 
-__host__ __device__ __forceinline__ int spad(int i) { return i + (i >> 4); }
+__host__ __device__ __forceinline__ int spad(int i, int psh) { return i + (i >> psh); }
 
 // Number of shared buffers a stage list needs per lane, given whether the
 // input is staged into shared memory and whether the output is staged out.
@@ -78,29 +100,41 @@ __host__ __device__ inline int engine_buffers(int nst, bool stage_in, bool stage
 }
 
 // One stage of one lane.  src == nullptr: read global through cx; dst ==
-// nullptr: write global through cx.
-template <int R, bool INV, class Ctx, class C>
-__device__ __forceinline__ void stage(const Ctx& cx, const C* __restrict__ src, C* __restrict__ dst, int n, int Ns,
-                                      const C* __restrict__ tw, int t, int P) {
+// nullptr: write global through cx.  Index arithmetic per butterfly, not per
+// element: a multiply for j mod Ns, one base on each side.
+template <int R, bool INV, bool PAD, class Ctx, class C>
+__device__ __forceinline__ void stage(const Ctx& cx, const C* __restrict__ src, C* __restrict__ dst, int n,
+                                      const StageDesc& sd, const C* __restrict__ tw, int t, int P) {
   const int nb = n / R;
   for (int j = t; j < nb; j += P) {
+    const int d = stage_stride(nb), Ns = stage_stride(sd.Ns);
     C v[R];
+    if (src) {
+      const C* p = src + stage_idx<PAD>(j);
 #pragma unroll
-    for (int r = 0; r < R; ++r) v[r] = src ? src[spad(j + r * nb)] : cx.gload(j + r * nb);
-    const int k = j % Ns;
+      for (int r = 0; r < R; ++r) v[r] = p[stage_off<PAD>(r, d)];
+    } else {
+#pragma unroll
+      for (int r = 0; r < R; ++r) v[r] = cx.gload(j + r * d);
+    }
+    const int k = stage_mod(j, Ns, sd.mg);
     if (Ns > 1) {
+      const C* w = tw + k;
 #pragma unroll
       for (int r = 1; r < R; ++r) {
-        const C wr = tw[(long long)(r - 1) * Ns + k];
+        const C wr = w[(r - 1) * Ns];
         v[r] = INV ? cmulc(v[r], wr) : cmul(v[r], wr);
       }
     }
     DFT<R, INV>::run(v);
     const int o = (j - k) * R + k;
+    if (dst) {
+      C* p = dst + stage_idx<PAD>(o);
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-      if (dst) dst[spad(o + r * Ns)] = v[r];
-      else cx.gstore(o + r * Ns, v[r]);
+      for (int r = 0; r < R; ++r) p[stage_off<PAD>(r, Ns)] = v[r];
+    } else {
+#pragma unroll
+      for (int r = 0; r < R; ++r) cx.gstore(o + r * Ns, v[r]);
     }
   }
 }
@@ -128,24 +162,34 @@ __device__ __forceinline__ C* run_stages(const Ctx& cx, const StageList& sl, con
     C* nxt = (last && !stage_out) ? nullptr : (cur == buf0 ? buf1 : buf0);
     const StageDesc s = sl.st[i];
     const C* twi = tw + s.twoff;
-#define AFC_ST(R) stage<R, INV>(cx, cur, nxt, sl.n, s.Ns, twi, t, P)
-    switch (s.R) {
-      case 2: AFC_ST(2); break;
-      case 3: AFC_ST(3); break;
-      case 4: AFC_ST(4); break;
-      case 5: AFC_ST(5); break;
-      case 6: AFC_ST(6); break;
-      case 7: AFC_ST(7); break;
-      case 8: AFC_ST(8); break;
-      case 9: AFC_ST(9); break;
-      case 10: AFC_ST(10); break;
-      case 12: AFC_ST(12); break;
-      case 14: AFC_ST(14); break;
-      case 15: AFC_ST(15); break;
-      case 11: AFC_ST(11); break;
-      case 13: AFC_ST(13); break;
-      case 16: AFC_ST(16); break;
-      default: break;
+#define AFC_ST(R, PAD) stage<R, INV, PAD>(cx, cur, nxt, sl.n, s, twi, t, P)
+    if (sl.psh == 4) {  // a power of two
+      switch (s.R) {
+        case 2: AFC_ST(2, true); break;
+        case 4: AFC_ST(4, true); break;
+        case 8: AFC_ST(8, true); break;
+        case 16: AFC_ST(16, true); break;
+        default: break;
+      }
+    } else {
+      switch (s.R) {
+        case 2: AFC_ST(2, false); break;
+        case 3: AFC_ST(3, false); break;
+        case 4: AFC_ST(4, false); break;
+        case 5: AFC_ST(5, false); break;
+        case 6: AFC_ST(6, false); break;
+        case 7: AFC_ST(7, false); break;
+        case 8: AFC_ST(8, false); break;
+        case 9: AFC_ST(9, false); break;
+        case 10: AFC_ST(10, false); break;
+        case 12: AFC_ST(12, false); break;
+        case 14: AFC_ST(14, false); break;
+        case 15: AFC_ST(15, false); break;
+        case 11: AFC_ST(11, false); break;
+        case 13: AFC_ST(13, false); break;
+        case 16: AFC_ST(16, false); break;
+        default: break;
+      }
     }
 #undef AFC_ST
     __syncthreads();

@@ -84,9 +84,9 @@ __device__ __forceinline__ void lanes_tile(const KArgs<T>& a, long long q0, unsi
 #pragma unroll
       for (int u = 0; u < 4; ++u) v[u] = gload(a, ib, colv, i + u * di);
 #pragma unroll
-      for (int u = 0; u < 4; ++u) dstl[spad(i + u * di)] = v[u];
+      for (int u = 0; u < 4; ++u) dstl[spad(i + u * di, a.sl.psh)] = v[u];
     }
-    for (; i < n; i += di) dstl[spad(i)] = gload(a, ib, colv, i);
+    for (; i < n; i += di) dstl[spad(i, a.sl.psh)] = gload(a, ib, colv, i);
     __syncthreads();
   } else if (a.stage_in) {
     // four independent loads in flight per thread before their shared stores
@@ -105,12 +105,12 @@ __device__ __forceinline__ void lanes_tile(const KArgs<T>& a, long long q0, unsi
       for (int u = 0; u < 4; ++u) {
         const int ee = e + u * stride;
         const int l2 = ee % lanes_here, i = ee / lanes_here;
-        sm[(long long)l2 * nbuf * ld + spad(i)] = v[u];
+        sm[(long long)l2 * nbuf * ld + spad(i, a.sl.psh)] = v[u];
       }
     }
     for (; e < total; e += stride) {
       const int l2 = e % lanes_here, i = e / lanes_here;
-      sm[(long long)l2 * nbuf * ld + spad(i)] = gload(a, lb[l2], lb[2 * L + l2], i);
+      sm[(long long)l2 * nbuf * ld + spad(i, a.sl.psh)] = gload(a, lb[l2], lb[2 * L + l2], i);
     }
     __syncthreads();
   }
@@ -122,7 +122,7 @@ __device__ __forceinline__ void lanes_tile(const KArgs<T>& a, long long q0, unsi
     const int l2 = tid % lanes_here, di = blockDim.x / lanes_here;
     const long long ob = lb[L + l2], colv = lb[2 * L + l2];
     const C* srcl = sm + (long long)l2 * nbuf * ld + off;
-    for (int i = tid / lanes_here; i < n; i += di) gstore(a, ob, colv, i, srcl[spad(i)], z);
+    for (int i = tid / lanes_here; i < n; i += di) gstore(a, ob, colv, i, srcl[spad(i, a.sl.psh)], z);
   } else if (a.stage_out) {
     // every lane ends in the same buffer slot: offset of res within its lane block
     const long long off = res ? (long long)(res - b0) : 0;
@@ -130,7 +130,7 @@ __device__ __forceinline__ void lanes_tile(const KArgs<T>& a, long long q0, unsi
     const C z = C{(T)0, (T)0};
     for (int e = tid; e < total; e += blockDim.x) {
       const int l2 = e % lanes_here, i = e / lanes_here;
-      gstore(a, lb[L + l2], lb[2 * L + l2], i, sm[(long long)l2 * nbuf * ld + off + spad(i)], z);
+      gstore(a, lb[L + l2], lb[2 * L + l2], i, sm[(long long)l2 * nbuf * ld + off + spad(i, a.sl.psh)], z);
     }
   }
 }
@@ -166,28 +166,34 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 __device__ __forceinline__ void cp_async_wait1() { asm volatile("cp.async.wait_group 1;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait0() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
 
-// element i of lane l: p[l * ls + i * is + (pad ? i >> 4 : 0)]
+// element i of lane l: p[l * ls + i * is + (i >> psh)]; padded views have is = 1
+// (StageList::psh), the linear input view psh = 31
 template <class C> struct SView {
   C* p;
-  int ls, is, pad;
-  __device__ __forceinline__ C& at(int l, int i) const { return p[l * ls + i * is + (pad ? (i >> 4) : 0)]; }
+  int ls, is, psh;
+  __device__ __forceinline__ C* base(int l, int i) const { return p + l * ls + i * is + (i >> psh); }
+  __device__ __forceinline__ int off(int r, int d) const { return r * d * is + ((r * d) >> psh); }
+  __device__ __forceinline__ C& at(int l, int i) const { return *base(l, i); }
 };
 
 template <int R, bool INV, class T>
 __device__ __forceinline__ void tstage(const KArgs<T>& a, SView<typename CT<T>::type> src, SView<typename CT<T>::type> dst,
-                                       bool to_global, long long ob, bool valid, int l, int n, int Ns,
+                                       bool to_global, long long ob, bool valid, int l, int n, const StageDesc& sd,
                                        const typename CT<T>::type* __restrict__ tw, int t, int P) {
   using C = typename CT<T>::type;
   const int nb = n / R;
   for (int j = t; j < nb; j += P) {
+    const int d0 = stage_stride(nb), Ns = stage_stride(sd.Ns);
     C v[R];
+    const C* s = src.base(l, j);
 #pragma unroll
-    for (int r = 0; r < R; ++r) v[r] = src.at(l, j + r * nb);
-    const int k = j % Ns;
+    for (int r = 0; r < R; ++r) v[r] = s[src.off(r, d0)];
+    const int k = stage_mod(j, Ns, sd.mg);
     if (Ns > 1) {
+      const C* w = tw + k;
 #pragma unroll
       for (int r = 1; r < R; ++r) {
-        const C wr = tw[(long long)(r - 1) * Ns + k];
+        const C wr = w[(r - 1) * Ns];
         v[r] = INV ? cmulc(v[r], wr) : cmul(v[r], wr);
       }
     }
@@ -195,16 +201,21 @@ __device__ __forceinline__ void tstage(const KArgs<T>& a, SView<typename CT<T>::
     const int o = (j - k) * R + k;
     if (to_global) {
       if (valid) {
+        const long long es = a.om.es, o0 = ob + (long long)o * es, st = (long long)Ns * es;
+        if (a.out_op == OUT_RE) {
+          T* d = static_cast<T*>(a.out) + o0;
 #pragma unroll
-        for (int r = 0; r < R; ++r) {
-          const long long off = ob + (long long)(o + r * Ns) * a.om.es;
-          if (a.out_op == OUT_RE) static_cast<T*>(a.out)[off] = v[r].x * a.scale;
-          else static_cast<C*>(a.out)[off] = cscale(v[r], a.scale);
+          for (int r = 0; r < R; ++r) d[r * st] = v[r].x * a.scale;
+        } else {
+          C* d = static_cast<C*>(a.out) + o0;
+#pragma unroll
+          for (int r = 0; r < R; ++r) d[r * st] = cscale(v[r], a.scale);
         }
       }
     } else {
+      C* d = dst.base(l, o);
 #pragma unroll
-      for (int r = 0; r < R; ++r) dst.at(l, o + r * Ns) = v[r];
+      for (int r = 0; r < R; ++r) d[dst.off(r, Ns)] = v[r];
     }
   }
 }
@@ -254,7 +265,8 @@ __global__ void __launch_bounds__(256) tile_kernel(const __grid_constant__ KArgs
   __syncthreads();
   tile_issue(a, bufs[0], lbi, tile * L, L, n, lm);
   cp_async_commit();
-  const SView<C> wv{work, ld, 1, 1};
+  const int psh = a.sl.psh;
+  const SView<C> wv{work, ld, 1, psh};
   for (int it = 0;; ++it) {
     const int cb = it & 1;
     const long long nxt = tile + gridDim.x;
@@ -272,8 +284,8 @@ __global__ void __launch_bounds__(256) tile_kernel(const __grid_constant__ KArgs
     const bool valid = q < a.lanes;
     const long long ob = lbo[cb * L + l];
     C* cur = bufs[cb];
-    const SView<C> inv_lin = lm ? SView<C>{cur, 1, L, 0} : SView<C>{cur, n, 1, 0};
-    const SView<C> cv{cur, ld, 1, 1};
+    const SView<C> inv_lin = lm ? SView<C>{cur, 1, L, 31} : SView<C>{cur, n, 1, 31};
+    const SView<C> cv{cur, ld, 1, psh};
     const int nst = a.sl.nst;
     if (nst == 0) {
       if (t == 0 && valid) {
@@ -288,7 +300,7 @@ __global__ void __launch_bounds__(256) tile_kernel(const __grid_constant__ KArgs
       const SView<C> src = s == 0 ? inv_lin : ((s & 1) ? wv : cv);
       const SView<C> dst = (s & 1) ? cv : wv;
       const C* twi = a.tw + sd.twoff;
-#define AFC_TS(R) tstage<R, INV, T>(a, src, dst, last, ob, valid, l, n, sd.Ns, twi, t, P)
+#define AFC_TS(R) tstage<R, INV, T>(a, src, dst, last, ob, valid, l, n, sd, twi, t, P)
       switch (sd.R) {
         case 2: AFC_TS(2); break;
         case 3: AFC_TS(3); break;
@@ -360,12 +372,12 @@ __device__ __forceinline__ void conv_tile(const KArgs<T>& a, long long q0, unsig
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         const int ee = e + u * stride;
-        sm[(long long)(ee % lanes_here) * 2 * ld + spad(ee / lanes_here)] = v[u];
+        sm[(long long)(ee % lanes_here) * 2 * ld + spad(ee / lanes_here, a.sl.psh)] = v[u];
       }
     }
     for (; e < total; e += stride) {
       const int l2 = e % lanes_here, i = e / lanes_here;
-      sm[(long long)l2 * 2 * ld + spad(i)] = gload(a, lb[l2], 0, i);
+      sm[(long long)l2 * 2 * ld + spad(i, a.sl.psh)] = gload(a, lb[l2], 0, i);
     }
   }
   __syncthreads();
@@ -389,13 +401,13 @@ __device__ __forceinline__ void conv_tile(const KArgs<T>& a, long long q0, unsig
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         const int ee = e + u * stride;
-        C* p = sm + (long long)(ee % lanes_here) * 2 * ld + off + spad(ee / lanes_here);
+        C* p = sm + (long long)(ee % lanes_here) * 2 * ld + off + spad(ee / lanes_here, a.sl.psh);
         *p = cmul(*p, w[u]);
       }
     }
     for (; e < total; e += stride) {
       const int l2 = e % lanes_here, i = e / lanes_here;
-      C* p = sm + (long long)l2 * 2 * ld + off + spad(i);
+      C* p = sm + (long long)l2 * 2 * ld + off + spad(i, a.sl.psh);
       *p = cmul(*p, a.spec[lb[2 * L + l2] * a.spec_ld + i]);
     }
   }
@@ -406,7 +418,7 @@ __device__ __forceinline__ void conv_tile(const KArgs<T>& a, long long q0, unsig
   const long long off2 = (long long)(res2 - b0);
   for (int e = tid; e < lanes_here * M; e += blockDim.x) {
     const int l2 = e % lanes_here, i = e / lanes_here;
-    gstore(a, lb[L + l2], lb[2 * L + l2], i, sm[(long long)l2 * 2 * ld + off2 + spad(i)], extra[2 * l2]);
+    gstore(a, lb[L + l2], lb[2 * L + l2], i, sm[(long long)l2 * 2 * ld + off2 + spad(i, a.sl.psh)], extra[2 * l2]);
   }
   if (rader && tid < lanes_here) {
     const C dc = cscale(cadd(extra[2 * tid], extra[2 * tid + 1]), a.scale);
@@ -764,7 +776,7 @@ template <int N> static void fx_list(StageList& sl) {
   using E = FxEng<float, N>;
   sl.n = N;
   sl.nst = E::NST;
-  for (int s = 0; s < E::NST; ++s) sl.st[s] = StageDesc{E::R(s), E::NS(s), E::twoff(s)};
+  for (int s = 0; s < E::NST; ++s) sl.st[s] = StageDesc{E::R(s), E::NS(s), E::twoff(s), 0u};
 }
 bool fx_stage_list(long long n, StageList& sl) {
   switch (n) {

@@ -86,6 +86,9 @@ __global__ void wait_probe_kernel(unsigned* err, int polls) {
 template <class C> struct TView {
   C* p;
   int ls, is, pad;
+  int psh = 31;  // out-of-place stages: element i at i is + (i >> psh) (StageList::psh; 31 in the linear views)
+  __device__ __forceinline__ C* base(int l, int i) const { return p + l * ls + i * is + (i >> psh); }
+  __device__ __forceinline__ int off(int r, int d) const { return r * d * is + ((r * d) >> psh); }
   __device__ __forceinline__ C& at(int l, int i) const { return p[l * ls + i * is + (pad ? (i >> 4) : 0)]; }
   // Elements i0 + r d (r < R) of lane l as a pointer and a fixed stride when
   // the padding term is linear in r: no padding, d a multiple of 16, or the
@@ -98,26 +101,36 @@ template <class C> struct TView {
   }
 };
 
-template <int R, bool INV, class C, class S>
-__device__ __forceinline__ void tma_stage(TView<C> src, TView<C> dst, int l, int n, int Ns, const C* __restrict__ tw,
-                                          int t, int P, bool scale_out, S sc) {
+// PAD: the power-of-two lists' padded views; the others are linear in r.
+template <int R, bool INV, bool PAD, class C, class S>
+__device__ __forceinline__ void tma_stage(TView<C> src, TView<C> dst, int l, int n, const StageDesc& sd,
+                                          const C* __restrict__ tw, int t, int P, S sc) {
   const int nb = n / R;
   for (int j = t; j < nb; j += P) {
+    const int Ns = stage_stride(sd.Ns), d0 = stage_stride(PAD ? nb : nb * src.is);
     C v[R];
+    const C* s = src.base(l, j);
 #pragma unroll
-    for (int r = 0; r < R; ++r) v[r] = src.at(l, j + r * nb);
-    const int k = j % Ns;
+    for (int r = 0; r < R; ++r) v[r] = s[PAD ? src.off(r, d0) : r * d0];
+    const int k = stage_mod(j, Ns, sd.mg);
     if (Ns > 1) {
+      const C* w = tw + k;
 #pragma unroll
       for (int r = 1; r < R; ++r) {
-        const C wr = tw[(long long)(r - 1) * Ns + k];
+        const C wr = w[(r - 1) * Ns];
         v[r] = INV ? cmulc(v[r], wr) : cmul(v[r], wr);
       }
     }
     DFT<R, INV>::run(v);
     const int o = (j - k) * R + k;
+    C* d = dst.base(l, o);
+    if (sc != (S)1) {
 #pragma unroll
-    for (int r = 0; r < R; ++r) dst.at(l, o + r * Ns) = scale_out ? cscale(v[r], sc) : v[r];
+      for (int r = 0; r < R; ++r) v[r] = cscale(v[r], sc);
+    }
+    const int d1 = stage_stride(PAD ? Ns : Ns * dst.is);
+#pragma unroll
+    for (int r = 0; r < R; ++r) d[PAD ? dst.off(r, d1) : r * d1] = v[r];
   }
 }
 
@@ -263,357 +276,29 @@ __device__ __forceinline__ void tma_issue_store(const TmaArgs<T>& a, long long t
 }
 
 // Threads per CTA and CTAs per SM each kernel build is compiled for.
-struct FixNone {
-  static constexpr int BUILD_THREADS = 0;
+template <class T, int V> struct TmaBuild {
+  static constexpr int threads = V == 2 ? 128 : 256;
+  static constexpr int ctas = threads == 128 ? 3 : (V == 3 || ((V == 1 || V == 4) && sizeof(T) == 4)) ? 2 : 1;
 };
-// FX::BUILD_THREADS > 0: a compile-time stage list built for that many threads
-// at one CTA per SM (wider strided tiles)
-template <class T, int V, class FX = FixNone> struct TmaBuild {
-  static constexpr int threads = FX::BUILD_THREADS ? FX::BUILD_THREADS
-                                 : (V == 2 || (V == 5 && sizeof(T) == 8)) ? 128
-                                                                           : 256;
-  // complex64 4096-point build: three CTAs per SM (80 registers; measured on
-  // B200 16384 x 4096 forward 255 -> 242 us against two); the complex64
-  // 256-point build gained nothing from a third CTA (256^3: 151 -> 154 us)
-  static constexpr int ctas = FX::BUILD_THREADS ? 1
-                              : threads == 128 || (V == 6 && sizeof(T) == 4)
-                                  ? 3
-                                  : (V == 3 || V == 7 || ((V == 1 || V == 4 || V == 5 || V == 8) && sizeof(T) == 4))
-                                        ? 2
-                                        : 1;
-};
-
-// n = 256 as two radix-16 stages in place, every shared-memory address a
-// compile-time offset from one per-thread base (variant 5).  The general
-// stage code computes each element's address from the runtime lane stride,
-// element stride and padding, and selects between the scaled and unscaled
-// output of every stage: on B200 that is more integer and select instructions
-// per point than FP64 ones.  Layouts as in the general path: the slot holds
-// the tile linearly (strided mode: element i of lane l at i LK + l;
-// contiguous: at 256 l + i), stage 0 writes the padded layout (element i at
-// 273 l + i + i / 16) and stage 1 writes the linear layout back.  The thread
-// (l, t) owns butterfly t < 16 of lane l in both stages.  Strided tiles hold
-// LK lanes (8 complex128 / 16 complex64).
-template <class T, bool INV, bool LM, int LK>
-__device__ __forceinline__ void stages256(const TmaArgs<T>& a, typename CT<T>::type* cur,
-                                          const typename CT<T>::type* __restrict__ twb, int l, int t) {
-  using C = typename CT<T>::type;
-  constexpr int LD = 273;                // padded lane stride of a 256-point lane
-  constexpr int S = LM ? 16 * LK : 16;   // linear layout: distance of elements t and t + 16
-  C* const lin = LM ? cur + l + t * LK : cur + l * 256 + t;
-  C v[16];
-#pragma unroll
-  for (int r = 0; r < 16; ++r) v[r] = lin[r * S];
-  __syncthreads();
-  DFT<16, INV>::run(v);
-  C* const p0 = cur + l * LD + 17 * t;  // outputs 16 t + r, no twiddles (Ns = 1)
-#pragma unroll
-  for (int r = 0; r < 16; ++r) p0[r] = v[r];
-  __syncthreads();
-  C* const p1 = cur + l * LD + t;  // inputs t + 16 r at t + 17 r
-#pragma unroll
-  for (int r = 0; r < 16; ++r) v[r] = p1[17 * r];
-  __syncthreads();
-  const C* const tw = twb + a.sl.st[1].twoff + t;  // Ns = 16: twiddle (r - 1) 16 + t
-#pragma unroll
-  for (int r = 1; r < 16; ++r) v[r] = INV ? cmulc(v[r], tw[(r - 1) * 16]) : cmul(v[r], tw[(r - 1) * 16]);
-  DFT<16, INV>::run(v);
-  const T sc = a.scale;
-  if (sc != (T)1) {
-#pragma unroll
-    for (int r = 0; r < 16; ++r) v[r] = cscale(v[r], sc);
-  }
-#pragma unroll
-  for (int r = 0; r < 16; ++r) lin[r * S] = v[r];  // outputs t + 16 r
-  __syncthreads();
-}
-
-// n = 4096 as three radix-16 stages in place on one contiguous lane per tile
-// (variant 6), addresses fixed as in stages256: thread t < 256 owns butterfly
-// t of every stage.  Stage 0 reads the linear lane (t + 256 r) and writes the
-// padded layout (element i at i + i / 16) at 16 t + r; stage 1 (Ns = 16) reads
-// t + 256 r and writes 16 (t - k) + k + 16 r with k = t mod 16; stage 2
-// (Ns = 256) reads t + 256 r and writes the linear lane at t + 256 r.
-template <class T, bool INV>
-__device__ __forceinline__ void stages4096(const TmaArgs<T>& a, typename CT<T>::type* cur,
-                                           const typename CT<T>::type* __restrict__ twb, int t) {
-  using C = typename CT<T>::type;
-  C v[16];
-  C* const lin = cur + t;
-#pragma unroll
-  for (int r = 0; r < 16; ++r) v[r] = lin[256 * r];
-  __syncthreads();
-  DFT<16, INV>::run(v);
-  C* const p0 = cur + 17 * t;
-#pragma unroll
-  for (int r = 0; r < 16; ++r) p0[r] = v[r];
-  __syncthreads();
-  C* const pin = cur + t + (t >> 4);  // padded t + 256 r: t + t / 16 + 272 r
-#pragma unroll
-  for (int r = 0; r < 16; ++r) v[r] = pin[272 * r];
-  __syncthreads();
-  const int k = t & 15;
-  const C* const tw1 = twb + a.sl.st[1].twoff + k;
-#pragma unroll
-  for (int r = 1; r < 16; ++r) v[r] = INV ? cmulc(v[r], tw1[(r - 1) * 16]) : cmul(v[r], tw1[(r - 1) * 16]);
-  DFT<16, INV>::run(v);
-  C* const p1 = cur + 272 * (t >> 4) + k;  // padded 256 (t / 16) + k + 16 r
-#pragma unroll
-  for (int r = 0; r < 16; ++r) p1[17 * r] = v[r];
-  __syncthreads();
-#pragma unroll
-  for (int r = 0; r < 16; ++r) v[r] = pin[272 * r];
-  __syncthreads();
-  const C* const tw2 = twb + a.sl.st[2].twoff + t;
-#pragma unroll
-  for (int r = 1; r < 16; ++r) v[r] = INV ? cmulc(v[r], tw2[(r - 1) * 256]) : cmul(v[r], tw2[(r - 1) * 256]);
-  DFT<16, INV>::run(v);
-  const T sc = a.scale;
-  if (sc != (T)1) {
-#pragma unroll
-    for (int r = 0; r < 16; ++r) v[r] = cscale(v[r], sc);
-  }
-#pragma unroll
-  for (int r = 0; r < 16; ++r) lin[256 * r] = v[r];
-  __syncthreads();
-}
-
-// A stage list fixed at compile time (variant 7): length N as radices R0 R1
-// [R2], P threads per lane, LK lanes per strided tile (0: contiguous lanes).
-// Each stage is the general out-of-place Stockham stage with every stride a
-// constant, and without the 16-element padding: the smooth odd lengths this
-// build serves (343 = 7^3, 243 = 9 9 3, 250 = 10 5 5) have odd or
-// non-power-of-two strides, so their shared-memory accesses do not need it.
-// Intermediate stages ping-pong between the slot and the work buffer in the
-// lane layout (element i of lane l at N l + i); contiguous tiles hold the
-// same layout, strided tiles hold element i of lane l at LK i + l.
-template <int N_, int R0_, int R1_, int R2_, int P_, int LK_> struct Fix {
-  static constexpr int BUILD_THREADS = 0;
-  static constexpr int N = N_, P = P_, LK = LK_;
-  static constexpr int NST = R2_ ? 3 : 2;
-  static constexpr int R(int s) { return s == 0 ? R0_ : s == 1 ? R1_ : R2_; }
-  static constexpr int NS(int s) { return s == 0 ? 1 : s == 1 ? R0_ : R0_ * R1_; }
-};
-
-template <class T, bool INV, class FX, int S>
-__device__ __forceinline__ void fixed_stage(const TmaArgs<T>& a, const typename CT<T>::type* src,
-                                            typename CT<T>::type* dst, const typename CT<T>::type* __restrict__ twb,
-                                            int l, int t) {
-  using C = typename CT<T>::type;
-  constexpr int N = FX::N, P = FX::P, R = FX::R(S), NS = FX::NS(S), NB = N / R, IT = (NB + P - 1) / P;
-  constexpr bool LM = FX::LK > 0, LAST = S == FX::NST - 1;
-  // intermediate lanes at an odd stride: the lanes of a strided tile sit in the
-  // same wavefront (8 complex128 / 16 complex64 lanes, one element each), and an
-  // odd stride puts them in distinct banks
-  constexpr int LDU = N | 1;
-  constexpr int SLS = S == 0 ? (LM ? 1 : N) : LDU, SIS = (S == 0 && LM) ? FX::LK : 1;
-  constexpr int DLS = LAST ? (LM ? 1 : N) : LDU, DIS = (LAST && LM) ? FX::LK : 1;
-  const C* const tw = twb + a.sl.st[S].twoff;
-  const T sc = a.scale;
-#pragma unroll
-  for (int it = 0; it < IT; ++it) {
-    const int j = t + it * P;
-    if (j < NB) {
-      C v[R];
-      const C* s = src + l * SLS + j * SIS;
-#pragma unroll
-      for (int r = 0; r < R; ++r) v[r] = s[r * NB * SIS];
-      const int k = NS == 1 ? 0 : j % NS;
-      if (NS > 1) {
-#pragma unroll
-        for (int r = 1; r < R; ++r) {
-          const C w = tw[(r - 1) * NS + k];
-          v[r] = INV ? cmulc(v[r], w) : cmul(v[r], w);
-        }
-      }
-      DFT<R, INV>::run(v);
-      if (LAST && sc != (T)1) {
-#pragma unroll
-        for (int r = 0; r < R; ++r) v[r] = cscale(v[r], sc);
-      }
-      C* d = dst + l * DLS + ((j - k) * R + k) * DIS;
-#pragma unroll
-      for (int r = 0; r < R; ++r) d[r * NS * DIS] = v[r];
-    }
-  }
-}
-
-// A power-of-two stage list fixed at compile time and run in place in the
-// slot (variant 8): length N as radices R0 R1 R2 [R3], P threads per lane
-// (a thread holds N / (R P) butterflies of a stage across its barrier), LK
-// lanes per strided tile (0: contiguous lanes, whose stage 0 may read real
-// input and whose last stage may store real parts).  The padded layout
-// (element i of lane l at LD l + i + i / 16) keeps every address a
-// compile-time offset from one per-butterfly base wherever the stage's
-// input stride N / R and output stride Ns are multiples of 16 or the
-// first stage is radix 16; elsewhere the padding term is computed per element.
-// Padded lane stride of the in-place builds: the plan's (odd) stride for
-// contiguous tiles; for strided tiles of LK lanes, whose lanes share a
-// shared-memory wavefront (128 bytes: 16 complex64 or 8 complex128 elements,
-// LK lanes x 16 / LK or 8 / LK butterflies), the first stride at least as
-// large that is congruent to (elements per wavefront) / LK, so the lanes'
-// elements fall in distinct banks.
-__host__ __device__ constexpr int fixip_ld(int n, int lk, int csz) {
-  const int ld = (n + (n - 1) / 16 + 1) | 1;
-  const int per = 128 / csz;
-  if (lk <= 1 || lk >= per) return ld;
-  const int want = per / lk;
-  int v = ld;
-  while (v % per != want) ++v;
-  return v;
-}
-
-template <int N_, int R0_, int R1_, int R2_, int R3_, int P_, int LK_> struct FixIP {
-  static constexpr int BUILD_THREADS = LK_ * P_ > 256 ? LK_ * P_ : 0;
-  static constexpr int N = N_, P = P_, LK = LK_;
-  static constexpr int NST = R3_ ? 4 : R2_ ? 3 : 2;
-  static constexpr int R(int s) { return s == 0 ? R0_ : s == 1 ? R1_ : s == 2 ? R2_ : R3_; }
-  static constexpr int NS(int s) { return s == 0 ? 1 : R(s - 1) * NS(s - 1); }
-};
-
-template <class T, bool INV, class FX, int S>
-__device__ __forceinline__ void fixed_stage_ip(const TmaArgs<T>& a, typename CT<T>::type* cur,
-                                               const typename CT<T>::type* __restrict__ twb, int l, int t) {
-  using C = typename CT<T>::type;
-  constexpr int N = FX::N, P = FX::P, LD = fixip_ld(FX::N, FX::LK, (int)sizeof(C)), R = FX::R(S), NS = FX::NS(S),
-                NB = N / R;
-  constexpr int NBT = (NB + P - 1) / P;
-  constexpr bool LM = FX::LK > 0, LAST = S == FX::NST - 1;
-  static_assert(NB % P == 0, "every thread holds the same number of butterflies");
-  C v[NBT][R];
-  // ── reads: element j + r NB ──
-#pragma unroll
-  for (int b = 0; b < NBT; ++b) {
-    const int j = t + b * P;
-    if constexpr (S == 0) {
-      if (!LM && a.real_in) {
-        const T* s = reinterpret_cast<const T*>(cur) + l * N + j;
-#pragma unroll
-        for (int r = 0; r < R; ++r) v[b][r] = C{s[r * NB], (T)0};
-      } else {
-        const C* s = LM ? cur + l + j * FX::LK : cur + l * N + j;
-#pragma unroll
-        for (int r = 0; r < R; ++r) v[b][r] = s[r * NB * (LM ? FX::LK : 1)];
-      }
-    } else {
-      static_assert(NB % 16 == 0, "padded reads need a stride that is a multiple of 16");
-      const C* s = cur + l * LD + j + (j >> 4);
-#pragma unroll
-      for (int r = 0; r < R; ++r) v[b][r] = s[r * (NB + NB / 16)];
-    }
-  }
-  __syncthreads();
-  const T sc = a.scale;
-#pragma unroll
-  for (int b = 0; b < NBT; ++b) {
-    const int j = t + b * P;
-    const int k = j & (NS - 1);
-    if constexpr (NS > 1) {
-      const C* const tw = twb + a.sl.st[S].twoff + k;
-#pragma unroll
-      for (int r = 1; r < R; ++r) {
-        const C w = tw[(r - 1) * NS];
-        v[b][r] = INV ? cmulc(v[b][r], w) : cmul(v[b][r], w);
-      }
-    }
-    DFT<R, INV>::run(v[b]);
-    const int o = (j - k) * R + k;  // outputs o + r NS
-    if constexpr (LAST) {
-      if (sc != (T)1) {
-#pragma unroll
-        for (int r = 0; r < R; ++r) v[b][r] = cscale(v[b][r], sc);
-      }
-      if (!LM && a.real_out) {
-        T* d = reinterpret_cast<T*>(cur) + l * N + o;
-#pragma unroll
-        for (int r = 0; r < R; ++r) d[r * NS] = v[b][r].x;
-      } else {
-        C* d = LM ? cur + l + o * FX::LK : cur + l * N + o;
-#pragma unroll
-        for (int r = 0; r < R; ++r) d[r * NS * (LM ? FX::LK : 1)] = v[b][r];
-      }
-    } else if constexpr (NS % 16 == 0) {
-      C* d = cur + l * LD + o + (o >> 4);
-#pragma unroll
-      for (int r = 0; r < R; ++r) d[r * (NS + NS / 16)] = v[b][r];
-    } else if constexpr (NS == 1 && R == 16) {
-      C* d = cur + l * LD + 17 * j;  // o + r = 16 j + r, padded 17 j + r
-#pragma unroll
-      for (int r = 0; r < R; ++r) d[r] = v[b][r];
-    } else {
-      C* d = cur + l * LD;
-#pragma unroll
-      for (int r = 0; r < R; ++r) {
-        const int p = o + r * NS;
-        d[p + (p >> 4)] = v[b][r];
-      }
-    }
-  }
-  __syncthreads();
-}
-
-template <class T, bool INV, class FX>
-__device__ __forceinline__ void fixed_stages_ip(const TmaArgs<T>& a, typename CT<T>::type* cur,
-                                                const typename CT<T>::type* twb, int l, int t) {
-  fixed_stage_ip<T, INV, FX, 0>(a, cur, twb, l, t);
-  fixed_stage_ip<T, INV, FX, 1>(a, cur, twb, l, t);
-  if constexpr (FX::NST >= 3) fixed_stage_ip<T, INV, FX, 2>(a, cur, twb, l, t);
-  if constexpr (FX::NST >= 4) fixed_stage_ip<T, INV, FX, 3>(a, cur, twb, l, t);
-}
-
-// Every stage of a fixed list; returns the buffer holding the linear result.
-template <class T, bool INV, class FX>
-__device__ __forceinline__ typename CT<T>::type* fixed_stages(const TmaArgs<T>& a, typename CT<T>::type* cur,
-                                                              typename CT<T>::type* work,
-                                                              const typename CT<T>::type* twb, int l, int t) {
-  fixed_stage<T, INV, FX, 0>(a, cur, work, twb, l, t);
-  __syncthreads();
-  fixed_stage<T, INV, FX, 1>(a, work, cur, twb, l, t);
-  __syncthreads();
-  if constexpr (FX::NST == 3) {
-    fixed_stage<T, INV, FX, 2>(a, cur, work, twb, l, t);
-    __syncthreads();
-    return work;
-  } else {
-    return cur;
-  }
-}
 
 // Every stage of the tile in slot `cur` (`work` is the ping-pong buffer when
 // the stages do not run in place).  Returns the buffer that holds the result in
 // the linear layout, the TMA store's source.  Every thread of the CTA calls it
 // (the stages hold CTA barriers); (l, t) is the thread's lane and position in
 // the lane, with t >= P for a thread that has no butterflies in this tile.
-template <class T, bool INV, int V, bool IP, class FX = FixNone>
+template <class T, bool INV, int V, bool IP>
 __device__ __forceinline__ typename CT<T>::type* tma_stages(const TmaArgs<T>& a, typename CT<T>::type* cur,
                                                             typename CT<T>::type* work,
                                                             const typename CT<T>::type* twb, int l, int t) {
   constexpr bool P2 = V == 1 || V == 2 || V == 4;
   constexpr bool S7 = V == 3;
   using C = typename CT<T>::type;
-  if constexpr (V == 7) return fixed_stages<T, INV, FX>(a, cur, work, twb, l, t);
-  if constexpr (V == 8) {
-    fixed_stages_ip<T, INV, FX>(a, cur, twb, l, t);
-    return cur;
-  }
-  if constexpr (V == 5) {
-    constexpr int LK = sizeof(T) == 8 ? 8 : 16;
-    if (a.mode == 1)
-      stages256<T, INV, true, LK>(a, cur, twb, l, t);
-    else
-      stages256<T, INV, false, LK>(a, cur, twb, l, t);
-    return cur;
-  }
-  if constexpr (V == 6) {
-    stages4096<T, INV>(a, cur, twb, t);
-    return cur;
-  }
   const int L = a.L, P = a.P, n = a.sl.n, ld = a.ld;
   const bool lm = a.mode == 1;
-  const TView<C> wv{work, ld, 1, 1};
+  const TView<C> wv{work, ld, 1, 1, a.sl.psh};
   const int nst = a.sl.nst;
   const TView<C> lin = lm ? TView<C>{cur, 1, L, 0} : TView<C>{cur, n, 1, 0};
-  const TView<C> cpad{cur, ld, 1, 1};
+  const TView<C> cpad{cur, ld, 1, 1, a.sl.psh};
   // output buffer (linear layout): the one the last stage does not read
   C* obuf = (IP || !(nst & 1)) ? cur : work;
   const TView<C> olin = lm ? TView<C>{obuf, 1, L, 0} : TView<C>{obuf, n, 1, 0};
@@ -657,7 +342,8 @@ __device__ __forceinline__ typename CT<T>::type* tma_stages(const TmaArgs<T>& a,
     const TView<C> src = s == 0 ? lin : ((s & 1) ? wv : cpad);
     const TView<C> dst = last ? olin : ((s & 1) ? cpad : wv);
     const C* twi = twb + sd.twoff;
-#define AFC_TM(R) tma_stage<R, INV>(src, dst, l, n, sd.Ns, twi, t, P, last, a.scale)
+    const T sc = last ? a.scale : (T)1;
+#define AFC_TM(R) tma_stage<R, INV, P2>(src, dst, l, n, sd, twi, t, P, sc)
     if constexpr (P2) {
       switch (sd.R) {
         case 2: AFC_TM(2); break;
@@ -717,11 +403,9 @@ __device__ __forceinline__ typename CT<T>::type* tma_stages(const TmaArgs<T>& a,
 // Variant 3: 7-smooth plans (radix 2/3/4/5/7/8/16, no 11 or 13), built for two
 // CTAs of up to 256 threads per SM (at most 128 registers).  Variant 4:
 // complex64 power-of-two in place with two butterflies per thread in the
-// radix <= 8 stages (the 256-thread build of variant 1 otherwise).  Variant 5:
-// n = 256 as radix 16 x 16 in place (stages256), 16 threads per lane, built
-// like variant 2 for complex128 and like variant 1 for complex64.
-template <class T, bool INV, int V, bool IP, class FX = FixNone>
-__global__ void __launch_bounds__(TmaBuild<T, V, FX>::threads, TmaBuild<T, V, FX>::ctas)
+// radix <= 8 stages (the 256-thread build of variant 1 otherwise).
+template <class T, bool INV, int V, bool IP>
+__global__ void __launch_bounds__(TmaBuild<T, V>::threads, TmaBuild<T, V>::ctas)
     tma_kernel(const __grid_constant__ TmaArgs<T> a) {
   using C = typename CT<T>::type;
   extern __shared__ __align__(128) unsigned char smraw[];
@@ -794,7 +478,7 @@ __global__ void __launch_bounds__(TmaBuild<T, V, FX>::threads, TmaBuild<T, V, FX
       return;
     }
     C* cur = slots[cs];
-    C* obuf = tma_stages<T, INV, V, IP, FX>(a, cur, work, twb, l, t);
+    C* obuf = tma_stages<T, INV, V, IP>(a, cur, work, twb, l, t);
     fence_proxy_async();
     __syncthreads();
     if (tid == 0) tma_issue_store(a, tile, obuf);
@@ -1094,43 +778,14 @@ static long long twiddle_count(const StageList& sl) {
 
 // CTAs per SM the register budget of a kernel build allows (its launch bounds).
 static int build_ctas_per_sm(int variant, bool dbl) {
-  if (variant == 2 || (variant == 5 && dbl) || (variant == 6 && !dbl)) return 3;
-  if (variant == 3 || variant == 7 || ((variant == 1 || variant == 4 || variant == 5 || variant == 8) && !dbl))
-    return 2;
+  if (variant == 2) return 3;
+  if (variant == 3 || ((variant == 1 || variant == 4) && !dbl)) return 2;
   return 1;
 }
 
 // Threads per CTA a kernel build is compiled for (its launch bounds).
-static int build_threads(int variant, bool dbl) { return (variant == 2 || (variant == 5 && dbl)) ? 128 : 256; }
+static int build_threads(int variant) { return variant == 2 ? 128 : 256; }
 
-// The compile-time stage lists built (variant 7): the smooth odd axis lengths
-// of the 243 x 250 x 343 volume, with the thread and lane counts tma_plan
-// picks for them (contiguous tiles, and strided tiles of 8 complex128 / 16
-// complex64 lanes).
-#define AFC_FIXED_LIST(X)                                                                                \
-  X(true, 343, 7, 7, 7, 22, 0) X(true, 343, 7, 7, 7, 22, 8) X(true, 243, 9, 9, 3, 16, 0)              \
-  X(true, 243, 9, 9, 3, 16, 8) X(true, 250, 10, 5, 5, 16, 0) X(true, 250, 10, 5, 5, 16, 8)            \
-  X(false, 343, 7, 7, 7, 22, 0) X(false, 343, 7, 7, 7, 11, 16) X(false, 243, 9, 9, 3, 16, 0)          \
-  X(false, 243, 9, 9, 3, 16, 16) X(false, 250, 10, 5, 5, 16, 0) X(false, 250, 10, 5, 5, 16, 16)
-struct FixedEntry {
-  bool dbl;
-  int n, r0, r1, r2, r3, P, LK;
-};
-static const FixedEntry kFixed[] = {
-#define AFC_FX_ENTRY(D, N, R0, R1, R2, P, LK) {D, N, R0, R1, R2, 0, P, LK},
-    AFC_FIXED_LIST(AFC_FX_ENTRY)
-#undef AFC_FX_ENTRY
-};
-// The in-place power-of-two stage lists built (variant 8): 2048 points in
-// complex64 (the 2048 x 2048 images), contiguous (complex or real lanes) and
-// strided tiles of 2 lanes.
-#define AFC_FIXED_IP_LIST(X)                                                                            \
-  X(false, 2048, 16, 16, 8, 0, 128, 0) X(false, 2048, 16, 16, 8, 0, 128, 4) X(false, 2048, 16, 16, 8, 0, 128, 2)
-static const FixedEntry kFixedIP[] = {
-#define AFC_FXI_ENTRY(D, N, R0, R1, R2, R3, P, LK) {D, N, R0, R1, R2, R3, P, LK},
-    AFC_FIXED_IP_LIST(AFC_FXI_ENTRY)
-#undef AFC_FXI_ENTRY
-};
 // Keeps the twiddle table resident in shared memory when that costs no CTA
 // per SM (228 KB per SM, 1 KB reserved per CTA), for the odd-radix builds
 // only: measured on B200, 243 x 250 x 343 complex128 went from 1.32 to 1.25 ms
@@ -1139,7 +794,7 @@ static const FixedEntry kFixedIP[] = {
 static void plan_resident_twiddles(const StageList& sl, bool dbl, TmaPlan& tp, size_t extra = 0) {
   const size_t csz = dbl ? 16 : 8;
   tp.tw_res = 0;
-  if (tp.variant != 0 && tp.variant != 3 && tp.variant != 7) return;
+  if (tp.variant != 0 && tp.variant != 3) return;
   const long long twc = twiddle_count(sl);
   if (twc <= 0) return;
   const size_t base = tma_smem_bytes(tp, csz) + extra;
@@ -1246,74 +901,6 @@ bool tma_plan(const StageList& sl, int ld, long long lanes, const LaneMap& im, c
     tp.variant = 4;
   }
   if (real && !tp.inplace) return false;
-  // a 7-smooth out-of-place plan whose stage list, threads and tile are built
-  // at compile time (AFC_TMA_FIXED=0 keeps the general build; read at every plan)
-  {
-    const char* fx_env = getenv("AFC_TMA_FIXED");
-    const bool fx_on = !(fx_env && *fx_env && atoi(fx_env) == 0);
-    const int nent = (int)(sizeof(kFixed) / sizeof(kFixed[0]));
-    for (int i = 0; fx_on && tp.variant == 3 && !tp.inplace && !real && i < nent; ++i) {
-      const FixedEntry& e = kFixed[i];
-      const int nst = e.r2 ? 3 : 2;
-      if (e.dbl != dbl || e.n != n || sl.nst != nst || sl.st[0].R != e.r0 || sl.st[1].R != e.r1 ||
-          (nst == 3 && sl.st[2].R != e.r2) || P != e.P)
-        continue;
-      if (e.LK == 0 ? tp.mode != 0 : (tp.mode != 1 || tp.L != e.LK)) continue;
-      tp.variant = 7;
-      tp.fix = i;
-      break;
-    }
-    const int nip = (int)(sizeof(kFixedIP) / sizeof(kFixedIP[0]));
-    for (int i = 0; fx_on && (tp.variant == 1 || tp.variant == 4) && tp.inplace && i < nip; ++i) {
-      const FixedEntry& e = kFixedIP[i];
-      const int nst = e.r3 ? 4 : e.r2 ? 3 : 2;
-      if (e.dbl != dbl || e.n != n || sl.nst != nst || sl.st[0].R != e.r0 || sl.st[1].R != e.r1 ||
-          (nst >= 3 && sl.st[2].R != e.r2) || (nst >= 4 && sl.st[3].R != e.r3) || P != e.P)
-        continue;
-      // strided tiles of 4 lanes at 512 threads (one CTA per SM, two 70 KB
-      // slots) in place of the planner's 2 lanes at two CTAs per SM: half as
-      // many 16-byte TMA rows per point.  Measured on B200, 8 x 2048^2 R2C
-      // forward 0.31 -> 0.285 ms, forward + backward 1.59 -> 1.47 ms.
-      // AFC_TMA_L4=0 keeps 2 lanes.
-      const char* l4_env = getenv("AFC_TMA_L4");
-      const bool l4_on = !(l4_env && *l4_env && atoi(l4_env) == 0);
-      const bool widen = e.LK == 4 && l4_on && tp.mode == 1 && tp.L == 2 && !real;
-      if (!widen && (e.LK == 0 ? tp.mode != 0 : (tp.mode != 1 || tp.L != e.LK || real))) continue;
-      if (ld != ((e.n + (e.n - 1) / 16 + 1) | 1) || (!widen && tp.L * P > 256)) continue;
-      if (widen) {
-        tp.L = 4;
-        tp.kb = (im.es + tp.L - 1) / tp.L;
-      }
-      tp.variant = 8;
-      tp.fix = i;
-      break;
-    }
-  }
-  // n = 256 as radix 16 x 16 on complex lanes: the build with fixed addresses.
-  // Measured on B200 at 256^3 (forward, 20 warm repetitions): complex64 went
-  // from 206 to 151 us per transform (2.6x fewer instructions: the general
-  // stages' address and select arithmetic bounded the passes), while
-  // complex128, whose passes are DRAM-bound at 3 CTAs per SM either way, went
-  // from 285 to 298 us (twiddles resident in shared memory changed nothing),
-  // so complex128 keeps the general build.  AFC_TMA_N256: 0 off, 1 complex64
-  // (default), 2 both; read at every plan.
-  const char* n256_env = getenv("AFC_TMA_N256");
-  const int n256_on = n256_env && *n256_env ? atoi(n256_env) : 1;
-  if (n256_on && (!dbl || n256_on >= 2) && n == 256 && sl.nst == 2 && sl.st[0].R == 16 && sl.st[1].R == 16 && sl.st[0].Ns == 1 &&
-      sl.st[1].Ns == 16 && tp.inplace && !real && ld == 273 && P == 16 &&
-      (tp.variant == 2 || (tp.variant == 1 && !dbl)) && tp.L * P == build_threads(5, dbl) &&
-      (tp.mode == 0 || tp.L == (dbl ? 8 : 16)))
-    tp.variant = 5;
-  // n = 4096 as radix 16 x 16 x 16 on one contiguous complex lane per tile:
-  // the fixed-address build.  Measured on B200: 16384 x 4096 complex64
-  // forward from 350 to 255 us, 64 x 4096 complex128 forward + inverse from
-  // 20.8 to 17.9 us.  AFC_TMA_N4096: 0 off, 1 complex64 only, 2 both (default).
-  const char* n4096_env = getenv("AFC_TMA_N4096");
-  const int n4096_on = n4096_env && *n4096_env ? atoi(n4096_env) : 2;
-  if (n4096_on && (!dbl || n4096_on >= 2) && n == 4096 && sl.nst == 3 && sl.st[0].R == 16 && sl.st[1].R == 16 &&
-      sl.st[2].R == 16 && sl.st[0].Ns == 1 && sl.st[1].Ns == 16 && sl.st[2].Ns == 256 && tp.inplace && !real &&
-      ld == 4353 && P == 256 && tp.mode == 0 && tp.L == 1 && tp.variant == 1)
-    tp.variant = 6;
   tp.real_in = real_in;
   tp.real_out = real_out;
   const int align = dbl ? 8 : 16;  // 128-byte aligned slots
@@ -1327,11 +914,6 @@ bool tma_plan(const StageList& sl, int ld, long long lanes, const LaneMap& im, c
     se = (long long)tp.L * std::max<long long>(ld, n);
     se = (se + align - 1) / align * align;
     tp.slot_elems = (int)se;
-  }
-  if (tp.variant == 8) {  // the slot holds the tile in the build's padded layout
-    const FixedEntry& e = kFixedIP[tp.fix];
-    const long long need = ((long long)tp.L * fixip_ld(e.n, e.LK, (int)csz) + align - 1) / align * align;
-    if (need > tp.slot_elems) tp.slot_elems = (int)need;
   }
   if (tma_smem_bytes(tp, csz) > 220 * 1024) return false;
   // a third slot (two tile loads in flight per CTA) when it costs no CTA per
@@ -1414,42 +996,14 @@ static int sm_count() {
   return g_tma_sm;
 }
 
-template <class T, bool INV> static auto fixed_kernel(int fix) -> decltype(&tma_kernel<T, INV, 0, false>) {
-  int i = 0;
-#define AFC_FX_KERNEL(D, N, R0, R1, R2, P, LK)                                  \
-  if constexpr ((sizeof(T) == 8) == D) {                                        \
-    if (fix == i) return &tma_kernel<T, INV, 7, false, Fix<N, R0, R1, R2, P, LK>>; \
-  }                                                                             \
-  ++i;
-  AFC_FIXED_LIST(AFC_FX_KERNEL)
-#undef AFC_FX_KERNEL
-  return nullptr;
-}
-template <class T, bool INV> static auto fixed_ip_kernel(int fix) -> decltype(&tma_kernel<T, INV, 0, false>) {
-  int i = 0;
-#define AFC_FXI_KERNEL(D, N, R0, R1, R2, R3, P, LK)                                       \
-  if constexpr ((sizeof(T) == 8) == D) {                                                  \
-    if (fix == i) return &tma_kernel<T, INV, 8, true, FixIP<N, R0, R1, R2, R3, P, LK>>; \
-  }                                                                                       \
-  ++i;
-  AFC_FIXED_IP_LIST(AFC_FXI_KERNEL)
-#undef AFC_FXI_KERNEL
-  return nullptr;
-}
-
 template <class T, bool INV>
 static cudaError_t launch_tma_t(const LaunchDesc& d, const TmaPlan& tp, unsigned* err, cudaStream_t st) {
   using C = typename CT<T>::type;
-  auto k = tp.variant == 8  ? fixed_ip_kernel<T, INV>(tp.fix)
-           : tp.variant == 7 ? fixed_kernel<T, INV>(tp.fix)
-           : tp.variant == 6 ? tma_kernel<T, INV, 6, true>
-           : tp.variant == 5 ? tma_kernel<T, INV, 5, true>
-           : tp.variant == 4 ? tma_kernel<T, INV, 4, true>
+  auto k = tp.variant == 4   ? tma_kernel<T, INV, 4, true>
            : tp.variant == 2 ? tma_kernel<T, INV, 2, true>
            : tp.variant == 1 ? (tp.inplace ? tma_kernel<T, INV, 1, true> : tma_kernel<T, INV, 1, false>)
            : tp.variant == 3 ? tma_kernel<T, INV, 3, false>
                              : tma_kernel<T, INV, 0, false>;
-  if (!k) return cudaErrorInvalidValue;
   const size_t smem = tma_smem_bytes(tp, sizeof(C));
   cudaError_t e = kernel_smem_grant(reinterpret_cast<const void*>(k), smem);
   if (e != cudaSuccess) return e;
@@ -1499,9 +1053,7 @@ static cudaError_t launch_tma_t(const LaunchDesc& d, const TmaPlan& tp, unsigned
 }
 
 template <class T, bool INV> static const void* pair_kernel_ptr(int variant, bool ip) {
-  auto k = variant == 6   ? tma_pair_kernel<T, INV, 6, true>
-           : variant == 5 ? tma_pair_kernel<T, INV, 5, true>
-           : variant == 4 ? tma_pair_kernel<T, INV, 4, true>
+  auto k = variant == 4   ? tma_pair_kernel<T, INV, 4, true>
            : variant == 2 ? tma_pair_kernel<T, INV, 2, true>
            : variant == 1 ? (ip ? tma_pair_kernel<T, INV, 1, true> : tma_pair_kernel<T, INV, 1, false>)
                           : tma_pair_kernel<T, INV, 3, false>;
@@ -1554,9 +1106,7 @@ bool tma_pair_plan(const LaunchDesc& d0, const LaunchDesc& d1, long long planes,
   const size_t csz = dbl ? 16 : 8;
   pp.slot_elems = std::max(a.slot_elems, b.slot_elems);
   pp.threads = std::max(a.L * a.P, b.L * b.P);
-  if (pp.threads > build_threads(a.variant, dbl)) return false;
-  // the fixed-address build gives every thread a butterfly in both phases
-  if (a.variant == 5 && (a.L * a.P != pp.threads || b.L * b.P != pp.threads)) return false;
+  if (pp.threads > build_threads(a.variant)) return false;
   pp.smem = 2 * (size_t)pp.slot_elems * csz +
             (a.inplace ? 0 : (size_t)std::max(a.L * a.ld, b.L * b.ld) * csz) + 64;
   if (pp.smem > 220 * 1024) return false;
