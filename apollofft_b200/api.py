@@ -21,6 +21,8 @@ direct sums, the `_fast` forms the Kaiser-Bessel plans (oversampling 2).
 """
 from __future__ import annotations
 
+import functools
+
 import numpy as np
 
 from . import _lib as L
@@ -58,8 +60,16 @@ def _to_f16_storage(a: np.ndarray) -> np.ndarray:
     return a.astype(np.float16).astype(np.float32)
 
 
+# The plans of the last calls' shapes: the library caches plans process-wide, so
+# this only saves the wrapper (its lookup and size queries cost a small volume
+# about a third of each call).
+@functools.lru_cache(maxsize=128)
+def _cached_plan(shape, prec, kind, device):
+    return CudaPlan(list(shape), precision=prec, kind=kind, device=device)
+
+
 def _plan(shape, prec, kind, device=0):
-    return CudaPlan(list(shape), precision="f64" if prec == "f64" else "f32", kind=kind, device=device)
+    return _cached_plan(tuple(shape), "f64" if prec == "f64" else "f32", kind, device)
 
 
 # ── input kinds: numpy arrays, torch tensors (CUDA or CPU), DLPack producers ──
