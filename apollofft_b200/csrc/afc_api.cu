@@ -1299,10 +1299,13 @@ struct afc_nufft_plan_s {
   int64_t n = 0, m = 0;
   int w = 0;
   double dx = 0, beta = 0, i0b = 1;
+  afc::NuPoly f;
   int device = 0;
   afc_plan fft = nullptr;          // C2C f64 plan of length m
   double* deconv = nullptr;        // 1 / kb_ft(k_signed / m), k < n
   void* grid = nullptr;            // plan-owned oversampled grid (m complex128)
+  afc::NuTileLaunch tiles;         // sorted spreading: bins, and bin / rank / index per point
+  int64_t pts_cap = 0;             // points the latter hold
   std::mutex mu;                   // one caller enqueues on the grid at a time
   afc::Fence fence;                // the grid's last use on the GPU
   ~afc_nufft_plan_s();
@@ -1316,12 +1319,14 @@ struct afc_nufft3d_plan_s {
   double d[3] = {0, 0, 0};
   int w = 0;
   double beta = 0, i0b = 1;
+  afc::NuPoly f;
   int device = 0;
   afc_plan fft = nullptr;
   double* deconv = nullptr;  // nx + ny + nz factors, axis after axis
   void* grid = nullptr;      // mx my mz complex128, C order
   afc::NuTileLaunch tiles;   // B = 0: per-point kernels
   int64_t pts_cap = 0;       // points the tile / rank / index buffers hold
+  int64_t rec_cap = 0;       // points the record buffer holds
   std::mutex mu;             // one caller enqueues on the grid at a time
   afc::Fence fence;          // the grid's (and tile buffers') last use on the GPU
   ~afc_nufft3d_plan_s();
@@ -2255,14 +2260,17 @@ static afc_status no_alloc_scratch(int dev, void** ptr) {
 using namespace afc;
 
 afc_nufft_plan_s::~afc_nufft_plan_s() {
+  for (int* b : {tiles.cnt, tiles.tile})
+    if (b) cudaFree(b);
   if (fft) afc_plan_destroy(fft);
   if (deconv) cudaFree(deconv);
   if (grid) cudaFree(grid);
 }
 
 afc_nufft3d_plan_s::~afc_nufft3d_plan_s() {
-  for (int* b : {tiles.cnt, tiles.off, tiles.tile, tiles.rank, tiles.idx})
+  for (int* b : {tiles.cnt, tiles.off, tiles.tile})
     if (b) cudaFree(b);
+  if (tiles.rec) cudaFree(tiles.rec);
   if (fft) afc_plan_destroy(fft);
   if (deconv) cudaFree(deconv);
   if (grid) cudaFree(grid);
@@ -2783,6 +2791,24 @@ static double nu_i0_host(double z) {
   }
   return sum;
 }
+// phi's coefficients in s = w^2 - x^2: (beta / 2w)^2k / (k!)^2 / I0(beta).
+static NuPoly nu_poly(double beta, int w) {
+  NuPoly f;
+  const long double q = 0.25L * (long double)beta * (long double)beta;
+  std::vector<long double> t{1.0L};
+  long double sum = 1.0L;
+  for (int k = 1; k <= 256; ++k) {
+    t.push_back(t.back() * q / ((long double)k * (long double)k));
+    sum += t.back();
+    if ((long double)k * k > q && t.back() < sum * 0x1p-60L) break;
+  }
+  t.pop_back();
+  if ((int)t.size() > NuPoly::max) return f;
+  f.K = (int)t.size();
+  long double w2k = 1.0L;
+  for (int k = 0; k < f.K; ++k, w2k *= (long double)w * w) f.c[k] = (double)(t[k] / sum / w2k);
+  return f;
+}
 static double nu_kb_ft(double xi, int w, double beta, double i0b) {
   const double twx = 2.0 * M_PI * (double)w * xi;
   const double z2 = beta * beta - twx * twx;
@@ -2813,6 +2839,7 @@ afc_status afc_nufft1d_plan_create(afc_nufft_plan* out, int64_t n, double dx, in
   p->dx = dx;
   p->beta = M_PI * (1.0 - 1.0 / (2.0 * (double)sigma)) * (double)(2 * kernel_width);
   p->i0b = nu_i0_host(p->beta);
+  p->f = nu_poly(p->beta, p->w);
   p->device = device;
   afc_status s = afc_plan_create(&p->fft, 1, &p->m, AFC_PREC_F64, AFC_KIND_C2C, 1, device);
   if (s != AFC_OK) return s;
@@ -2835,8 +2862,30 @@ static NuLaunch nu_launch(const afc_nufft_plan_s& p) {
   L.w = p.w;
   L.beta = p.beta;
   L.i0b = p.i0b;
+  L.f = p.f;
   L.len = (double)p.n * p.dx;
   return L;
+}
+
+// Buffers of a sorted spread (synchronous allocation when a call brings more
+// points than any before it).
+static afc_status nu1_reserve(afc_nufft_plan_s& p, int64_t npts) {
+  if (!nufft_sorted(nu_launch(p), npts)) return AFC_OK;
+  if (!p.tiles.cnt) {
+    const int w = nufft_bin_width(p.m);
+    const size_t bins = (size_t)((p.m + w - 1) / w);
+    AFC_CUDA(dev_alloc((void**)&p.tiles.cnt, (2 * bins + 1) * sizeof(int)), "NUFFT bins");  // cnt, then off
+    p.tiles.off = p.tiles.cnt + bins;
+  }
+  if (npts <= p.pts_cap) return AFC_OK;
+  if (p.tiles.tile) cudaFree(p.tiles.tile);  // tile, rank and idx are one allocation
+  p.tiles.tile = p.tiles.rank = p.tiles.idx = nullptr;
+  p.pts_cap = 0;
+  AFC_CUDA(dev_alloc((void**)&p.tiles.tile, 3 * (size_t)npts * sizeof(int)), "NUFFT point bins");
+  p.tiles.rank = p.tiles.tile + npts;
+  p.tiles.idx = p.tiles.rank + npts;
+  p.pts_cap = npts;
+  return AFC_OK;
 }
 
 afc_status afc_nufft1d_type1(afc_nufft_plan plan, const double* positions, const void* values, int64_t npts, void* out,
@@ -2851,7 +2900,9 @@ afc_status afc_nufft1d_type1(afc_nufft_plan plan, const double* positions, const
   const bool cap = stream_capturing(st);
   AFC_CUDA(plan->fence.before(st, cap), "NUFFT ordering");
   AFC_CUDA(cudaMemsetAsync(plan->grid, 0, (size_t)plan->m * 16, st), "NUFFT grid");
-  AFC_CUDA(nufft_spread_dev(nu_launch(*plan), positions, values, npts, plan->grid, st), "NUFFT spread");
+  afc_status r = nu1_reserve(*plan, npts);
+  if (r != AFC_OK) return r;
+  AFC_CUDA(nufft_spread_dev(nu_launch(*plan), plan->tiles, positions, values, npts, plan->grid, st), "NUFFT spread");
   afc_status s = afc_execute(plan->fft, plan->grid, plan->grid, AFC_FORWARD, stream);
   if (s != AFC_OK) return s;
   AFC_CUDA(nufft_deconv_out_dev(plan->grid, plan->deconv, plan->n, plan->m, out, st), "NUFFT deconvolution");
@@ -2973,6 +3024,7 @@ afc_status afc_nufft3d_plan_create(afc_nufft3d_plan* out, int64_t nx, int64_t ny
   p->w = (int)kernel_width;
   p->beta = M_PI * (1.0 - 1.0 / (2.0 * (double)sigma)) * (double)(2 * kernel_width);
   p->i0b = nu_i0_host(p->beta);
+  p->f = nu_poly(p->beta, p->w);
   p->device = device;
   int64_t total_n = 0;
   for (int a = 0; a < 3; ++a) {
@@ -3016,16 +3068,26 @@ afc_status afc_nufft3d_plan_create(afc_nufft3d_plan* out, int64_t nx, int64_t ny
 
 // Grows the per-point tile buffers (synchronous allocation) when a call brings
 // more points than any call before it; false -> the per-point kernels run.
+static afc_status nu3_reserve_records(afc_nufft3d_plan_s& p, int64_t npts, cudaStream_t st) {
+  const int64_t n = std::min<int64_t>(npts, kNu3Slice);
+  if (n <= p.rec_cap) return AFC_OK;
+  if (p.tiles.rec) cudaFree(p.tiles.rec);
+  p.tiles.rec = nullptr;
+  p.rec_cap = 0;
+  AFC_CUDA(dev_alloc((void**)&p.tiles.rec, (size_t)n * nufft3_rec_bytes(p.w)), "NUFFT point records");
+  AFC_CUDA(cudaMemsetAsync(p.tiles.rec, 0, (size_t)n * nufft3_rec_bytes(p.w), st), "NUFFT point records");
+  p.rec_cap = n;
+  return AFC_OK;
+}
 static afc_status nu3_reserve(afc_nufft3d_plan_s& p, int64_t npts, bool* tiled) {
   *tiled = p.tiles.B != 0 && npts > 0 && npts <= INT32_MAX;
   if (!*tiled || npts <= p.pts_cap) return AFC_OK;
-  for (int** b : {&p.tiles.tile, &p.tiles.rank, &p.tiles.idx}) {
-    if (*b) cudaFree(*b);
-    *b = nullptr;
-  }
+  if (p.tiles.tile) cudaFree(p.tiles.tile);  // tile, rank and idx are one allocation
+  p.tiles.tile = p.tiles.rank = p.tiles.idx = nullptr;
   p.pts_cap = 0;
-  for (int** b : {&p.tiles.tile, &p.tiles.rank, &p.tiles.idx})
-    AFC_CUDA(dev_alloc((void**)b, (size_t)npts * sizeof(int)), "NUFFT point buckets");
+  AFC_CUDA(dev_alloc((void**)&p.tiles.tile, 3 * (size_t)npts * sizeof(int)), "NUFFT point buckets");
+  p.tiles.rank = p.tiles.tile + npts;
+  p.tiles.idx = p.tiles.rank + npts;
   p.pts_cap = npts;
   return AFC_OK;
 }
@@ -3043,6 +3105,7 @@ static NuLaunch3 nu_launch3(const afc_nufft3d_plan_s& p) {
   L.w = p.w;
   L.beta = p.beta;
   L.i0b = p.i0b;
+  L.f = p.f;
   L.lx = (double)p.n[0] * p.d[0];
   L.ly = (double)p.n[1] * p.d[1];
   L.lz = (double)p.n[2] * p.d[2];
@@ -3065,7 +3128,11 @@ afc_status afc_nufft3d_type1(afc_nufft3d_plan plan, const double* positions, con
   bool tiled = false;
   afc_status r = nu3_reserve(*plan, npts, &tiled);
   if (r != AFC_OK) return r;
-  if (tiled)
+  if (tiled && nufft3_boxes(L)) {
+    r = nu3_reserve_records(*plan, npts, st);
+    if (r != AFC_OK) return r;
+    AFC_CUDA(nufft3_boxes_dev(L, plan->tiles, true, positions, values, npts, plan->grid, nullptr, st), "NUFFT spread");
+  } else if (tiled)
     AFC_CUDA(nufft3_tiled_dev(L, plan->tiles, true, positions, values, npts, plan->grid, st), "NUFFT spread");
   else
     AFC_CUDA(nufft3_spread_dev(L, positions, values, npts, plan->grid, st), "NUFFT spread");
@@ -3098,7 +3165,12 @@ afc_status afc_nufft3d_type2(afc_nufft3d_plan plan, const void* modes, const dou
   bool tiled = false;
   s = nu3_reserve(*plan, npts, &tiled);
   if (s != AFC_OK) return s;
-  if (tiled)
+  if (tiled && nufft3_boxes(L)) {
+    s = nu3_reserve_records(*plan, npts, st);
+    if (s != AFC_OK) return s;
+    AFC_CUDA(nufft3_boxes_dev(L, plan->tiles, false, positions, nullptr, npts, plan->grid, out, st),
+             "NUFFT interpolation");
+  } else if (tiled)
     AFC_CUDA(nufft3_tiled_dev(L, plan->tiles, false, positions, plan->grid, npts, out, st), "NUFFT interpolation");
   else
     AFC_CUDA(nufft3_interp_dev(L, plan->grid, positions, npts, out, st), "NUFFT interpolation");

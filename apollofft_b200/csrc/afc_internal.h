@@ -200,13 +200,25 @@ struct TcLaunch {
 cudaError_t launch_tc_fft(const TcLaunch& d, bool fp16, cudaStream_t st);
 
 // 1D NUFFT spreading / interpolation (afc_nufft.cu), complex128 grids
+// Coefficients of phi in s = w^2 - x^2 (K = 0: none, the series is evaluated).
+struct NuPoly {
+  static constexpr int max = 80;  // terms for w <= 12 at sigma = 2
+  int K = 0;
+  double c[max] = {};
+};
 struct NuLaunch {
   long long m = 0;   // oversampled grid length
   int w = 0;         // kernel half width
   double beta = 0, i0b = 1, len = 1;
+  NuPoly f;
 };
-cudaError_t nufft_spread_dev(const NuLaunch& L, const double* pos, const void* val, long long npts, void* grid,
-                             cudaStream_t st);
+struct NuTileLaunch;
+// Whether a spread of npts points sorts them first (the plan then holds bins of
+// nufft_bin_width cells, at most 16384, and a bin, rank and index per point).
+bool nufft_sorted(const NuLaunch& L, long long npts);
+inline int nufft_bin_width(long long m) { return (int)std::max<long long>(8, (m + 16383) / 16384); }
+cudaError_t nufft_spread_dev(const NuLaunch& L, const NuTileLaunch& TL, const double* pos, const void* val,
+                             long long npts, void* grid, cudaStream_t st);
 cudaError_t nufft_interp_dev(const NuLaunch& L, const void* grid, const double* pos, long long npts, void* out,
                              cudaStream_t st);
 cudaError_t nufft_deconv_out_dev(const void* grid, const double* deconv, long long n, long long m, void* out,
@@ -215,6 +227,7 @@ struct NuLaunch3 {
   long long nx = 0, ny = 0, nz = 0, mx = 0, my = 0, mz = 0;
   int w = 0;
   double beta = 0, i0b = 1, lx = 1, ly = 1, lz = 1;
+  NuPoly f;
 };
 cudaError_t nufft3_spread_dev(const NuLaunch3& L, const double* pos, const void* val, long long npts, void* grid,
                               cudaStream_t st);
@@ -229,7 +242,15 @@ struct NuTileLaunch {
   int* tile = nullptr;  // npts
   int* rank = nullptr;  // npts
   int* idx = nullptr;   // npts
+  double* rec = nullptr;  // box kernels: a record per point of a slice, zeroed when allocated
 };
+// Points the box kernels take at a time (bounds their record buffer).
+constexpr long long kNu3Slice = 1 << 18;
+bool nufft3_boxes(const NuLaunch3& L);
+size_t nufft3_box_smem(int w);
+size_t nufft3_rec_bytes(int w);
+cudaError_t nufft3_boxes_dev(const NuLaunch3& L, const NuTileLaunch& TL, bool spread, const double* pos,
+                             const void* val, long long npts, void* grid, void* out, cudaStream_t st);
 int nufft3_tile_size(int w);
 size_t nufft3_tile_smem(int B, int w);
 cudaError_t nufft3_tiled_dev(const NuLaunch3& L, const NuTileLaunch& TL, bool spread, const double* pos,

@@ -54,11 +54,82 @@ __device__ __forceinline__ double nu_kb(double x, double w, double beta, double 
   return nu_i0(beta * sqrt(1.0 - u2)) / i0b;
 }
 
+// phi as a polynomial: I0's series in (z/2)^2 = (beta / 2w)^2 s, s = w^2 - x^2,
+// divided by I0(beta), has the fixed positive coefficients NuPoly::c, so Horner
+// needs one FMA per term instead of the running product's three operations, no
+// division and no square root; s = (w - x)(w + x) does not cancel at the edge.  The first dropped term is below 2^-60 of phi(0) = 1.  Measured
+// on B200 at w = 6 (46 terms): the weights were about half of a 1D call.  K = 0
+// (kernels too wide for the table): the series.
+__device__ __forceinline__ double nu_phi(const NuPoly& f, double x, double w, double beta, double i0b) {
+  if (f.K == 0) return nu_kb(x, w, beta, i0b);
+  const double s = (w - x) * (w + x);
+  if (!(s > 0.0)) return 0.0;
+  double a = f.c[f.K - 1];
+#pragma unroll 5
+  for (int k = f.K - 2; k >= 0; --k) a = fma(a, s, f.c[k]);
+  return a;
+}
+
+// Taps p0 .. p0 + 3 of one axis at once (four independent chains per coefficient).
+__device__ __forceinline__ void nu_phi4(const NuPoly& f, int p0, double d, int w, double beta, double i0b, double* o) {
+  if (f.K == 0) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) o[i] = nu_kb((double)(p0 + i - w) - d, (double)w, beta, i0b);
+    return;
+  }
+  double s[4], a[4];
+  const double c0 = f.c[f.K - 1];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const double x = (double)(p0 + i - w) - d;
+    s[i] = ((double)w - x) * ((double)w + x);
+    a[i] = c0;
+  }
+#pragma unroll 5
+  for (int k = f.K - 2; k >= 0; --k) {
+    const double c = f.c[k];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) a[i] = fma(a[i], s[i], c);
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) o[i] = s[i] > 0.0 ? a[i] : 0.0;
+}
+
+// All T taps of one axis in one walk over the coefficients (T independent chains:
+// a coefficient load feeds T FMAs instead of four, and no tap is evaluated past
+// the kernel).
+template <int T>
+__device__ __forceinline__ void nu_phi_all(const NuPoly& f, double d, double beta, double i0b, double (&o)[T]) {
+  constexpr int w = T / 2;
+  if (f.K == 0) {
+#pragma unroll
+    for (int i = 0; i < T; ++i) o[i] = nu_kb((double)(i - w) - d, (double)w, beta, i0b);
+    return;
+  }
+  double s[T];
+  const double c0 = f.c[f.K - 1];
+#pragma unroll
+  for (int i = 0; i < T; ++i) {
+    const double x = (double)(i - w) - d;
+    s[i] = ((double)w - x) * ((double)w + x);
+    o[i] = c0;
+  }
+#pragma unroll 2
+  for (int k = f.K - 2; k >= 0; --k) {
+    const double c = f.c[k];
+#pragma unroll
+    for (int i = 0; i < T; ++i) o[i] = fma(o[i], s[i], c);
+  }
+#pragma unroll
+  for (int i = 0; i < T; ++i) o[i] = s[i] > 0.0 ? o[i] : 0.0;
+}
+
 struct NuGeom {
   long long m;     // oversampled length
   int w;           // kernel half width
   double beta, i0b;
   double len;      // periodic domain length n dx
+  NuPoly f;
 };
 
 // Position -> (m0, d): x mod L (Euclidean), t = m x / L, m0 = round(t) (half
@@ -77,37 +148,166 @@ __device__ __forceinline__ long long nu_wrap(long long i, long long m) {
   return r < 0 ? r + m : r;
 }
 
-__global__ void nu_spread(NuGeom g, const double* __restrict__ pos, const double2* __restrict__ val, long long npts,
+__global__ void nu_spread(const __grid_constant__ NuGeom g, const double* __restrict__ pos, const double2* __restrict__ val, long long npts,
                           double2* grid) {
   for (long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x; j < npts; j += (long long)gridDim.x * blockDim.x) {
     long long m0;
     double d;
     nu_place(g, pos[j], m0, d);
     const double2 v = val[j];
-    for (int p = -g.w; p <= g.w; ++p) {
-      const double wt = nu_kb((double)p - d, (double)g.w, g.beta, g.i0b);
-      if (wt != 0.0) {
-        double2* c = grid + nu_wrap(m0 + p, g.m);
-        atomicAdd(&c->x, v.x * wt);
-        atomicAdd(&c->y, v.y * wt);
+    long long cell = nu_wrap(m0 - g.w, g.m);
+    for (int p = 0; p <= 2 * g.w; p += 4) {
+      double wt[4];
+      nu_phi4(g.f, p, d, g.w, g.beta, g.i0b, wt);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        if (p + i <= 2 * g.w && wt[i] != 0.0) {
+          double2* c = grid + cell;
+          atomicAdd(&c->x, v.x * wt[i]);
+          atomicAdd(&c->y, v.y * wt[i]);
+        }
+        if (++cell >= g.m) cell -= g.m;
       }
     }
   }
 }
 
-__global__ void nu_interp(NuGeom g, const double2* __restrict__ grid, const double* __restrict__ pos, long long npts,
+// Spreading of sorted points.  The kernel above is bound by its FP64 atomics
+// (2 (2w + 1) per point, about 140 G/s), and crowded points contend for the same
+// cells.  Sorted by bins of cells, the 32 points of a warp fall within a few
+// cells of each other: each lane evaluates its point's weights, then the warp
+// takes a window of 32 cells, one per lane, and every lane sums what the points
+// of the window add to its cell before one atomic add: about 20 cells per 32
+// points and window instead of 32 (2w + 1).  Points too far from the first one
+// wait for the next window.
+constexpr int kNu1Warps = 4;
+__host__ __device__ constexpr size_t nu1_smem(int T) {
+  return (size_t)kNu1Warps * ((size_t)T * 33 * sizeof(double) + 32 * (sizeof(double2) + sizeof(int)));
+}
+
+__global__ void nu1_bin(const __grid_constant__ NuGeom g, int width, const double* __restrict__ pos, long long npts,
+                        int* __restrict__ cnt, int* __restrict__ bin, int* __restrict__ rank) {
+  for (long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x; j < npts; j += (long long)gridDim.x * blockDim.x) {
+    long long m0;
+    double d;
+    nu_place(g, pos[j], m0, d);
+    const int b = (int)nu_wrap(m0, g.m) / width;
+    bin[j] = b;
+    rank[j] = atomicAdd(&cnt[b], 1);
+  }
+}
+
+// TC: taps at compile time (0: any width)
+template <int TC>
+__global__ void __launch_bounds__(32 * kNu1Warps) nu1_spread(const __grid_constant__ NuGeom g, const int* __restrict__ idx,
+                                                             const double* __restrict__ pos,
+                                                             const double2* __restrict__ val, long long npts,
+                                                             double2* grid) {
+  extern __shared__ __align__(16) unsigned char nu_smem[];
+  const int T = TC ? TC : 2 * g.w + 1, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  double2* const sv = reinterpret_cast<double2*>(nu_smem) + 32 * wid;
+  double* const sw = reinterpret_cast<double*>(reinterpret_cast<double2*>(nu_smem) + 32 * kNu1Warps) + wid * T * 33;
+  int* const sc = reinterpret_cast<int*>(reinterpret_cast<double*>(reinterpret_cast<double2*>(nu_smem) + 32 * kNu1Warps) +
+                                         kNu1Warps * T * 33) + 32 * wid;
+  const long long step = (long long)gridDim.x * kNu1Warps * 32;
+  for (long long base = ((long long)blockIdx.x * kNu1Warps + wid) * 32; base < npts; base += step) {
+    const bool valid = base + lane < npts;
+    int c = 0;
+    if (valid) {
+      const int j = idx[base + lane];
+      long long m0;
+      double d;
+      nu_place(g, pos[j], m0, d);
+      c = (int)nu_wrap(m0, g.m);
+      sv[lane] = val[j];
+      if constexpr (TC > 0) {
+        double o[TC];
+        nu_phi_all<TC>(g.f, d, g.beta, g.i0b, o);
+#pragma unroll
+        for (int i = 0; i < TC; ++i) sw[i * 33 + lane] = o[i];
+      } else {
+        for (int p = 0; p < T; p += 4) {
+          double o[4];
+          nu_phi4(g.f, p, d, g.w, g.beta, g.i0b, o);
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            if (p + i < T) sw[(p + i) * 33 + lane] = o[i];
+        }
+      }
+      sc[lane] = c;
+    }
+    __syncwarp();
+    unsigned rem = __ballot_sync(0xffffffffu, valid);
+    while (rem) {
+      const bool left = rem >> lane & 1;
+      const int c0 = (int)__reduce_min_sync(0xffffffffu, left ? (unsigned)c : 0xffffffffu);
+      const bool hit = left && c - c0 <= 31 - 2 * g.w;
+      unsigned mask = __ballot_sync(0xffffffffu, hit);
+      rem &= ~mask;
+      double ax = 0.0, ay = 0.0;
+      while (mask) {
+        const int p = __ffs(mask) - 1;
+        mask &= mask - 1;
+        const int tap = lane - (sc[p] - c0);  // cell c0 - w + lane of point p
+        const double2 v = sv[p];
+        const double wt = tap >= 0 && tap < T ? sw[tap * 33 + p] : 0.0;
+        if (wt != 0.0) {
+          ax = fma(v.x, wt, ax);
+          ay = fma(v.y, wt, ay);
+        }
+      }
+      if (ax != 0.0 || ay != 0.0) {
+        long long cell = (long long)c0 - g.w + lane;
+        if (cell < 0) cell += g.m;
+        if (cell >= g.m) cell -= g.m;
+        atomicAdd(&grid[cell].x, ax);
+        atomicAdd(&grid[cell].y, ay);
+      }
+    }
+    __syncwarp();
+  }
+}
+
+// TC: taps at compile time (0: any width)
+template <int TC>
+__global__ void __launch_bounds__(256) nu_interp(const __grid_constant__ NuGeom g, const double2* __restrict__ grid, const double* __restrict__ pos, long long npts,
                           double2* out) {
   for (long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x; j < npts; j += (long long)gridDim.x * blockDim.x) {
     long long m0;
     double d;
     nu_place(g, pos[j], m0, d);
     double2 acc = make_double2(0.0, 0.0);
-    for (int p = -g.w; p <= g.w; ++p) {
-      const double wt = nu_kb((double)p - d, (double)g.w, g.beta, g.i0b);
-      if (wt != 0.0) {
-        const double2 c = grid[nu_wrap(m0 + p, g.m)];
-        acc.x += c.x * wt;
-        acc.y += c.y * wt;
+    long long cell = nu_wrap(m0 - g.w, g.m);
+    if constexpr (TC > 0) {
+      double wt[TC];
+      nu_phi_all<TC>(g.f, d, g.beta, g.i0b, wt);
+#pragma unroll
+      for (int i = 0; i < TC; ++i) {
+        const double2 c = grid[cell];
+        if (wt[i] != 0.0) {
+          acc.x += c.x * wt[i];
+          acc.y += c.y * wt[i];
+        }
+        if (++cell >= g.m) cell -= g.m;
+      }
+      out[j] = acc;
+      continue;
+    }
+    for (int p = 0; p <= 2 * g.w; p += 4) {
+      double2 c[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {  // the loads fly while the weights are evaluated
+        c[i] = p + i <= 2 * g.w ? grid[cell] : make_double2(0.0, 0.0);
+        if (++cell >= g.m) cell -= g.m;
+      }
+      double wt[4];
+      nu_phi4(g.f, p, d, g.w, g.beta, g.i0b, wt);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        if (wt[i] != 0.0) {  // a tap outside the kernel adds nothing, whatever its cell holds
+          acc.x += c[i].x * wt[i];
+          acc.y += c[i].y * wt[i];
+        }
       }
     }
     out[j] = acc;
@@ -150,6 +350,7 @@ struct NuGeom3 {
   int w;
   double beta, i0b;
   double lx, ly, lz;
+  NuPoly f;
 };
 
 constexpr int kNuMaxTaps = 65;       // T for w <= 32
@@ -167,7 +368,7 @@ __device__ __forceinline__ long long nu_axis_weights(double x, double len, long 
   const double t = nu_axis_t(x, len, m);
   const double rt = round(t);
   const double d = t - rt;
-  for (int p = lane; p <= 2 * g.w; p += 32) wt[p] = nu_kb((double)(p - g.w) - d, (double)g.w, g.beta, g.i0b);
+  for (int p = lane; p <= 2 * g.w; p += 32) wt[p] = nu_phi(g.f, (double)(p - g.w) - d, (double)g.w, g.beta, g.i0b);
   return (long long)rt;
 }
 
@@ -177,7 +378,7 @@ struct NuPlaneWalk {  // lane's (py, pz) start and the constant stride of 32 fla
       : py0(lane / T), pz0(lane % T), dpy(32 / T), dpz(32 % T), iters((T * T + 31) / 32) {}
 };
 
-__global__ void __launch_bounds__(32 * kNuWarps) nu_spread3(NuGeom3 g, const double* __restrict__ pos,
+__global__ void __launch_bounds__(32 * kNuWarps) nu_spread3(const __grid_constant__ NuGeom3 g, const double* __restrict__ pos,
                                                               const double2* __restrict__ val, long long npts,
                                                               double2* grid) {
   __shared__ double sw[kNuWarps][3][kNuMaxTaps];
@@ -218,7 +419,7 @@ __global__ void __launch_bounds__(32 * kNuWarps) nu_spread3(NuGeom3 g, const dou
   }
 }
 
-__global__ void __launch_bounds__(32 * kNuWarps) nu_interp3(NuGeom3 g, const double2* __restrict__ grid,
+__global__ void __launch_bounds__(32 * kNuWarps) nu_interp3(const __grid_constant__ NuGeom3 g, const double2* __restrict__ grid,
                                                               const double* __restrict__ pos, long long npts,
                                                               double2* out) {
   __shared__ double sw[kNuWarps][3][kNuMaxTaps];
@@ -290,7 +491,7 @@ __device__ __forceinline__ int nu_centre(double x, double len, long long m) {
   return (int)((long long)round(nu_axis_t(x, len, m)) & (m - 1));
 }
 
-__global__ void nu3_bin(NuGeom3 g, int B, int nty, int ntz, const double* __restrict__ pos, long long npts,
+__global__ void nu3_bin(const __grid_constant__ NuGeom3 g, int B, int nty, int ntz, const double* __restrict__ pos, long long npts,
                         int* __restrict__ cnt, int* __restrict__ tile, int* __restrict__ rank) {
   for (long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x; j < npts; j += (long long)gridDim.x * blockDim.x) {
     const int cx = nu_centre(pos[3 * j], g.lx, g.mx);
@@ -357,7 +558,7 @@ __device__ __forceinline__ double nu_tile_weight(const NuGeom3& g, const NuTiles
   const double t = nu_axis_t(pos[a], len, m);
   const double rt = round(t);
   if (lc) *lc = (int)((long long)rt & (m - 1)) - t0 * tl.B;
-  return nu_kb((double)(tap - g.w) - (t - rt), (double)g.w, g.beta, g.i0b);
+  return nu_phi(g.f, (double)(tap - g.w) - (t - rt), (double)g.w, g.beta, g.i0b);
 }
 
 // The lane's cells of a T x T (py, pz) plane: at most kNuTileIters, packed
@@ -375,7 +576,7 @@ struct NuLaneCells {
   }
 };
 
-__global__ void __launch_bounds__(kNuTileThreads) nu3_spread_tiles(NuGeom3 g, NuTiles tl,
+__global__ void __launch_bounds__(kNuTileThreads) nu3_spread_tiles(const __grid_constant__ NuGeom3 g, NuTiles tl,
                                                                     const double* __restrict__ pos,
                                                                     const double2* __restrict__ val, double2* grid) {
   extern __shared__ __align__(16) unsigned char nu_smem[];
@@ -452,14 +653,274 @@ __global__ void __launch_bounds__(kNuTileThreads) nu3_spread_tiles(NuGeom3 g, Nu
   }
 }
 
-__global__ void __launch_bounds__(kNuTileThreads) nu3_interp_tiles(NuGeom3 g, NuTiles tl,
+// ─── 3D spreading and interpolation by boxes of cells ───
+// The tile kernels are bound by shared memory (a 16-byte cell per tap, read and
+// for spreading written back) and spreading adds every tile's halo to the grid
+// with atomics, 15 times the cells at w = 6.  Here the cells stay in registers
+// and the points move: a warp owns a box of 8 x 4 x 8 cells and meets every
+// point whose taps reach it (25 boxes per point at w = 6).  Per box the sums are
+// small FP64 matrix products (mma m8n8k4):
+//   spreading      C[x][z] += wx[point][x] (v wy wz)[point][z], 4 points at a
+//                  time, for each y and for both parts of v;
+//   interpolation  D[point][z] = sum_x wx[point][x] cell[x][z], 8 points at a
+//                  time, then summed over y and z with their weights.
+// One operand element per lane feeds 8 FMAs.  Measured at 2^18 points on 128^3
+// cells, w = 6 (kernel alone): tiles 1650 us spreading, 784 us interpolating; boxes
+// with scalar FMAs, bound by the broadcast weight loads, 1095 us spreading; these
+// 600 and 690 us, bound by the latency of the shared-memory loads behind each
+// group (the FP64 matrix pipe is a third busy).
+//  nu3_points: one record per point in tile order: value, centre, index, and the
+//              axis weights between runs of seven zeros, so no tap is range-checked;
+//  nu3_boxes:  a CTA of 8 warps owns 16 x 8 x 16 cells and streams the records of
+//              the tiles within w cells of it through shared memory, the next chunk
+//              in flight while one is worked on.  Each warp lists the records that
+//              meet its box and takes them in groups.
+// Boxes partition the grid: spreading writes each cell once, without atomics
+// unless a box's points are split over CTAs; interpolation adds a partial sum
+// per point and box to the outputs.
+constexpr int kNuBoxThreads = 256;
+// chunk and CTAs per SM measured at 2^18 points on 128^3 cells, w = 6 (spreading /
+// interpolation): 32 points, three CTAs 798 / 900 us for the whole call, 64 points,
+// two CTAs 845 / 927, 32 points, two CTAs 917 / 1027
+constexpr int kNuBoxChunk = 32;
+constexpr int kNuBoxRuns = 64;  // contiguous runs of candidate points per CTA
+
+// Record: v.x, v.y, centre cells and index (four ints), then x, y and z weights.
+__host__ __device__ constexpr int nu_xo(int) { return 11; }
+__host__ __device__ constexpr int nu_yo(int T) { return 18 + T; }
+__host__ __device__ constexpr int nu_zo(int T) { return 25 + 2 * T; }
+__host__ __device__ constexpr int nu_rec(int T) { return (32 + 3 * T + 1) / 2 * 2; }
+constexpr int kNuZeros = 16;  // a block of zeros: the record of the slots that fill up a group
+__host__ __device__ constexpr int nu_list() { return (kNuBoxChunk + 8) * 4; }  // ints per warp
+
+__device__ __forceinline__ void nu_cp16(void* smem, const void* gmem) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem)
+               : "memory");
+}
+
+// val null (interpolation): no value in the record.  The zeros are set when the
+// buffer is allocated.
+template <int T>
+__global__ void __launch_bounds__(256) nu3_points(const __grid_constant__ NuGeom3 g, const int* __restrict__ idx,
+                                                  const double* __restrict__ pos, const double2* __restrict__ val,
+                                                  long long npts, double* __restrict__ rec) {
+  constexpr int R = nu_rec(T);
+  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < 3 * npts; e += (long long)gridDim.x * blockDim.x) {
+    const long long k = e / 3;
+    const int a = (int)(e - 3 * k);
+    const int j = idx[k];
+    const long long m = a == 0 ? g.mx : a == 1 ? g.my : g.mz;
+    const double t = nu_axis_t(pos[3ll * j + a], a == 0 ? g.lx : a == 1 ? g.ly : g.lz, m);
+    const double rt = round(t);
+    double* r = rec + k * R;
+    double* w = r + (a == 0 ? nu_xo(T) : a == 1 ? nu_yo(T) : nu_zo(T));
+    double o[T];
+    nu_phi_all<T>(g.f, t - rt, g.beta, g.i0b, o);
+#pragma unroll
+    for (int i = 0; i < T; ++i) w[i] = o[i];
+    int* c = reinterpret_cast<int*>(r + 2);
+    c[a] = (int)((long long)rt & (m - 1));
+    if (a == 0) {
+      const double2 v = val ? val[j] : make_double2(0.0, 0.0);
+      r[0] = v.x;
+      r[1] = v.y;
+      c[3] = j;
+    }
+  }
+}
+
+// D += A B: A 8 x 4 (row lane / 4, column lane % 4), B 4 x 8 (row lane % 4,
+// column lane / 4), D 8 x 8 (row lane / 4, columns 2 (lane % 4) and the next).
+__device__ __forceinline__ void nu_mma(double2& d, double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
+               : "+d"(d.x), "+d"(d.y)
+               : "d"(a), "d"(b));
+}
+
+// SPREAD: records -> cells (add: the cells may be shared with other CTAs);
+// else: cells -> out (zeroed by the caller).
+template <bool SPREAD>
+__global__ void __launch_bounds__(kNuBoxThreads, 3)
+    nu3_boxes(int mx, int my, int mz, int w, const int* __restrict__ off, const double* __restrict__ rec,
+              double2* __restrict__ grid, double2* __restrict__ out, int add) {
+  extern __shared__ __align__(16) double nu_sm[];
+  __shared__ int run_start[kNuBoxRuns], run_pre[kNuBoxRuns + 1];
+  const int T = 2 * w + 1, S = nu_rec(T);
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int nby = my / 8, nbz = mz / 16;
+  const int b = blockIdx.x;
+  const int gx0 = b / (nby * nbz) * 16, gy0 = b / nbz % nby * 8, gz0 = b % nbz * 16;
+  // candidate tiles (8 cells a side): rows along z are runs of the sorted points
+  const int tx = mx / 8, ty = my / 8, tz = mz / 8, wt = (w + 7) / 8;
+  const int cx = min(tx, 2 + 2 * wt), cy = min(ty, 1 + 2 * wt), cz = min(tz, 2 + 2 * wt);
+  const int bx = gx0 / 8 - wt, by = gy0 / 8 - wt, bz = (gz0 / 8 - wt) & (tz - 1);
+  const int nrun = cx * cy * 2;  // a run may wrap: two pieces
+  if (tid < nrun) {
+    const int row = tid >> 1;
+    const int base = (((bx + row / cy) & (tx - 1)) * ty + ((by + row % cy) & (ty - 1))) * tz;
+    const int first = min(cz, tz - bz);  // tiles before the wrap
+    const int lo = tid & 1 ? base : base + bz, hi = tid & 1 ? base + cz - first : base + bz + first;
+    run_start[tid] = off[lo];
+    run_pre[tid + 1] = off[hi] - off[lo];
+  }
+  const int ZB = 2 * kNuBoxChunk * S;  // the zero block
+  if (tid < kNuZeros) nu_sm[ZB + tid] = 0.0;
+  int4* const list = reinterpret_cast<int4*>(nu_sm + ZB + kNuZeros) + wid * (kNuBoxChunk + 8);
+  __syncthreads();
+  if (tid == 0) {
+    run_pre[0] = 0;
+    for (int i = 0; i < nrun; ++i) run_pre[i + 1] += run_pre[i];
+  }
+  __syncthreads();
+  const int total = run_pre[nrun];
+  const int nchunk = (total + kNuBoxChunk - 1) / kNuBoxChunk;
+  int c = blockIdx.y;
+  if (c >= nchunk) return;
+  // a few threads per record, 16 bytes a copy.  The points of a chunk are nchunk
+  // apart, so it samples all candidate tiles and the warps of the CTA meet about
+  // as many of its points each (in run order a chunk is a tile, which some boxes
+  // meet whole and others not at all)
+  auto stage = [&](int ch, int slot) {
+    constexpr int TPP = kNuBoxThreads / kNuBoxChunk;  // threads per record
+    const int p = tid / TPP, ord = p * nchunk + ch;
+    if (ord < total) {
+      int lo = 0, hi = nrun;  // last run with run_pre <= ord
+      while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (run_pre[mid] <= ord) lo = mid;
+        else hi = mid;
+      }
+      const double* r = rec + (long long)(run_start[lo] + ord - run_pre[lo]) * S;
+      double* d = nu_sm + (slot * kNuBoxChunk + p) * S;
+      for (int i = 2 * (tid % TPP); i < S; i += 2 * TPP) nu_cp16(d + i, r + i);
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+  // this warp's box; the lane's row and column in the products
+  const int x0 = gx0 + (wid >> 2) * 8, y0 = gy0 + ((wid >> 1) & 1) * 4, z0 = gz0 + (wid & 1) * 8;
+  const int lr = lane >> 2, lk = lane & 3;
+  stage(c, 0);
+  double2 acc[4][2];     // SPREAD: C[x = lr][z = 2 lk, 2 lk + 1] of row y, real and imaginary
+  double cell[4][2][2];  // else: B[x = lk + 4 s][z = lr] of row y, real and imaginary
+  const long long sx = (long long)my * mz;
+  if constexpr (SPREAD) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[j][0] = acc[j][1] = make_double2(0.0, 0.0);
+  } else {
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int s = 0; s < 2; ++s) {
+        const double2 v = grid[(x0 + 4 * s + lk) * sx + (long long)(y0 + j) * mz + z0 + lr];
+        cell[j][s][0] = v.x;
+        cell[j][s][1] = v.y;
+      }
+  }
+  bool any = false;
+  for (int k = 0; c < nchunk; ++k, c += gridDim.y) {
+    const int slot = k & 1;
+    if (c + (int)gridDim.y < nchunk) {
+      stage(c + gridDim.y, slot ^ 1);
+      asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+    } else {
+      asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    }
+    __syncthreads();
+    // the chunk's records that meet this box: offsets of its first weights (in
+    // doubles from nu_sm; a box may start up to seven zeros before a row)
+    int n = 0;
+#pragma unroll
+    for (int h = 0; h < kNuBoxChunk / 32; ++h) {
+      const int p = lane + 32 * h, rp = (slot * kNuBoxChunk + p) * S;
+      bool hit = false;
+      int4 e = make_int4(0, 0, 0, 0);
+      if (p * nchunk + c < total) {
+        const int4 cc = *reinterpret_cast<const int4*>(nu_sm + rp + 2);
+        const int dx = (x0 - cc.x + w) & (mx - 1), dy = (y0 - cc.y + w) & (my - 1), dz = (z0 - cc.z + w) & (mz - 1);
+        hit = (dx < T || dx > mx - 8) && (dy < T || dy > my - 4) && (dz < T || dz > mz - 8);
+        e = make_int4(rp + nu_xo(T) + (dx < T ? dx : dx - mx), rp + nu_yo(T) + (dy < T ? dy : dy - my),
+                      rp + nu_zo(T) + (dz < T ? dz : dz - mz), SPREAD ? rp : cc.w);
+      }
+      const unsigned mask = __ballot_sync(0xffffffffu, hit);
+      if (hit) list[n + __popc(mask & ((1u << lane) - 1))] = e;
+      n += __popc(mask);
+    }
+    any = any || n;
+    if (lane < 8) list[n + lane] = make_int4(ZB, ZB, ZB, SPREAD ? ZB : -1);  // fills up the last group
+    __syncwarp();
+    constexpr int G = SPREAD ? 4 : 8;
+#pragma unroll 2
+    for (int i = 0; i < n; i += G) {
+      const int4 e = list[i + (SPREAD ? lk : lr)];
+      if constexpr (SPREAD) {
+        const double2 v = *reinterpret_cast<const double2*>(nu_sm + e.w);
+        const double wz = nu_sm[e.z + lr], ax = nu_sm[e.x + lr];
+        const double vr = v.x * wz, vi = v.y * wz;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const double wy = nu_sm[e.y + j];
+          nu_mma(acc[j][0], ax, vr * wy);
+          nu_mma(acc[j][1], ax, vi * wy);
+        }
+      } else {
+        const double a0 = nu_sm[e.x + lk], a1 = nu_sm[e.x + 4 + lk];
+        const double w0 = nu_sm[e.z + 2 * lk], w1 = nu_sm[e.z + 2 * lk + 1];
+        double re = 0.0, im = 0.0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          double2 dr = make_double2(0.0, 0.0), di = dr;
+          nu_mma(dr, a0, cell[j][0][0]);
+          nu_mma(di, a0, cell[j][0][1]);
+          nu_mma(dr, a1, cell[j][1][0]);
+          nu_mma(di, a1, cell[j][1][1]);
+          const double wy = nu_sm[e.y + j];
+          re = fma(wy, fma(w1, dr.y, w0 * dr.x), re);
+          im = fma(wy, fma(w1, di.y, w0 * di.x), im);
+        }
+#pragma unroll
+        for (int o = 1; o < 4; o <<= 1) {
+          re += __shfl_xor_sync(0xffffffffu, re, o);
+          im += __shfl_xor_sync(0xffffffffu, im, o);
+        }
+        if (lk < 2 && e.w >= 0) atomicAdd(lk ? &out[e.w].y : &out[e.w].x, lk ? im : re);
+      }
+    }
+    __syncthreads();  // the slot is refilled
+  }
+  if constexpr (SPREAD) {
+    if (!any) return;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      double2* o = grid + (x0 + lr) * sx + (long long)(y0 + j) * mz + z0 + 2 * lk;
+      const double2 c0 = make_double2(acc[j][0].x, acc[j][1].x), c1 = make_double2(acc[j][0].y, acc[j][1].y);
+      if (add) {
+        atomicAdd(&o[0].x, c0.x);
+        atomicAdd(&o[0].y, c0.y);
+        atomicAdd(&o[1].x, c1.x);
+        atomicAdd(&o[1].y, c1.y);
+      } else {
+        o[0] = c0;
+        o[1] = c1;
+      }
+    }
+  }
+}
+
+// T: taps per axis at compile time.  A lane holds the point's x-weights in
+// registers and sums its (py, pz) columns over x first, two FMAs and one
+// shared-memory load per tap (with the weight product inside the loop and the
+// cell list checked at run time it was 936 instructions per lane and point at
+// w = 6).  The shared loads (4 wavefronts per 32 cells) bound it.
+template <int T>
+__global__ void __launch_bounds__(kNuTileThreads) nu3_interp_tiles(const __grid_constant__ NuGeom3 g, NuTiles tl,
                                                                     const double2* __restrict__ grid,
                                                                     const double* __restrict__ pos, double2* out) {
   extern __shared__ __align__(16) unsigned char nu_smem[];
   const int tile = blockIdx.x;
   const int start = tl.off[tile], end = tl.off[tile + 1];
   if (start == end) return;
-  const int T = 2 * g.w + 1, E = tl.E, E2 = E * E, E3 = E2 * E;
+  constexpr int IT = (T * T + 31) / 32, G4 = (T + 3) / 4;
+  const int E = tl.E, E2 = E * E, E3 = E2 * E;
   double2* cells = reinterpret_cast<double2*>(nu_smem);
   double* wts = reinterpret_cast<double*>(cells + E3);       // kNuChunk x 3 x T
   int* loc = reinterpret_cast<int*>(wts + kNuChunk * 3 * T);  // kNuChunk x 3
@@ -472,49 +933,54 @@ __global__ void __launch_bounds__(kNuTileThreads) nu3_interp_tiles(NuGeom3 g, Nu
     const int cx = c / E2, cy = (c / E) % E, cz = c % E;
     cells[c] = grid[(((gx0 + cx) & mxm) * g.my + ((gy0 + cy) & mym)) * g.mz + ((gz0 + cz) & mzm)];
   }
-  const NuLaneCells lc(T, lane);
-  int coff[kNuTileIters];
+  int coff[IT];  // the lane's columns; past the plane: column 0 with weight 0
 #pragma unroll
-  for (int it = 0; it < kNuTileIters; ++it) coff[it] = lc.pyz[it] >= 0 ? (lc.pyz[it] >> 8) * E + (lc.pyz[it] & 255) : 0;
+  for (int it = 0; it < IT; ++it) {
+    const int f = it * 32 + lane;
+    coff[it] = f < T * T ? (f / T) * E + f % T : 0;
+  }
   for (int base = start; base < end; base += kNuChunk) {
     const int cnt = min(kNuChunk, end - base);
     __syncthreads();  // cells loaded / previous chunk's weights consumed
-    // the chunk's 3T axis weights per point over all threads of the CTA
-    for (int e = threadIdx.x; e < cnt * 3 * T; e += kNuTileThreads) {
-      const int p = e / (3 * T), r = e - p * 3 * T, a = r / T, tap = r - a * T;
-      const long long j = tl.idx[base + p];
-      wts[e] = nu_tile_weight(g, tl, tc, pos + 3 * j, a, tap, tap == 0 ? &loc[p * 3 + a] : nullptr);
+    // the chunk's axis weights, four taps of one point and axis per thread
+    for (int e = threadIdx.x; e < cnt * 3 * G4; e += kNuTileThreads) {
+      const int p = e / (3 * G4), r = e - p * 3 * G4, a = r / G4, t0 = (r - a * G4) * 4;
+      const double* ps = pos + 3 * (long long)tl.idx[base + p];
+      const long long m = a == 0 ? g.mx : a == 1 ? g.my : g.mz;
+      const double t = nu_axis_t(ps[a], a == 0 ? g.lx : a == 1 ? g.ly : g.lz, m);
+      const double rt = round(t);
+      if (t0 == 0) loc[p * 3 + a] = (int)((long long)rt & (m - 1)) - (a == 0 ? tc.tx : a == 1 ? tc.ty : tc.tz) * tl.B;
+      double o[4];
+      nu_phi4(g.f, t0, t - rt, g.w, g.beta, g.i0b, o);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (t0 + i < T) wts[p * 3 * T + a * T + t0 + i] = o[i];
     }
     __syncthreads();
     for (int p = wid; p < cnt; p += kNuTileWarps) {
-      const double* wx = wts + p * 3 * T;
-      const double* wy = wx + T;
-      const double* wz = wy + T;
-      double wyz[kNuTileIters];
+      const double* wp = wts + p * 3 * T;
+      double wx[T];
 #pragma unroll
-      for (int it = 0; it < kNuTileIters; ++it)
-        wyz[it] = lc.pyz[it] >= 0 ? wy[lc.pyz[it] >> 8] * wz[lc.pyz[it] & 255] : 0.0;
-      // two accumulator pairs (even / odd cells) halve the dependent FMA chain
-      double ax0 = 0.0, ay0 = 0.0, ax1 = 0.0, ay1 = 0.0;
-      const double2* plane = cells + loc[p * 3] * E2 + loc[p * 3 + 1] * E + loc[p * 3 + 2];
-      for (int px = 0; px < T; ++px, plane += E2) {
-        const double wxv = wx[px];
+      for (int i = 0; i < T; ++i) wx[i] = wp[i];
+      double ax = 0.0, ay = 0.0;
+      const double2* corner = cells + loc[p * 3] * E2 + loc[p * 3 + 1] * E + loc[p * 3 + 2];
 #pragma unroll
-        for (int it = 0; it < kNuTileIters; ++it) {
-          if (lc.pyz[it] >= 0) {
-            const double wt = wxv * wyz[it];
-            const double2 c = plane[coff[it]];
-            if (it & 1) {
-              ax1 += c.x * wt;
-              ay1 += c.y * wt;
-            } else {
-              ax0 += c.x * wt;
-              ay0 += c.y * wt;
-            }
-          }
+      for (int it = 0; it < IT; ++it) {
+        const int f = it * 32 + lane;
+        const double wyz = f < T * T ? wp[T + f / T] * wp[2 * T + f % T] : 0.0;
+        const double2* col = corner + coff[it];
+        double sx = 0.0, sy = 0.0;
+#pragma unroll
+        for (int px = 0; px < T; ++px) {
+          const double2 c = col[px * E2];
+          sx = fma(wx[px], c.x, sx);
+          sy = fma(wx[px], c.y, sy);
+        }
+        if (f < T * T) {
+          ax = fma(wyz, sx, ax);
+          ay = fma(wyz, sy, ay);
         }
       }
-      double ax = ax0 + ax1, ay = ay0 + ay1;
       for (int o = 16; o > 0; o >>= 1) {
         ax += __shfl_xor_sync(0xffffffffu, ax, o);
         ay += __shfl_xor_sync(0xffffffffu, ay, o);
@@ -550,10 +1016,44 @@ static unsigned nu_grid(long long work) {
   return (unsigned)b;
 }
 
-cudaError_t nufft_spread_dev(const NuLaunch& L, const double* pos, const void* val, long long npts, void* grid,
-                             cudaStream_t st) {
+// Sorting costs three passes over the points (about 60 us per million); below
+// about a million taps, or when the window of 32 cells leaves few centre cells,
+// the direct atomics are faster unless the points crowd the grid.
+bool nufft_sorted(const NuLaunch& L, long long npts) {
+  const long long T = 2 * L.w + 1;
+  return T <= 25 && L.m >= 64 && L.m < (1ll << 31) - 64 && npts <= INT32_MAX &&
+         (npts * T >= (1 << 21) || (npts >= 16 * L.m && npts >= 4096));
+}
+
+cudaError_t nufft_spread_dev(const NuLaunch& L, const NuTileLaunch& TL, const double* pos, const void* val,
+                             long long npts, void* grid, cudaStream_t st) {
   if (npts <= 0) return cudaSuccess;
-  const NuGeom g{L.m, L.w, L.beta, L.i0b, L.len};
+  const NuGeom g{L.m, L.w, L.beta, L.i0b, L.len, L.f};
+  if (TL.idx && nufft_sorted(L, npts)) {
+    const int width = nufft_bin_width(L.m), bins = (int)((L.m + width - 1) / width);
+    cudaError_t e = cudaMemsetAsync(TL.cnt, 0, (size_t)bins * sizeof(int), st);
+    if (e != cudaSuccess) return e;
+    nu1_bin<<<nu_grid(npts), 256, 0, st>>>(g, width, pos, npts, TL.cnt, TL.tile, TL.rank);
+    nu3_scan<<<1, 1024, 0, st>>>(TL.cnt, TL.off, bins);
+    nu3_scatter<<<nu_grid(npts), 256, 0, st>>>(TL.tile, TL.rank, TL.off, npts, TL.idx);
+    const size_t smem = nu1_smem(2 * L.w + 1);
+    auto k = nu1_spread<0>;
+    switch (L.w) {
+      case 4: k = nu1_spread<9>; break;
+      case 5: k = nu1_spread<11>; break;
+      case 6: k = nu1_spread<13>; break;
+      case 7: k = nu1_spread<15>; break;
+      case 8: k = nu1_spread<17>; break;
+      default: break;
+    }
+    e = kernel_smem_grant(reinterpret_cast<const void*>(k), smem);
+    if (e != cudaSuccess) return e;
+    const long long blocks = (npts + 32 * kNu1Warps - 1) / (32 * kNu1Warps);
+    k<<<(unsigned)std::min<long long>(blocks, 1 << 20), 32 * kNu1Warps, smem, st>>>(
+        g, TL.idx, pos, static_cast<const double2*>(val), npts, static_cast<double2*>(grid));
+    count_launch(4);
+    return cudaGetLastError();
+  }
   nu_spread<<<nu_grid(npts), 256, 0, st>>>(g, pos, static_cast<const double2*>(val), npts, static_cast<double2*>(grid));
   count_launch(1);
   return cudaGetLastError();
@@ -562,8 +1062,17 @@ cudaError_t nufft_spread_dev(const NuLaunch& L, const double* pos, const void* v
 cudaError_t nufft_interp_dev(const NuLaunch& L, const void* grid, const double* pos, long long npts, void* out,
                              cudaStream_t st) {
   if (npts <= 0) return cudaSuccess;
-  const NuGeom g{L.m, L.w, L.beta, L.i0b, L.len};
-  nu_interp<<<nu_grid(npts), 256, 0, st>>>(g, static_cast<const double2*>(grid), pos, npts, static_cast<double2*>(out));
+  const NuGeom g{L.m, L.w, L.beta, L.i0b, L.len, L.f};
+  auto k = nu_interp<0>;
+  switch (L.w) {
+    case 4: k = nu_interp<9>; break;
+    case 5: k = nu_interp<11>; break;
+    case 6: k = nu_interp<13>; break;
+    case 7: k = nu_interp<15>; break;
+    case 8: k = nu_interp<17>; break;
+    default: break;
+  }
+  k<<<nu_grid(npts), 256, 0, st>>>(g, static_cast<const double2*>(grid), pos, npts, static_cast<double2*>(out));
   count_launch(1);
   return cudaGetLastError();
 }
@@ -584,7 +1093,7 @@ cudaError_t nufft_place_coeffs_dev(const void* coeffs, const double* deconv, lon
 }
 
 static NuGeom3 geom3(const NuLaunch3& L) {
-  return NuGeom3{L.mx, L.my, L.mz, L.w, L.beta, L.i0b, L.lx, L.ly, L.lz};
+  return NuGeom3{L.mx, L.my, L.mz, L.w, L.beta, L.i0b, L.lx, L.ly, L.lz, L.f};
 }
 
 static unsigned nu_warp_grid(long long npts) {
@@ -633,6 +1142,69 @@ size_t nufft3_tile_smem(int B, int w) {
   return cells + kNuChunk * 3 * T * sizeof(double) + kNuChunk * 3 * sizeof(int);
 }
 
+// The box kernel serves grids whose axes hold a kernel and a box side by side
+// (a padded x row is not periodic) and whose candidate runs fit its table.
+bool nufft3_boxes(const NuLaunch3& L) {
+  const long long lo = std::min(L.mx, std::min(L.my, L.mz)), hi = std::max(L.mx, std::max(L.my, L.mz));
+  const int T = 2 * L.w + 1, wt = (L.w + 7) / 8;
+  return lo >= 16 && lo >= T + 8 && hi < (1 << 20) && (2 + 2 * wt) * (1 + 2 * wt) * 2 <= kNuBoxRuns &&
+         nufft3_box_smem(L.w) <= 112 * 1024;
+}
+size_t nufft3_box_smem(int w) {
+  return ((size_t)2 * kNuBoxChunk * nu_rec(2 * w + 1) + kNuZeros) * sizeof(double) +
+         (size_t)(kNuBoxThreads / 32) * nu_list() * sizeof(int);
+}
+size_t nufft3_rec_bytes(int w) { return (size_t)nu_rec(2 * w + 1) * sizeof(double); }
+
+// Spreads npts points onto the zeroed grid, or interpolates the grid at them
+// into out; kNu3Slice points at a time (their records take nufft3_rec_bytes each).
+cudaError_t nufft3_boxes_dev(const NuLaunch3& L, const NuTileLaunch& TL, bool spread, const double* pos,
+                             const void* val, long long npts, void* grid, void* out, cudaStream_t st) {
+  const NuGeom3 g = geom3(L);
+  const int nty = (int)(L.my / 8), ntz = (int)(L.mz / 8), ntiles = (int)(L.mx / 8) * nty * ntz;
+  const size_t smem = nufft3_box_smem(L.w);
+  auto k = spread ? nu3_boxes<true> : nu3_boxes<false>;
+  cudaError_t e = kernel_smem_grant(reinterpret_cast<const void*>(k), smem);
+  if (e != cudaSuccess) return e;
+  if (!spread && npts > 0) {
+    e = cudaMemsetAsync(out, 0, (size_t)npts * 16, st);
+    if (e != cudaSuccess) return e;
+  }
+  const int boxes = (int)(L.mx / 16) * (int)(L.my / 8) * (int)(L.mz / 16);
+  for (long long p0 = 0; p0 < npts; p0 += kNu3Slice) {
+    const long long n = std::min<long long>(kNu3Slice, npts - p0);
+    const double* ps = pos + 3 * p0;
+    e = cudaMemsetAsync(TL.cnt, 0, (size_t)ntiles * sizeof(int), st);
+    if (e != cudaSuccess) return e;
+    nu3_bin<<<nu_grid(n), 256, 0, st>>>(g, 8, nty, ntz, ps, n, TL.cnt, TL.tile, TL.rank);
+    nu3_scan<<<1, 1024, 0, st>>>(TL.cnt, TL.off, ntiles);
+    nu3_scatter<<<nu_grid(n), 256, 0, st>>>(TL.tile, TL.rank, TL.off, n, TL.idx);
+    void (*points)(const NuGeom3, const int*, const double*, const double2*, long long, double*) = nullptr;
+    switch (L.w) {  // nufft3_tile_size: 2 <= w <= 9
+      case 2: points = nu3_points<5>; break;
+      case 3: points = nu3_points<7>; break;
+      case 4: points = nu3_points<9>; break;
+      case 5: points = nu3_points<11>; break;
+      case 6: points = nu3_points<13>; break;
+      case 7: points = nu3_points<15>; break;
+      case 8: points = nu3_points<17>; break;
+      case 9: points = nu3_points<19>; break;
+      default: return cudaErrorInvalidValue;
+    }
+    points<<<nu_grid(3 * n), 256, 0, st>>>(g, TL.idx, ps, spread ? static_cast<const double2*>(val) + p0 : nullptr, n,
+                                           TL.rec);
+    // a box's chunks are dealt to `split` CTAs: about 4096 CTAs in all, so a
+    // grid of few boxes, or points crowded into some of them, still fills the chip
+    const long long chunks = (n + kNuBoxChunk - 1) / kNuBoxChunk;
+    const int split = (int)std::max<long long>(1, std::min<long long>(chunks, std::min(32, 4096 / boxes)));
+    k<<<dim3((unsigned)boxes, (unsigned)split), kNuBoxThreads, smem, st>>>(
+        (int)L.mx, (int)L.my, (int)L.mz, L.w, TL.off, TL.rec, static_cast<double2*>(grid),
+        spread ? nullptr : static_cast<double2*>(out) + p0, split > 1 || npts > kNu3Slice);
+    count_launch(5);
+  }
+  return cudaGetLastError();
+}
+
 cudaError_t nufft3_tiled_dev(const NuLaunch3& L, const NuTileLaunch& TL, bool spread, const double* pos,
                              const void* src, long long npts, void* dst, cudaStream_t st) {
   if (npts <= 0) return cudaSuccess;
@@ -651,10 +1223,21 @@ cudaError_t nufft3_tiled_dev(const NuLaunch3& L, const NuTileLaunch& TL, bool sp
     nu3_spread_tiles<<<ntiles, kNuTileThreads, smem, st>>>(g, tl, pos, static_cast<const double2*>(src),
                                                            static_cast<double2*>(dst));
   } else {
-    e = kernel_smem_grant(reinterpret_cast<const void*>(nu3_interp_tiles), smem);
+    void (*k)(const NuGeom3, NuTiles, const double2*, const double*, double2*) = nullptr;
+    switch (L.w) {  // nufft3_tile_size: 2 <= w <= 9
+      case 2: k = nu3_interp_tiles<5>; break;
+      case 3: k = nu3_interp_tiles<7>; break;
+      case 4: k = nu3_interp_tiles<9>; break;
+      case 5: k = nu3_interp_tiles<11>; break;
+      case 6: k = nu3_interp_tiles<13>; break;
+      case 7: k = nu3_interp_tiles<15>; break;
+      case 8: k = nu3_interp_tiles<17>; break;
+      case 9: k = nu3_interp_tiles<19>; break;
+      default: return cudaErrorInvalidValue;
+    }
+    e = kernel_smem_grant(reinterpret_cast<const void*>(k), smem);
     if (e != cudaSuccess) return e;
-    nu3_interp_tiles<<<ntiles, kNuTileThreads, smem, st>>>(g, tl, static_cast<const double2*>(src), pos,
-                                                           static_cast<double2*>(dst));
+    k<<<ntiles, kNuTileThreads, smem, st>>>(g, tl, static_cast<const double2*>(src), pos, static_cast<double2*>(dst));
   }
   count_launch(4);
   return cudaGetLastError();

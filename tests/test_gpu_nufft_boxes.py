@@ -1,0 +1,61 @@
+"""NUFFT spreading and interpolation where the box kernel, its padded weight
+rows, its candidate runs and the polynomial kernel can go wrong: every kernel
+width, grids one box wide and up, crowded points (a box's points split over
+CTAs), points on cell boundaries, against the reference algorithm restated in
+numpy."""
+import numpy as np
+import pytest
+import torch
+
+from conftest import rel_l2
+from oracle.nufft import RefPlan, RefPlan3
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("shape,w,npts,layout", [
+    ((16, 16, 16), 2, 500, "uniform"), ((16, 16, 16), 4, 500, "uniform"), ((16, 9, 16), 5, 700, "cells"),
+    ((16, 16, 16), 6, 3000, "dense"), ((10, 17, 33), 6, 2500, "uniform"), ((33, 16, 12), 7, 1500, "cells"),
+    ((20, 16, 9), 8, 800, "dense"), ((16, 16, 16), 9, 300, "uniform"), ((16, 12, 16), 6, 1, "uniform"),
+    ((40, 20, 16), 3, 4000, "dense"),
+])
+def test_3d_boxes(afc, oracle, cuda, shape, w, npts, layout):
+    from apollofft_b200.nufft import NufftPlan3D
+    rng = np.random.default_rng(npts + w)
+    spacing = (0.5, 0.25, 1.0)
+    ref = RefPlan3(shape, spacing, 2, w)
+    L = np.array([n * d for n, d in zip(shape, spacing)])
+    u = rng.uniform(-0.3, 1.3, (npts, 3))
+    if layout == "dense":
+        u = 0.5 + 0.03 * rng.standard_normal((npts, 3))
+    if layout == "cells":  # on cells and half way between them
+        m = np.array(ref.m)
+        u = np.round(u * m * 2) / (2 * m)
+    pos = np.ascontiguousarray(u * L)
+    val = rng.standard_normal(npts) + 1j * rng.standard_normal(npts)
+    modes = rng.standard_normal(shape) + 1j * rng.standard_normal(shape)
+    plan = NufftPlan3D(shape, spacing, 2, w)
+    p_t = torch.from_numpy(pos).cuda()
+    y1 = plan.type1(p_t, torch.from_numpy(val).cuda()).cpu().numpy()
+    y2 = plan.type2(torch.from_numpy(modes).cuda(), p_t).cpu().numpy()
+    # sums of (2w + 1)^3 rounded products per point
+    assert rel_l2(y1, ref.type1(pos, val, oracle)) < 1e-12
+    assert rel_l2(y2, ref.type2(modes, pos, oracle)) < 1e-12
+
+
+@pytest.mark.parametrize("n,w,npts", [(1, 2, 5), (3, 6, 40), (64, 4, 1000), (257, 6, 3001), (1000, 8, 500), (50, 13, 64),
+                                      (40, 20, 64)])
+def test_1d_widths(afc, oracle, cuda, n, w, npts):
+    from apollofft_b200.nufft import NufftPlan1D
+    rng = np.random.default_rng(n + w)
+    ref = RefPlan(n, 0.3, 2, w)
+    pos = rng.uniform(-0.5 * n * 0.3, 1.5 * n * 0.3, npts)
+    pos[: npts // 4] = np.round(pos[: npts // 4] / 0.15) * 0.15  # on cells
+    val = rng.standard_normal(npts) + 1j * rng.standard_normal(npts)
+    coef = rng.standard_normal(n) + 1j * rng.standard_normal(n)
+    plan = NufftPlan1D(n, 0.3, 2, w)
+    p_t = torch.from_numpy(pos).cuda()
+    y1 = plan.type1(p_t, torch.from_numpy(val).cuda()).cpu().numpy()
+    y2 = plan.type2(torch.from_numpy(coef).cuda(), p_t).cpu().numpy()
+    assert rel_l2(y1, ref.type1(pos, val, oracle)) < 1e-12
+    assert rel_l2(y2, ref.type2(coef, pos, oracle)) < 1e-12
