@@ -3068,14 +3068,13 @@ afc_status afc_nufft3d_plan_create(afc_nufft3d_plan* out, int64_t nx, int64_t ny
 
 // Grows the per-point tile buffers (synchronous allocation) when a call brings
 // more points than any call before it; false -> the per-point kernels run.
-static afc_status nu3_reserve_records(afc_nufft3d_plan_s& p, int64_t npts, cudaStream_t st) {
+static afc_status nu3_reserve_records(afc_nufft3d_plan_s& p, int64_t npts) {
   const int64_t n = std::min<int64_t>(npts, kNu3Slice);
   if (n <= p.rec_cap) return AFC_OK;
   if (p.tiles.rec) cudaFree(p.tiles.rec);
   p.tiles.rec = nullptr;
   p.rec_cap = 0;
   AFC_CUDA(dev_alloc((void**)&p.tiles.rec, (size_t)n * nufft3_rec_bytes(p.w)), "NUFFT point records");
-  AFC_CUDA(cudaMemsetAsync(p.tiles.rec, 0, (size_t)n * nufft3_rec_bytes(p.w), st), "NUFFT point records");
   p.rec_cap = n;
   return AFC_OK;
 }
@@ -3129,7 +3128,7 @@ afc_status afc_nufft3d_type1(afc_nufft3d_plan plan, const double* positions, con
   afc_status r = nu3_reserve(*plan, npts, &tiled);
   if (r != AFC_OK) return r;
   if (tiled && nufft3_boxes(L)) {
-    r = nu3_reserve_records(*plan, npts, st);
+    r = nu3_reserve_records(*plan, npts);
     if (r != AFC_OK) return r;
     AFC_CUDA(nufft3_boxes_dev(L, plan->tiles, true, positions, values, npts, plan->grid, nullptr, st), "NUFFT spread");
   } else if (tiled)
@@ -3166,7 +3165,7 @@ afc_status afc_nufft3d_type2(afc_nufft3d_plan plan, const void* modes, const dou
   s = nu3_reserve(*plan, npts, &tiled);
   if (s != AFC_OK) return s;
   if (tiled && nufft3_boxes(L)) {
-    s = nu3_reserve_records(*plan, npts, st);
+    s = nu3_reserve_records(*plan, npts);
     if (s != AFC_OK) return s;
     AFC_CUDA(nufft3_boxes_dev(L, plan->tiles, false, positions, nullptr, npts, plan->grid, out, st),
              "NUFFT interpolation");

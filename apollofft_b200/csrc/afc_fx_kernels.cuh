@@ -9,16 +9,18 @@
 namespace afc {
 
 // CTAs per SM a kernel is built for.  16 points are 32 (complex64) or 64
-// (complex128) registers; 768 threads leave 80 registers, 512 leave 128.  The
-// odd lengths hold at most 10 points: 1024 threads of 64 registers.
-template <class T, int N> constexpr int fx_min_ctas(int threads) {
+// (complex128) registers; 1024 threads leave 64 registers, 768 80, 512 128.
+// Complex64 rows fit 64 without spills (16384 x 4096 both ways 391 -> 369 us);
+// the columns' strides and the convolution's second network do not (8 x 2^20
+// 151 -> 164 us) and keep 80.  The odd lengths hold at most 10 points.
+template <class T, int N, int FORM, int MODE> constexpr int fx_min_ctas(int threads) {
   if (!fx_pow2(N)) return (sizeof(T) == 4 ? 1024 : 512) / ((threads + 31) / 32 * 32);
   if (threads > 256) return sizeof(T) == 4 ? 2 : 1;
-  return (sizeof(T) == 4 ? 3 : 2) * (256 / threads);
+  return (sizeof(T) == 8 ? 2 : FORM == FX_ROWS && MODE != FX_CONV ? 4 : 3) * (256 / threads);
 }
 
 template <class T, int N, int FORM, int MODE, int IN, int OUT, bool HALF>
-__global__ void __launch_bounds__(FxTile<T, N, FORM>::threads, fx_min_ctas<T, N>(FxTile<T, N, FORM>::threads))
+__global__ void __launch_bounds__(FxTile<T, N, FORM>::threads, fx_min_ctas<T, N, FORM, MODE>(FxTile<T, N, FORM>::threads))
     fx_kernel(const __grid_constant__ KArgs<T> a) {
   extern __shared__ __align__(16) unsigned char smraw[];
   constexpr int L = FxTile<T, N, FORM>::L;
@@ -112,14 +114,16 @@ template <class T> static FxEntry fx_lookup(const LaunchDesc& d) {
   return FxEntry{};
 }
 
-// Programmatic stream serialization for launches of at most one wave: their
-// CTAs set up while the previous launch drains.
-static bool fx_pdl(long long grid, int threads) {
+// Programmatic stream serialization: a launch's CTAs set up while the previous
+// one drains, and none reads anything before that one has completed (every
+// thread waits first).  256^3 complex128 both ways 518 -> 504 us, 16384 x 4096
+// complex64 391 -> 381, 4096 CZTs 99 -> 96.  AFC_PDL=0 launches plainly.
+static bool fx_pdl() {
   static const int pdl_env = [] {
     const char* e = getenv("AFC_PDL");
     return e && *e ? atoi(e) : 1;
   }();
-  return pdl_env >= 2 || (pdl_env == 1 && grid * threads <= 148LL * 512);
+  return pdl_env != 0;
 }
 
 template <class T> static cudaError_t launch_fx_t(const LaunchDesc& d, cudaStream_t st) {
@@ -139,7 +143,7 @@ template <class T> static cudaError_t launch_fx_t(const LaunchDesc& d, cudaStrea
   cfg.dynamicSmemBytes = e.smem;
   cfg.stream = st;
   cfg.attrs = attr;
-  cfg.numAttrs = fx_pdl(grid, e.threads) ? 1 : 0;
+  cfg.numAttrs = fx_pdl() ? 1 : 0;
   ce = cudaLaunchKernelExC(&cfg, e.k, args);
   count_launch(1);
   return ce;

@@ -242,7 +242,7 @@ struct NuTileLaunch {
   int* tile = nullptr;  // npts
   int* rank = nullptr;  // npts
   int* idx = nullptr;   // npts
-  double* rec = nullptr;  // box kernels: a record per point of a slice, zeroed when allocated
+  double* rec = nullptr;  // box kernels: a record per point of a slice
 };
 // Points the box kernels take at a time (bounds their record buffer).
 constexpr long long kNu3Slice = 1 << 18;

@@ -691,41 +691,54 @@ __host__ __device__ constexpr int nu_yo(int T) { return 18 + T; }
 __host__ __device__ constexpr int nu_zo(int T) { return 25 + 2 * T; }
 __host__ __device__ constexpr int nu_rec(int T) { return (32 + 3 * T + 1) / 2 * 2; }
 constexpr int kNuZeros = 16;  // a block of zeros: the record of the slots that fill up a group
-__host__ __device__ constexpr int nu_list() { return (kNuBoxChunk + 8) * 4; }  // ints per warp
+__host__ __device__ constexpr int nu_list() { return (kNuBoxChunk + 16) * 4; }  // ints per warp
 
 __device__ __forceinline__ void nu_cp16(void* smem, const void* gmem) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem)
                : "memory");
 }
 
-// val null (interpolation): no value in the record.  The zeros are set when the
-// buffer is allocated.
+// Block of kNuPts points, three threads each (one per axis): the records are put
+// together in shared memory and stored whole (rows written straight to global
+// memory were 13 eight-byte stores per thread to 32 places each: 97 us at 2^18
+// points).  val null (interpolation): no value in the record.
+constexpr int kNuPts = 64;
 template <int T>
-__global__ void __launch_bounds__(256) nu3_points(const __grid_constant__ NuGeom3 g, const int* __restrict__ idx,
-                                                  const double* __restrict__ pos, const double2* __restrict__ val,
-                                                  long long npts, double* __restrict__ rec) {
+__global__ void __launch_bounds__(3 * kNuPts) nu3_points(const __grid_constant__ NuGeom3 g, const int* __restrict__ idx,
+                                                         const double* __restrict__ pos,
+                                                         const double2* __restrict__ val, int npts,
+                                                         double* __restrict__ rec) {
   constexpr int R = nu_rec(T);
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < 3 * npts; e += (long long)gridDim.x * blockDim.x) {
-    const long long k = e / 3;
-    const int a = (int)(e - 3 * k);
-    const int j = idx[k];
-    const long long m = a == 0 ? g.mx : a == 1 ? g.my : g.mz;
-    const double t = nu_axis_t(pos[3ll * j + a], a == 0 ? g.lx : a == 1 ? g.ly : g.lz, m);
-    const double rt = round(t);
-    double* r = rec + k * R;
-    double* w = r + (a == 0 ? nu_xo(T) : a == 1 ? nu_yo(T) : nu_zo(T));
-    double o[T];
-    nu_phi_all<T>(g.f, t - rt, g.beta, g.i0b, o);
+  __shared__ __align__(16) double sm[kNuPts * R];
+  for (int i = threadIdx.x; i < kNuPts * R; i += 3 * kNuPts) sm[i] = 0.0;
+  const int p = threadIdx.x / 3, a = threadIdx.x - 3 * p;
+  for (int base = blockIdx.x * kNuPts; base < npts; base += gridDim.x * kNuPts) {
+    const int cnt = min(kNuPts, npts - base);
+    __syncthreads();  // zeroed / the previous records are stored
+    if (p < cnt) {
+      const int j = idx[base + p];
+      const long long m = a == 0 ? g.mx : a == 1 ? g.my : g.mz;
+      const double t = nu_axis_t(pos[3ll * j + a], a == 0 ? g.lx : a == 1 ? g.ly : g.lz, m);
+      const double rt = round(t);
+      double* r = sm + p * R;
+      double* w = r + (a == 0 ? nu_xo(T) : a == 1 ? nu_yo(T) : nu_zo(T));
+      double o[T];
+      nu_phi_all<T>(g.f, t - rt, g.beta, g.i0b, o);
 #pragma unroll
-    for (int i = 0; i < T; ++i) w[i] = o[i];
-    int* c = reinterpret_cast<int*>(r + 2);
-    c[a] = (int)((long long)rt & (m - 1));
-    if (a == 0) {
-      const double2 v = val ? val[j] : make_double2(0.0, 0.0);
-      r[0] = v.x;
-      r[1] = v.y;
-      c[3] = j;
+      for (int i = 0; i < T; ++i) w[i] = o[i];
+      int* c = reinterpret_cast<int*>(r + 2);
+      c[a] = (int)((long long)rt & (m - 1));
+      if (a == 0) {
+        const double2 v = val ? val[j] : make_double2(0.0, 0.0);
+        r[0] = v.x;
+        r[1] = v.y;
+        c[3] = j;
+      }
     }
+    __syncthreads();
+    const double2* s2 = reinterpret_cast<const double2*>(sm);
+    double2* d2 = reinterpret_cast<double2*>(rec + (long long)base * R);
+    for (int i = threadIdx.x; i < cnt * R / 2; i += 3 * kNuPts) d2[i] = s2[i];
   }
 }
 
@@ -765,7 +778,7 @@ __global__ void __launch_bounds__(kNuBoxThreads, 3)
   }
   const int ZB = 2 * kNuBoxChunk * S;  // the zero block
   if (tid < kNuZeros) nu_sm[ZB + tid] = 0.0;
-  int4* const list = reinterpret_cast<int4*>(nu_sm + ZB + kNuZeros) + wid * (kNuBoxChunk + 8);
+  int4* const list = reinterpret_cast<int4*>(nu_sm + ZB + kNuZeros) + wid * (kNuBoxChunk + 16);
   __syncthreads();
   if (tid == 0) {
     run_pre[0] = 0;
@@ -846,12 +859,14 @@ __global__ void __launch_bounds__(kNuBoxThreads, 3)
       n += __popc(mask);
     }
     any = any || n;
-    if (lane < 8) list[n + lane] = make_int4(ZB, ZB, ZB, SPREAD ? ZB : -1);  // fills up the last group
+    // fills up the last group, and one group past it for the loop's look-ahead
+    if (lane < 16) list[n + lane] = make_int4(ZB, ZB, ZB, SPREAD ? ZB : -1);
     __syncwarp();
     constexpr int G = SPREAD ? 4 : 8;
+    int4 e = list[SPREAD ? lk : lr];
 #pragma unroll 2
     for (int i = 0; i < n; i += G) {
-      const int4 e = list[i + (SPREAD ? lk : lr)];
+      const int4 e_next = list[i + G + (SPREAD ? lk : lr)];
       if constexpr (SPREAD) {
         const double2 v = *reinterpret_cast<const double2*>(nu_sm + e.w);
         const double wz = nu_sm[e.z + lr], ax = nu_sm[e.x + lr];
@@ -884,6 +899,7 @@ __global__ void __launch_bounds__(kNuBoxThreads, 3)
         }
         if (lk < 2 && e.w >= 0) atomicAdd(lk ? &out[e.w].y : &out[e.w].x, lk ? im : re);
       }
+      e = e_next;
     }
     __syncthreads();  // the slot is refilled
   }
@@ -1179,7 +1195,7 @@ cudaError_t nufft3_boxes_dev(const NuLaunch3& L, const NuTileLaunch& TL, bool sp
     nu3_bin<<<nu_grid(n), 256, 0, st>>>(g, 8, nty, ntz, ps, n, TL.cnt, TL.tile, TL.rank);
     nu3_scan<<<1, 1024, 0, st>>>(TL.cnt, TL.off, ntiles);
     nu3_scatter<<<nu_grid(n), 256, 0, st>>>(TL.tile, TL.rank, TL.off, n, TL.idx);
-    void (*points)(const NuGeom3, const int*, const double*, const double2*, long long, double*) = nullptr;
+    void (*points)(const NuGeom3, const int*, const double*, const double2*, int, double*) = nullptr;
     switch (L.w) {  // nufft3_tile_size: 2 <= w <= 9
       case 2: points = nu3_points<5>; break;
       case 3: points = nu3_points<7>; break;
@@ -1191,8 +1207,8 @@ cudaError_t nufft3_boxes_dev(const NuLaunch3& L, const NuTileLaunch& TL, bool sp
       case 9: points = nu3_points<19>; break;
       default: return cudaErrorInvalidValue;
     }
-    points<<<nu_grid(3 * n), 256, 0, st>>>(g, TL.idx, ps, spread ? static_cast<const double2*>(val) + p0 : nullptr, n,
-                                           TL.rec);
+    points<<<(unsigned)((n + kNuPts - 1) / kNuPts), 3 * kNuPts, 0, st>>>(
+        g, TL.idx, ps, spread ? static_cast<const double2*>(val) + p0 : nullptr, (int)n, TL.rec);
     // a box's chunks are dealt to `split` CTAs: about 4096 CTAs in all, so a
     // grid of few boxes, or points crowded into some of them, still fills the chip
     const long long chunks = (n + kNuBoxChunk - 1) / kNuBoxChunk;
