@@ -415,31 +415,34 @@ struct AxisPlan {
 
 static afc_status build_axis(int64_t n, bool dbl, AxisPlan& ap, cudaStream_t st);
 
-// What the plans of one batch share while they are built: the two-pass plan of
-// each convolution length, and one scratch allocation for table FFTs (each was
+// What the plans of one batch share while they are built: the plans of each
+// convolution length, and scratch allocations for table FFTs (each was
 // allocated, waited for and freed per table).
 struct BuildShare {
-  std::map<int64_t, std::shared_ptr<AxisPlan>> sub;
-  void* scratch = nullptr;
-  size_t bytes = 0;
-  ~BuildShare() {
-    if (scratch) cudaFree(scratch);
-  }
-  // at least `need` bytes, or null; work already enqueued on the stream has
-  // finished with the old block before it is freed (cudaFree waits)
-  void* get(size_t need) {
-    if (need <= bytes) return scratch;
-    if (scratch) cudaFree(scratch);
-    scratch = nullptr;
-    bytes = 0;
-    if (dev_alloc(&scratch, need) != cudaSuccess) {
-      cudaGetLastError();
-      scratch = nullptr;
-      return nullptr;
+  std::map<int64_t, std::shared_ptr<AxisPlan>> sub, sub64;  // the plan's precision; FP64 for complex64 kernel spectra
+  struct Block {
+    void* p = nullptr;
+    size_t bytes = 0;
+    ~Block() {
+      if (p) cudaFree(p);
     }
-    bytes = need;
-    return scratch;
-  }
+    // at least `need` bytes, or null; work already enqueued on the stream has
+    // finished with the old block before it is freed (cudaFree waits)
+    void* get(size_t need) {
+      if (need <= bytes) return p;
+      if (p) cudaFree(p);
+      p = nullptr;
+      bytes = 0;
+      if (dev_alloc(&p, need) != cudaSuccess) {
+        cudaGetLastError();
+        p = nullptr;
+        return nullptr;
+      }
+      bytes = need;
+      return p;
+    }
+  };
+  Block ws, tables;  // FFT workspace; FP64 tables before they are narrowed
 };
 static thread_local BuildShare* tl_share = nullptr;
 
@@ -1001,7 +1004,7 @@ static afc_status fft_table(const AxisPlan& mp, bool dbl, void* buf, cudaStream_
   const bool own = !tl_share;
   if (wsb) {
     if (own) AFC_CUDA(dev_alloc(&ws, wsb), "table workspace");
-    else if (!(ws = tl_share->get(wsb))) return fail(AFC_ERR_OUT_OF_MEMORY, "table workspace: out of memory");
+    else if (!(ws = tl_share->ws.get(wsb))) return fail(AFC_ERR_OUT_OF_MEMORY, "table workspace: out of memory");
   }
   cudaError_t e = exec_axis(mp, dbl, false, io, ws, st);
   if (e == cudaSuccess && own) e = cudaStreamSynchronize(st);
@@ -1085,6 +1088,47 @@ static int64_t conv_length(int64_t need, size_t csz, bool bluestein) {
   return best;
 }
 
+// Spectra of a complex64 Bluestein kernel, both directions: chirp, kernel and
+// FFT in FP64, narrowed once (computed in FP32 the spectrum's own rounding was
+// about a fifth of the transform's error).
+static afc_status narrow_spectra(int64_t n, int64_t M, void* spec, cudaStream_t st) {
+  std::shared_ptr<AxisPlan> md;
+  afc_status s = AFC_OK;
+  if (tl_share && tl_share->sub64.count(M)) {
+    md = tl_share->sub64[M];
+  } else {
+    md.reset(new AxisPlan());
+    s = build_axis(M, true, *md, st);
+    if (s != AFC_OK) return s;
+    if (tl_share) tl_share->sub64[M] = md;
+  }
+  const size_t need = ((size_t)n + (size_t)M) * 16;
+  void* buf = nullptr;
+  if (tl_share) {
+    buf = tl_share->tables.get(need);
+    if (!buf) return fail(AFC_ERR_OUT_OF_MEMORY, "Bluestein tables: out of memory");
+  } else {
+    AFC_CUDA(dev_alloc(&buf, need), "Bluestein tables");
+  }
+  char* b = static_cast<char*>(buf);  // one kernel at a time, then the chirp
+  char* chirp = b + (size_t)M * 16;
+  cudaError_t e = gen_chirp_dev(chirp, n, true, st);
+  for (int inv = 0; inv < 2 && e == cudaSuccess && s == AFC_OK; ++inv) {
+    e = gen_bluestein_b_dev(b, chirp, n, M, inv != 0, true, st);
+    if (e == cudaSuccess) s = fft_table(*md, true, b, st);
+    if (e == cudaSuccess && s == AFC_OK)
+      e = narrow_table_dev(static_cast<char*>(spec) + (size_t)inv * M * 8, b, M, st);
+  }
+  if (!tl_share) {
+    cudaError_t es = cudaStreamSynchronize(st);
+    if (e == cudaSuccess) e = es;
+    cudaFree(buf);
+  }
+  if (s != AFC_OK) return s;
+  if (e != cudaSuccess) return cuda_fail(e, "Bluestein tables");
+  return AFC_OK;
+}
+
 static afc_status build_axis(int64_t n, bool dbl, AxisPlan& ap, cudaStream_t st) {
   const size_t csz = dbl ? 16 : 8;
   ap.n = n;
@@ -1136,15 +1180,21 @@ static afc_status build_axis(int64_t n, bool dbl, AxisPlan& ap, cudaStream_t st)
   AFC_CUDA(gen_chirp_dev(ap.chirp, n, dbl, st), "chirp");
   AFC_CUDA(dev_alloc(&ap.spec_f, 2 * (size_t)M * csz), "Bluestein spectrum");
   ap.spec_i = static_cast<char*>(ap.spec_f) + (size_t)M * csz;
-  AFC_CUDA(gen_bluestein_b_dev(ap.spec_f, ap.chirp, n, M, false, dbl, st), "Bluestein kernel");
-  AFC_CUDA(gen_bluestein_b_dev(ap.spec_i, ap.chirp, n, M, true, dbl, st), "Bluestein kernel");
-  afc_status s;
+  afc_status s = AFC_OK;
+  if (dbl) {
+    AFC_CUDA(gen_bluestein_b_dev(ap.spec_f, ap.chirp, n, M, false, true, st), "Bluestein kernel");
+    AFC_CUDA(gen_bluestein_b_dev(ap.spec_i, ap.chirp, n, M, true, true, st), "Bluestein kernel");
+  } else {
+    s = narrow_spectra(n, M, ap.spec_f, st);
+    if (s != AFC_OK) return s;
+  }
   // one tile up to 4096 points, else (8192 complex64 would still fit the
   // general engine's tile) the three compile-time passes
   if (plannable(M, csz) && !(M > 4096 && fx_conv_length(M))) {
     ap.conv_smem = true;
     s = build_lenplan(M, dbl, ap.lp, st);
     if (s != AFC_OK) return s;
+    if (!dbl) return AFC_OK;
     AxisPlan mp;
     mp.n = M;
     mp.algo = ALGO_SMEM;
@@ -1164,9 +1214,11 @@ static afc_status build_axis(int64_t n, bool dbl, AxisPlan& ap, cudaStream_t st)
     if (s != AFC_OK) return s;
     if (tl_share) tl_share->sub[M] = ap.sub;
   }
-  s = fft_table(*ap.sub, dbl, ap.spec_f, st);
-  if (s == AFC_OK) s = fft_table(*ap.sub, dbl, ap.spec_i, st);
-  if (s != AFC_OK) return s;
+  if (dbl) {
+    s = fft_table(*ap.sub, dbl, ap.spec_f, st);
+    if (s == AFC_OK) s = fft_table(*ap.sub, dbl, ap.spec_i, st);
+    if (s != AFC_OK) return s;
+  }
   // the fused middle pass reads each row k1 of the spectrum contiguously
   AFC_CUDA(dev_alloc(&ap.spec_rf, 2 * (size_t)M * csz), "Bluestein spectrum");
   ap.spec_ri = static_cast<char*>(ap.spec_rf) + (size_t)M * csz;  // same allocation

@@ -317,6 +317,7 @@ cudaError_t czt_inverse_dev(const void* spec, void* out, const void* nodes, cons
 cudaError_t stft_ola_dev(const void* frames, const void* window, long long nframes, long long flen, long long hop,
                          long long nsig, void* out, bool dbl, cudaStream_t st);
 cudaError_t gen_row_spectrum_dev(void* dst, const void* src, long long N1, long long N2, bool dbl, cudaStream_t st);
+cudaError_t narrow_table_dev(void* dst, const void* src, long long cnt, cudaStream_t st);
 cudaError_t gen_stage_twiddles_dev(void* tw, const StageList& sl, bool dbl, cudaStream_t st);
 cudaError_t gen_roots_dev(void* out, long long cnt, long long mult, long long N, bool dbl, cudaStream_t st);
 cudaError_t gen_chirp_dev(void* out, long long n, bool dbl, cudaStream_t st);

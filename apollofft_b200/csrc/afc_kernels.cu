@@ -561,6 +561,14 @@ __global__ void gen_rader_b(typename CT<T>::type* b, const int* scatter, long lo
   }
 }
 
+// Tables computed in FP64, narrowed once.
+__global__ void narrow_table(float2* dst, const double2* src, long long cnt) {
+  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < cnt; e += (long long)gridDim.x * blockDim.x) {
+    const double2 v = src[e];
+    dst[e] = make_float2((float)v.x, (float)v.y);
+  }
+}
+
 // The two factors of the step twiddle of the compile-time engine's columns.
 template <class T>
 __global__ void gen_fx_step(typename CT<T>::type* a, typename CT<T>::type* b, long long N1, long long N2) {
@@ -819,6 +827,11 @@ static unsigned table_grid(long long n) {
 cudaError_t gen_stage_twiddles_dev(void* tw, const StageList& sl, bool dbl, cudaStream_t st) {
   if (dbl) gen_stage_twiddles<double><<<table_grid(sl.n), 256, 0, st>>>(static_cast<double2*>(tw), sl);
   else gen_stage_twiddles<float><<<table_grid(sl.n), 256, 0, st>>>(static_cast<float2*>(tw), sl);
+  count_launch(1);
+  return cudaGetLastError();
+}
+cudaError_t narrow_table_dev(void* dst, const void* src, long long cnt, cudaStream_t st) {
+  narrow_table<<<table_grid(cnt), 256, 0, st>>>(static_cast<float2*>(dst), static_cast<const double2*>(src), cnt);
   count_launch(1);
   return cudaGetLastError();
 }

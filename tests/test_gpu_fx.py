@@ -150,3 +150,20 @@ def test_uneven_batches(afc, cuda, precision, lengths):
     z = t.clone()
     plan.execute(z, out=z, mode=2)
     assert torch.equal(z, plan.execute(t, mode=2))
+
+
+@pytest.mark.parametrize("n", [74, 1031, 8191, 65521, 100003])
+def test_chirp_transform_rounding_f32(afc, cuda, n):
+    # A level of either FFT rounds an add and a twiddle product, 0.5 u rms each,
+    # independent: 0.71 u.  2 log2 M levels, and the chirp before and after, the
+    # spectrum product and the narrowed spectrum as four more.  A kernel spectrum
+    # computed in FP32 would add log2 M levels of its own.
+    m = 1 << (2 * n - 2).bit_length()
+    bound = 0.71 * 2.0**-24 * np.sqrt(2 * np.log2(m) + 4)
+    rng = np.random.default_rng(n)
+    x = (rng.uniform(-1, 1, (4, n)) + 1j * rng.uniform(-1, 1, (4, n))).astype(np.complex64)
+    plan = afc.CudaPlan([n], precision="f32", batch=4)
+    import torch
+    y = plan.execute(torch.from_numpy(x).to(cuda)).cpu().numpy()
+    ref = np.fft.fft(x.astype(np.complex128))
+    assert np.linalg.norm(y - ref) <= bound * np.linalg.norm(ref)
