@@ -52,6 +52,7 @@ static afc_status cuda_fail(cudaError_t e, const char* what) {
 
 // Test hook: fail the next N device allocations with AFC_ERR_OUT_OF_MEMORY.
 static std::atomic<int> g_fail_allocs{0};
+static bool nu_pool_give_back();
 static cudaError_t dev_alloc(void** p, size_t bytes) {
   if (g_fail_allocs.load() > 0) {
     g_fail_allocs.fetch_sub(1);
@@ -59,7 +60,12 @@ static cudaError_t dev_alloc(void** p, size_t bytes) {
     return cudaErrorMemoryAllocation;
   }
   if (bytes == 0) bytes = 16;
-  return cudaMalloc(p, bytes);
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e == cudaErrorMemoryAllocation && nu_pool_give_back()) {
+    cudaGetLastError();
+    e = cudaMalloc(p, bytes);
+  }
+  return e;
 }
 
 // ───────────────────────────── integer layer ─────────────────────────────
@@ -1356,8 +1362,7 @@ struct afc_nufft_plan_s {
   afc_plan fft = nullptr;          // C2C f64 plan of length m
   double* deconv = nullptr;        // 1 / kb_ft(k_signed / m), k < n
   void* grid = nullptr;            // plan-owned oversampled grid (m complex128)
-  afc::NuTileLaunch tiles;         // sorted spreading: bins, and bin / rank / index per point
-  int64_t pts_cap = 0;             // points the latter hold
+  cudaMemPool_t pool = nullptr;    // where sorted spreads take their index buffers from
   std::mutex mu;                   // one caller enqueues on the grid at a time
   afc::Fence fence;                // the grid's last use on the GPU
   ~afc_nufft_plan_s();
@@ -2307,13 +2312,69 @@ static afc_status no_alloc_scratch(int dev, void** ptr) {
   return AFC_OK;
 }
 
+// Memory pools of the sorted 1D spreads, one per device that had 1D plans.  A
+// call takes its index buffers in stream order and gives them back the same way,
+// so no block is moved under a stream or a captured graph.  A pool keeps up to
+// 1 GiB while the device has 1D plans and 64 MiB after the last one, so that the
+// first call of a new plan does not pay for fresh memory again (12 MB for 2^20
+// points: about 1 ms); an allocation that finds no memory takes back the rest.
+constexpr unsigned long long kNuPoolBusy = 1ull << 30, kNuPoolIdle = 64ull << 20;
+struct NuPools {
+  std::mutex mu;
+  std::map<int, std::pair<cudaMemPool_t, int>> of;  // device: pool, plans
+};
+static NuPools& nu_pools() {
+  static NuPools* p = new NuPools();  // plans may outlive static destruction
+  return *p;
+}
+// null when the driver has none to give; spreads then stay unsorted
+static cudaMemPool_t nu_pool_take(int device) {
+  NuPools& P = nu_pools();
+  std::lock_guard<std::mutex> lk(P.mu);
+  auto& e = P.of[device];
+  if (!e.first) {
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    if (cudaMemPoolCreate(&e.first, &props) != cudaSuccess) {
+      cudaGetLastError();
+      e.first = nullptr;
+      return nullptr;
+    }
+  }
+  if (e.second++ == 0) {
+    unsigned long long keep = kNuPoolBusy;
+    cudaMemPoolSetAttribute(e.first, cudaMemPoolAttrReleaseThreshold, &keep);
+  }
+  return e.first;
+}
+static void nu_pool_release(int device) {
+  NuPools& P = nu_pools();
+  std::lock_guard<std::mutex> lk(P.mu);
+  auto& e = P.of[device];
+  if (--e.second == 0) {
+    unsigned long long keep = kNuPoolIdle;
+    cudaMemPoolSetAttribute(e.first, cudaMemPoolAttrReleaseThreshold, &keep);
+    cudaMemPoolTrimTo(e.first, kNuPoolIdle);
+  }
+}
+// whether there was a pool to give unused memory back
+static bool nu_pool_give_back() {
+  NuPools& P = nu_pools();
+  std::lock_guard<std::mutex> lk(P.mu);
+  bool any = false;
+  for (auto& e : P.of)
+    if (e.second.first) any = cudaMemPoolTrimTo(e.second.first, 0) == cudaSuccess || any;
+  return any;
+}
+
 }  // namespace afc
 
 using namespace afc;
 
 afc_nufft_plan_s::~afc_nufft_plan_s() {
-  for (int* b : {tiles.cnt, tiles.tile})
-    if (b) cudaFree(b);
+  if (pool) nu_pool_release(device);
   if (fft) afc_plan_destroy(fft);
   if (deconv) cudaFree(deconv);
   if (grid) cudaFree(grid);
@@ -2904,6 +2965,7 @@ afc_status afc_nufft1d_plan_create(afc_nufft_plan* out, int64_t n, double dx, in
   AFC_CUDA(dev_alloc((void**)&p->deconv, (size_t)n * sizeof(double)), "NUFFT deconvolution");
   AFC_CUDA(cudaMemcpy(p->deconv, dec.data(), (size_t)n * sizeof(double), cudaMemcpyHostToDevice), "NUFFT deconvolution");
   AFC_CUDA(dev_alloc(&p->grid, (size_t)p->m * 16), "NUFFT grid");
+  p->pool = nu_pool_take(device);
   *out = p.release();
   return AFC_OK;
 }
@@ -2919,25 +2981,33 @@ static NuLaunch nu_launch(const afc_nufft_plan_s& p) {
   return L;
 }
 
-// Buffers of a sorted spread (synchronous allocation when a call brings more
-// points than any before it).
-static afc_status nu1_reserve(afc_nufft_plan_s& p, int64_t npts) {
-  if (!nufft_sorted(nu_launch(p), npts)) return AFC_OK;
-  if (!p.tiles.cnt) {
+// Spread, sorted first where that pays.  A captured call spreads unsorted: its
+// graph then holds no allocation and no buffer of the pool.  So does a call the
+// pool has no memory for.
+static cudaError_t nu1_spread_all(afc_nufft_plan_s& p, const double* positions, const void* values, int64_t npts,
+                                  bool cap, cudaStream_t st) {
+  const NuLaunch L = nu_launch(p);
+  NuTileLaunch T;
+  if (!cap && p.pool && nufft_sorted(L, npts)) {
     const int w = nufft_bin_width(p.m);
     const size_t bins = (size_t)((p.m + w - 1) / w);
-    AFC_CUDA(dev_alloc((void**)&p.tiles.cnt, (2 * bins + 1) * sizeof(int)), "NUFFT bins");  // cnt, then off
-    p.tiles.off = p.tiles.cnt + bins;
+    void* buf = nullptr;  // counts, offsets; bin, rank and index per point
+    if (cudaMallocFromPoolAsync(&buf, (2 * bins + 1 + 3 * (size_t)npts) * sizeof(int), p.pool, st) == cudaSuccess) {
+      T.cnt = static_cast<int*>(buf);
+      T.off = T.cnt + bins;
+      T.tile = T.off + bins + 1;
+      T.rank = T.tile + npts;
+      T.idx = T.rank + npts;
+    } else {
+      cudaGetLastError();
+    }
   }
-  if (npts <= p.pts_cap) return AFC_OK;
-  if (p.tiles.tile) cudaFree(p.tiles.tile);  // tile, rank and idx are one allocation
-  p.tiles.tile = p.tiles.rank = p.tiles.idx = nullptr;
-  p.pts_cap = 0;
-  AFC_CUDA(dev_alloc((void**)&p.tiles.tile, 3 * (size_t)npts * sizeof(int)), "NUFFT point bins");
-  p.tiles.rank = p.tiles.tile + npts;
-  p.tiles.idx = p.tiles.rank + npts;
-  p.pts_cap = npts;
-  return AFC_OK;
+  cudaError_t e = nufft_spread_dev(L, T, positions, values, npts, p.grid, st);
+  if (T.cnt) {
+    const cudaError_t f = cudaFreeAsync(T.cnt, st);
+    if (e == cudaSuccess) e = f;
+  }
+  return e;
 }
 
 afc_status afc_nufft1d_type1(afc_nufft_plan plan, const double* positions, const void* values, int64_t npts, void* out,
@@ -2952,9 +3022,7 @@ afc_status afc_nufft1d_type1(afc_nufft_plan plan, const double* positions, const
   const bool cap = stream_capturing(st);
   AFC_CUDA(plan->fence.before(st, cap), "NUFFT ordering");
   AFC_CUDA(cudaMemsetAsync(plan->grid, 0, (size_t)plan->m * 16, st), "NUFFT grid");
-  afc_status r = nu1_reserve(*plan, npts);
-  if (r != AFC_OK) return r;
-  AFC_CUDA(nufft_spread_dev(nu_launch(*plan), plan->tiles, positions, values, npts, plan->grid, st), "NUFFT spread");
+  AFC_CUDA(nu1_spread_all(*plan, positions, values, npts, cap, st), "NUFFT spread");
   afc_status s = afc_execute(plan->fft, plan->grid, plan->grid, AFC_FORWARD, stream);
   if (s != AFC_OK) return s;
   AFC_CUDA(nufft_deconv_out_dev(plan->grid, plan->deconv, plan->n, plan->m, out, st), "NUFFT deconvolution");

@@ -213,8 +213,8 @@ struct NuLaunch {
   NuPoly f;
 };
 struct NuTileLaunch;
-// Whether a spread of npts points sorts them first (the plan then holds bins of
-// nufft_bin_width cells, at most 16384, and a bin, rank and index per point).
+// Whether a spread of npts points sorts them first, given buffers for bins of
+// nufft_bin_width cells (at most 16384) and a bin, rank and index per point.
 bool nufft_sorted(const NuLaunch& L, long long npts);
 inline int nufft_bin_width(long long m) { return (int)std::max<long long>(8, (m + 16383) / 16384); }
 cudaError_t nufft_spread_dev(const NuLaunch& L, const NuTileLaunch& TL, const double* pos, const void* val,

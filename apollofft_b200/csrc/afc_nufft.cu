@@ -1,15 +1,16 @@
 // afc_nufft.cu -- Kaiser-Bessel spreading / interpolation for the 1D NUFFT
-// (apollo-nufft NufftPlan1D, transform/dimension_1d.rs:156-272).
+// (apollo-nufft NufftPlan1D, transform/dimension_1d.rs:156-272), and below for
+// the 3D one.
 //
 // Type 1: every non-uniform point adds value * phi(p - d) to the 2w+1
-// oversampled grid cells around round(m x / L) (atomic adds: points are not
-// sorted), the grid goes through this library's forward FFT, and the n output
+// oversampled grid cells around round(m x / L) (atomic adds, after sorting where
+// that pays), the grid goes through this library's forward FFT, and the n output
 // bins are the grid bins k_signed mod m times the deconvolution factors.
 // Type 2: the n coefficients times the deconvolution factors are placed at
 // k_signed mod m, the grid goes through the unnormalized inverse FFT, and every
 // point gathers its 2w+1 cells weighted by phi.  phi is the reference's kernel
 // phi(x) = I0(beta sqrt(1 - (x/w)^2)) / I0(beta), |x| < w, with I0 by its power
-// series (kaiser_bessel.rs:55-116), evaluated in FP64 per tap.
+// series (kaiser_bessel.rs:55-116), evaluated in FP64 per tap as one polynomial.
 #include <cuda_runtime.h>
 #include "afc_internal.h"
 

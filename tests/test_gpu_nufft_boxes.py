@@ -59,3 +59,32 @@ def test_1d_widths(afc, oracle, cuda, n, w, npts):
     y2 = plan.type2(torch.from_numpy(coef).cuda(), p_t).cpu().numpy()
     assert rel_l2(y1, ref.type1(pos, val, oracle)) < 1e-12
     assert rel_l2(y2, ref.type2(coef, pos, oracle)) < 1e-12
+
+
+def test_1d_first_call_captured(afc, cuda):
+    # Points enough for a sorted spread, on a plan that has never run: the
+    # capture may not allocate, the graph may hold no buffer that a later, larger
+    # call moves, and both ways of spreading agree to the rounding of sums of
+    # npts (2w + 1) / m products a cell.
+    from apollofft_b200.nufft import NufftPlan1D
+    n, w, npts = 1024, 6, 200_000  # a one-pass grid transform: it needs no workspace
+    g = torch.Generator(device="cuda")
+    g.manual_seed(5)
+    pos = torch.rand(npts, dtype=torch.float64, device="cuda", generator=g) * n
+    val = torch.randn(npts, dtype=torch.complex128, device="cuda", generator=g)
+    big = torch.rand(3 * npts, dtype=torch.float64, device="cuda", generator=g) * n
+    bigv = torch.randn(3 * npts, dtype=torch.complex128, device="cuda", generator=g)
+    plan, other = NufftPlan1D(n, 1.0, 2, w), NufftPlan1D(n, 1.0, 2, w)
+    other.type1(pos, val)  # kernels are loaded outside a capture
+    out = torch.zeros(n, dtype=torch.complex128, device="cuda")
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        plan.type1(pos, val, out=out)
+    plan.type1(big, bigv)
+    del other
+    for _ in range(2):
+        out.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert rel_l2(out.cpu().numpy(), plan.type1(pos, val).cpu().numpy()) < 1e-13
