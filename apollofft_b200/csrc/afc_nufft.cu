@@ -64,7 +64,7 @@ __device__ __forceinline__ double nu_kb(double x, double w, double beta, double 
 __device__ __forceinline__ double nu_phi(const NuPoly& f, double x, double w, double beta, double i0b) {
   if (f.K == 0) return nu_kb(x, w, beta, i0b);
   const double s = (w - x) * (w + x);
-  if (!(s > 0.0)) return 0.0;
+  if (s <= 0.0) return 0.0;  // a NaN position gives NaN weights
   double a = f.c[f.K - 1];
 #pragma unroll 5
   for (int k = f.K - 2; k >= 0; --k) a = fma(a, s, f.c[k]);
@@ -93,7 +93,7 @@ __device__ __forceinline__ void nu_phi4(const NuPoly& f, int p0, double d, int w
     for (int i = 0; i < 4; ++i) a[i] = fma(a[i], s[i], c);
   }
 #pragma unroll
-  for (int i = 0; i < 4; ++i) o[i] = s[i] > 0.0 ? a[i] : 0.0;
+  for (int i = 0; i < 4; ++i) o[i] = s[i] <= 0.0 ? 0.0 : a[i];
 }
 
 // All T taps of one axis in one walk over the coefficients (T independent chains:
@@ -122,7 +122,7 @@ __device__ __forceinline__ void nu_phi_all(const NuPoly& f, double d, double bet
     for (int i = 0; i < T; ++i) o[i] = fma(o[i], s[i], c);
   }
 #pragma unroll
-  for (int i = 0; i < T; ++i) o[i] = s[i] > 0.0 ? o[i] : 0.0;
+  for (int i = 0; i < T; ++i) o[i] = s[i] <= 0.0 ? 0.0 : o[i];
 }
 
 struct NuGeom {

@@ -88,3 +88,46 @@ def test_1d_first_call_captured(afc, cuda):
         graph.replay()
         torch.cuda.synchronize()
         assert rel_l2(out.cpu().numpy(), plan.type1(pos, val).cpu().numpy()) < 1e-13
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("n,w,npts", [(64, 6, 500), (32, 6, 5000), (32, 5, 5000), (40, 13, 500)])
+def test_1d_position_not_finite(afc, cuda, bad, n, w, npts):
+    # Its weights are not numbers: no type-1 bin is one then, and of the type-2
+    # values only its own is not.  Direct and sorted spreads, wide kernels.
+    from apollofft_b200.nufft import NufftPlan1D
+    rng = np.random.default_rng(n + w)
+    pos = rng.uniform(0, n, npts)
+    val, coef = (rng.standard_normal(k) + 1j * rng.standard_normal(k) for k in (npts, n))
+    plan = NufftPlan1D(n, 1.0, 2, w)
+    c_t, v_t = torch.from_numpy(coef).cuda(), torch.from_numpy(val).cuda()
+    good = plan.type2(c_t, torch.from_numpy(pos).cuda()).cpu().numpy()
+    pos[npts // 3] = bad
+    p_t = torch.from_numpy(pos).cuda()
+    assert np.isnan(plan.type1(p_t, v_t).cpu().numpy()).all()
+    y2 = plan.type2(c_t, p_t).cpu().numpy()
+    assert np.isnan(y2[npts // 3])
+    keep = np.arange(npts) != npts // 3
+    assert np.array_equal(y2[keep], good[keep])
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("shape,w", [((16, 16, 16), 6), ((8, 16, 4), 6), ((4, 4, 4), 10)])
+def test_3d_position_not_finite(afc, cuda, bad, shape, w):
+    # box, tile and per-point kernels
+    from apollofft_b200.nufft import NufftPlan3D
+    rng = np.random.default_rng(w)
+    npts = 300
+    pos = rng.uniform(0, 1, (npts, 3)) * np.array(shape)
+    val = rng.standard_normal(npts) + 1j * rng.standard_normal(npts)
+    modes = rng.standard_normal(shape) + 1j * rng.standard_normal(shape)
+    plan = NufftPlan3D(shape, (1.0, 1.0, 1.0), 2, w)
+    m_t, v_t = torch.from_numpy(modes).cuda(), torch.from_numpy(val).cuda()
+    good = plan.type2(m_t, torch.from_numpy(pos).cuda()).cpu().numpy()
+    pos[100, 1] = bad
+    p_t = torch.from_numpy(pos).cuda()
+    assert np.isnan(plan.type1(p_t, v_t).cpu().numpy()).all()
+    y2 = plan.type2(m_t, p_t).cpu().numpy()
+    assert np.isnan(y2[100])
+    keep = np.arange(npts) != 100
+    assert rel_l2(y2[keep], good[keep]) < 1e-13
