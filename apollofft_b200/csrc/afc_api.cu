@@ -1094,10 +1094,21 @@ static int64_t conv_length(int64_t need, size_t csz, bool bluestein) {
   return best;
 }
 
+// Raises the shared-memory budget to a whole CTA's while it lives.
+struct FullSmemCap {
+  size_t old = tl_smem_cap;
+  FullSmemCap() { tl_smem_cap = kSmemMax; }
+  ~FullSmemCap() { tl_smem_cap = old; }
+};
+
 // Spectra of a complex64 Bluestein kernel, both directions: chirp, kernel and
 // FFT in FP64, narrowed once (computed in FP32 the spectrum's own rounding was
-// about a fifth of the transform's error).
+// about a fifth of the transform's error).  M was chosen for complex64 tiles,
+// which hold twice the points: the FP64 plan, used here only, has the whole
+// CTA's shared memory also while a batch plan is built, and where it still has
+// no split (2^25, say) or no memory the caller computes the spectra in FP32.
 static afc_status narrow_spectra(int64_t n, int64_t M, void* spec, cudaStream_t st) {
+  const FullSmemCap cap;
   std::shared_ptr<AxisPlan> md;
   afc_status s = AFC_OK;
   if (tl_share && tl_share->sub64.count(M)) {
@@ -1187,12 +1198,16 @@ static afc_status build_axis(int64_t n, bool dbl, AxisPlan& ap, cudaStream_t st)
   AFC_CUDA(dev_alloc(&ap.spec_f, 2 * (size_t)M * csz), "Bluestein spectrum");
   ap.spec_i = static_cast<char*>(ap.spec_f) + (size_t)M * csz;
   afc_status s = AFC_OK;
-  if (dbl) {
-    AFC_CUDA(gen_bluestein_b_dev(ap.spec_f, ap.chirp, n, M, false, true, st), "Bluestein kernel");
-    AFC_CUDA(gen_bluestein_b_dev(ap.spec_i, ap.chirp, n, M, true, true, st), "Bluestein kernel");
-  } else {
+  bool narrowed = false;
+  if (!dbl) {
     s = narrow_spectra(n, M, ap.spec_f, st);
-    if (s != AFC_OK) return s;
+    narrowed = s == AFC_OK;
+    if (!narrowed && s != AFC_ERR_UNSUPPORTED && s != AFC_ERR_OUT_OF_MEMORY) return s;
+    if (!narrowed) cudaGetLastError();  // the allocation that failed
+  }
+  if (!narrowed) {
+    AFC_CUDA(gen_bluestein_b_dev(ap.spec_f, ap.chirp, n, M, false, dbl, st), "Bluestein kernel");
+    AFC_CUDA(gen_bluestein_b_dev(ap.spec_i, ap.chirp, n, M, true, dbl, st), "Bluestein kernel");
   }
   // one tile up to 4096 points, else (8192 complex64 would still fit the
   // general engine's tile) the three compile-time passes
@@ -1200,7 +1215,7 @@ static afc_status build_axis(int64_t n, bool dbl, AxisPlan& ap, cudaStream_t st)
     ap.conv_smem = true;
     s = build_lenplan(M, dbl, ap.lp, st);
     if (s != AFC_OK) return s;
-    if (!dbl) return AFC_OK;
+    if (narrowed) return AFC_OK;
     AxisPlan mp;
     mp.n = M;
     mp.algo = ALGO_SMEM;
@@ -1220,7 +1235,7 @@ static afc_status build_axis(int64_t n, bool dbl, AxisPlan& ap, cudaStream_t st)
     if (s != AFC_OK) return s;
     if (tl_share) tl_share->sub[M] = ap.sub;
   }
-  if (dbl) {
+  if (!narrowed) {
     s = fft_table(*ap.sub, dbl, ap.spec_f, st);
     if (s == AFC_OK) s = fft_table(*ap.sub, dbl, ap.spec_i, st);
     if (s != AFC_OK) return s;
