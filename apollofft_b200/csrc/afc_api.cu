@@ -3265,7 +3265,7 @@ afc_status afc_nufft3d_type1(afc_nufft3d_plan plan, const double* positions, con
   if (tiled && nufft3_boxes(L)) {
     r = nu3_reserve_records(*plan, npts);
     if (r != AFC_OK) return r;
-    AFC_CUDA(nufft3_boxes_dev(L, plan->tiles, true, positions, values, npts, plan->grid, nullptr, st), "NUFFT spread");
+    AFC_CUDA(nufft3_boxes_dev(L, plan->tiles, positions, values, npts, plan->grid, st), "NUFFT spread");
   } else if (tiled)
     AFC_CUDA(nufft3_tiled_dev(L, plan->tiles, true, positions, values, npts, plan->grid, st), "NUFFT spread");
   else
@@ -3299,12 +3299,7 @@ afc_status afc_nufft3d_type2(afc_nufft3d_plan plan, const void* modes, const dou
   bool tiled = false;
   s = nu3_reserve(*plan, npts, &tiled);
   if (s != AFC_OK) return s;
-  if (tiled && nufft3_boxes(L)) {
-    s = nu3_reserve_records(*plan, npts);
-    if (s != AFC_OK) return s;
-    AFC_CUDA(nufft3_boxes_dev(L, plan->tiles, false, positions, nullptr, npts, plan->grid, out, st),
-             "NUFFT interpolation");
-  } else if (tiled)
+  if (tiled)
     AFC_CUDA(nufft3_tiled_dev(L, plan->tiles, false, positions, plan->grid, npts, out, st), "NUFFT interpolation");
   else
     AFC_CUDA(nufft3_interp_dev(L, plan->grid, positions, npts, out, st), "NUFFT interpolation");

@@ -654,45 +654,44 @@ __global__ void __launch_bounds__(kNuTileThreads) nu3_spread_tiles(const __grid_
   }
 }
 
-// ─── 3D spreading and interpolation by boxes of cells ───
-// The tile kernels are bound by shared memory (a 16-byte cell per tap, read and
-// for spreading written back) and spreading adds every tile's halo to the grid
-// with atomics, 15 times the cells at w = 6.  Here the cells stay in registers
-// and the points move: a warp owns a box of 8 x 4 x 8 cells and meets every
-// point whose taps reach it (25 boxes per point at w = 6).  Per box the sums are
-// small FP64 matrix products (mma m8n8k4):
-//   spreading      C[x][z] += wx[point][x] (v wy wz)[point][z], 4 points at a
-//                  time, for each y and for both parts of v;
-//   interpolation  D[point][z] = sum_x wx[point][x] cell[x][z], 8 points at a
-//                  time, then summed over y and z with their weights.
-// One operand element per lane feeds 8 FMAs.  Measured at 2^18 points on 128^3
-// cells, w = 6 (kernel alone): tiles 1650 us spreading, 784 us interpolating; boxes
-// with scalar FMAs, bound by the broadcast weight loads, 1095 us spreading; these
-// 600 and 690 us, bound by the latency of the shared-memory loads behind each
-// group (the FP64 matrix pipe is a third busy).
-//  nu3_points: one record per point in tile order: value, centre, index, and the
-//              axis weights between runs of seven zeros, so no tap is range-checked;
+// ─── 3D spreading by boxes of cells ───
+// The tile kernel is bound by shared memory (a 16-byte cell per tap, read and
+// written back) and adds every tile's halo to the grid with atomics, 15 times
+// the cells at w = 6.  Here the cells stay in registers and the points move: a
+// warp owns a box of 8 x 4 x 8 cells and meets every point whose taps reach it
+// (25 boxes per point at w = 6).  Per box the sums are small FP64 matrix products
+// (mma m8n8k4), C[x][z] += wx[point][x] (v wy wz)[point][z], 4 points at a time,
+// for each y and for both parts of v.  One operand element per lane feeds 8 FMAs.
+// Measured at 2^18 points on 128^3 cells, w = 6 (kernel alone): tiles 1650 us;
+// boxes with scalar FMAs, bound by the broadcast weight loads, 1095 us; these 612
+// us, bound by the shared-memory loads and chunk barriers ahead of each group
+// (FP64 pipe 6-8 % busy).
+// Interpolation keeps the tile kernel: a point's boxes would have to add their
+// parts to its value in whatever order they finish, and 711 us of box kernel and
+// 54 us of records are no gain on its 784 us that would be worth values that
+// change in the last bit from call to call.
+//  nu3_points: one record per point in tile order: value, centre, and the axis
+//              weights between runs of seven zeros, so no tap is range-checked;
 //  nu3_boxes:  a CTA of 8 warps owns 16 x 8 x 16 cells and streams the records of
 //              the tiles within w cells of it through shared memory, the next chunk
 //              in flight while one is worked on.  Each warp lists the records that
 //              meet its box and takes them in groups.
-// Boxes partition the grid: spreading writes each cell once, without atomics
-// unless a box's points are split over CTAs; interpolation adds a partial sum
-// per point and box to the outputs.
+// Boxes partition the grid: each cell is written once, without atomics unless a
+// box's points are split over CTAs.
 constexpr int kNuBoxThreads = 256;
-// chunk and CTAs per SM measured at 2^18 points on 128^3 cells, w = 6 (spreading /
-// interpolation): 32 points, three CTAs 798 / 900 us for the whole call, 64 points,
-// two CTAs 845 / 927, 32 points, two CTAs 917 / 1027
+// chunk and CTAs per SM measured at 2^18 points on 128^3 cells, w = 6: 32 points,
+// three CTAs 798 us for the whole call, 64 points, two CTAs 845, 32 points, two
+// CTAs 917
 constexpr int kNuBoxChunk = 32;
 constexpr int kNuBoxRuns = 64;  // contiguous runs of candidate points per CTA
 
-// Record: v.x, v.y, centre cells and index (four ints), then x, y and z weights.
+// Record: v.x, v.y, centre cells (three of four ints), then x, y and z weights.
 __host__ __device__ constexpr int nu_xo(int) { return 11; }
 __host__ __device__ constexpr int nu_yo(int T) { return 18 + T; }
 __host__ __device__ constexpr int nu_zo(int T) { return 25 + 2 * T; }
 __host__ __device__ constexpr int nu_rec(int T) { return (32 + 3 * T + 1) / 2 * 2; }
 constexpr int kNuZeros = 16;  // a block of zeros: the record of the slots that fill up a group
-__host__ __device__ constexpr int nu_list() { return (kNuBoxChunk + 16) * 4; }  // ints per warp
+__host__ __device__ constexpr int nu_list() { return (kNuBoxChunk + 8) * 4; }  // ints per warp
 
 __device__ __forceinline__ void nu_cp16(void* smem, const void* gmem) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem)
@@ -702,7 +701,7 @@ __device__ __forceinline__ void nu_cp16(void* smem, const void* gmem) {
 // Block of kNuPts points, three threads each (one per axis): the records are put
 // together in shared memory and stored whole (rows written straight to global
 // memory were 13 eight-byte stores per thread to 32 places each: 97 us at 2^18
-// points).  val null (interpolation): no value in the record.
+// points).
 constexpr int kNuPts = 64;
 template <int T>
 __global__ void __launch_bounds__(3 * kNuPts) nu3_points(const __grid_constant__ NuGeom3 g, const int* __restrict__ idx,
@@ -730,10 +729,9 @@ __global__ void __launch_bounds__(3 * kNuPts) nu3_points(const __grid_constant__
       int* c = reinterpret_cast<int*>(r + 2);
       c[a] = (int)((long long)rt & (m - 1));
       if (a == 0) {
-        const double2 v = val ? val[j] : make_double2(0.0, 0.0);
+        const double2 v = val[j];
         r[0] = v.x;
         r[1] = v.y;
-        c[3] = j;
       }
     }
     __syncthreads();
@@ -751,12 +749,10 @@ __device__ __forceinline__ void nu_mma(double2& d, double a, double b) {
                : "d"(a), "d"(b));
 }
 
-// SPREAD: records -> cells (add: the cells may be shared with other CTAs);
-// else: cells -> out (zeroed by the caller).
-template <bool SPREAD>
+// Records -> cells (add: the cells may be shared with other CTAs).
 __global__ void __launch_bounds__(kNuBoxThreads, 3)
     nu3_boxes(int mx, int my, int mz, int w, const int* __restrict__ off, const double* __restrict__ rec,
-              double2* __restrict__ grid, double2* __restrict__ out, int add) {
+              double2* __restrict__ grid, int add) {
   extern __shared__ __align__(16) double nu_sm[];
   __shared__ int run_start[kNuBoxRuns], run_pre[kNuBoxRuns + 1];
   const int T = 2 * w + 1, S = nu_rec(T);
@@ -779,7 +775,7 @@ __global__ void __launch_bounds__(kNuBoxThreads, 3)
   }
   const int ZB = 2 * kNuBoxChunk * S;  // the zero block
   if (tid < kNuZeros) nu_sm[ZB + tid] = 0.0;
-  int4* const list = reinterpret_cast<int4*>(nu_sm + ZB + kNuZeros) + wid * (kNuBoxChunk + 16);
+  int4* const list = reinterpret_cast<int4*>(nu_sm + ZB + kNuZeros) + wid * (kNuBoxChunk + 8);
   __syncthreads();
   if (tid == 0) {
     run_pre[0] = 0;
@@ -814,22 +810,10 @@ __global__ void __launch_bounds__(kNuBoxThreads, 3)
   const int x0 = gx0 + (wid >> 2) * 8, y0 = gy0 + ((wid >> 1) & 1) * 4, z0 = gz0 + (wid & 1) * 8;
   const int lr = lane >> 2, lk = lane & 3;
   stage(c, 0);
-  double2 acc[4][2];     // SPREAD: C[x = lr][z = 2 lk, 2 lk + 1] of row y, real and imaginary
-  double cell[4][2][2];  // else: B[x = lk + 4 s][z = lr] of row y, real and imaginary
+  double2 acc[4][2];  // C[x = lr][z = 2 lk, 2 lk + 1] of row y, real and imaginary
   const long long sx = (long long)my * mz;
-  if constexpr (SPREAD) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[j][0] = acc[j][1] = make_double2(0.0, 0.0);
-  } else {
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-#pragma unroll
-      for (int s = 0; s < 2; ++s) {
-        const double2 v = grid[(x0 + 4 * s + lk) * sx + (long long)(y0 + j) * mz + z0 + lr];
-        cell[j][s][0] = v.x;
-        cell[j][s][1] = v.y;
-      }
-  }
+  for (int j = 0; j < 4; ++j) acc[j][0] = acc[j][1] = make_double2(0.0, 0.0);
   bool any = false;
   for (int k = 0; c < nchunk; ++k, c += gridDim.y) {
     const int slot = k & 1;
@@ -853,7 +837,7 @@ __global__ void __launch_bounds__(kNuBoxThreads, 3)
         const int dx = (x0 - cc.x + w) & (mx - 1), dy = (y0 - cc.y + w) & (my - 1), dz = (z0 - cc.z + w) & (mz - 1);
         hit = (dx < T || dx > mx - 8) && (dy < T || dy > my - 4) && (dz < T || dz > mz - 8);
         e = make_int4(rp + nu_xo(T) + (dx < T ? dx : dx - mx), rp + nu_yo(T) + (dy < T ? dy : dy - my),
-                      rp + nu_zo(T) + (dz < T ? dz : dz - mz), SPREAD ? rp : cc.w);
+                      rp + nu_zo(T) + (dz < T ? dz : dz - mz), rp);
       }
       const unsigned mask = __ballot_sync(0xffffffffu, hit);
       if (hit) list[n + __popc(mask & ((1u << lane) - 1))] = e;
@@ -861,64 +845,38 @@ __global__ void __launch_bounds__(kNuBoxThreads, 3)
     }
     any = any || n;
     // fills up the last group, and one group past it for the loop's look-ahead
-    if (lane < 16) list[n + lane] = make_int4(ZB, ZB, ZB, SPREAD ? ZB : -1);
+    if (lane < 8) list[n + lane] = make_int4(ZB, ZB, ZB, ZB);
     __syncwarp();
-    constexpr int G = SPREAD ? 4 : 8;
-    int4 e = list[SPREAD ? lk : lr];
+    int4 e = list[lk];
 #pragma unroll 2
-    for (int i = 0; i < n; i += G) {
-      const int4 e_next = list[i + G + (SPREAD ? lk : lr)];
-      if constexpr (SPREAD) {
-        const double2 v = *reinterpret_cast<const double2*>(nu_sm + e.w);
-        const double wz = nu_sm[e.z + lr], ax = nu_sm[e.x + lr];
-        const double vr = v.x * wz, vi = v.y * wz;
+    for (int i = 0; i < n; i += 4) {
+      const int4 e_next = list[i + 4 + lk];
+      const double2 v = *reinterpret_cast<const double2*>(nu_sm + e.w);
+      const double wz = nu_sm[e.z + lr], ax = nu_sm[e.x + lr];
+      const double vr = v.x * wz, vi = v.y * wz;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const double wy = nu_sm[e.y + j];
-          nu_mma(acc[j][0], ax, vr * wy);
-          nu_mma(acc[j][1], ax, vi * wy);
-        }
-      } else {
-        const double a0 = nu_sm[e.x + lk], a1 = nu_sm[e.x + 4 + lk];
-        const double w0 = nu_sm[e.z + 2 * lk], w1 = nu_sm[e.z + 2 * lk + 1];
-        double re = 0.0, im = 0.0;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          double2 dr = make_double2(0.0, 0.0), di = dr;
-          nu_mma(dr, a0, cell[j][0][0]);
-          nu_mma(di, a0, cell[j][0][1]);
-          nu_mma(dr, a1, cell[j][1][0]);
-          nu_mma(di, a1, cell[j][1][1]);
-          const double wy = nu_sm[e.y + j];
-          re = fma(wy, fma(w1, dr.y, w0 * dr.x), re);
-          im = fma(wy, fma(w1, di.y, w0 * di.x), im);
-        }
-#pragma unroll
-        for (int o = 1; o < 4; o <<= 1) {
-          re += __shfl_xor_sync(0xffffffffu, re, o);
-          im += __shfl_xor_sync(0xffffffffu, im, o);
-        }
-        if (lk < 2 && e.w >= 0) atomicAdd(lk ? &out[e.w].y : &out[e.w].x, lk ? im : re);
+      for (int j = 0; j < 4; ++j) {
+        const double wy = nu_sm[e.y + j];
+        nu_mma(acc[j][0], ax, vr * wy);
+        nu_mma(acc[j][1], ax, vi * wy);
       }
       e = e_next;
     }
     __syncthreads();  // the slot is refilled
   }
-  if constexpr (SPREAD) {
-    if (!any) return;
+  if (!any) return;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      double2* o = grid + (x0 + lr) * sx + (long long)(y0 + j) * mz + z0 + 2 * lk;
-      const double2 c0 = make_double2(acc[j][0].x, acc[j][1].x), c1 = make_double2(acc[j][0].y, acc[j][1].y);
-      if (add) {
-        atomicAdd(&o[0].x, c0.x);
-        atomicAdd(&o[0].y, c0.y);
-        atomicAdd(&o[1].x, c1.x);
-        atomicAdd(&o[1].y, c1.y);
-      } else {
-        o[0] = c0;
-        o[1] = c1;
-      }
+  for (int j = 0; j < 4; ++j) {
+    double2* o = grid + (x0 + lr) * sx + (long long)(y0 + j) * mz + z0 + 2 * lk;
+    const double2 c0 = make_double2(acc[j][0].x, acc[j][1].x), c1 = make_double2(acc[j][0].y, acc[j][1].y);
+    if (add) {
+      atomicAdd(&o[0].x, c0.x);
+      atomicAdd(&o[0].y, c0.y);
+      atomicAdd(&o[1].x, c1.x);
+      atomicAdd(&o[1].y, c1.y);
+    } else {
+      o[0] = c0;
+      o[1] = c1;
     }
   }
 }
@@ -1173,20 +1131,15 @@ size_t nufft3_box_smem(int w) {
 }
 size_t nufft3_rec_bytes(int w) { return (size_t)nu_rec(2 * w + 1) * sizeof(double); }
 
-// Spreads npts points onto the zeroed grid, or interpolates the grid at them
-// into out; kNu3Slice points at a time (their records take nufft3_rec_bytes each).
-cudaError_t nufft3_boxes_dev(const NuLaunch3& L, const NuTileLaunch& TL, bool spread, const double* pos,
-                             const void* val, long long npts, void* grid, void* out, cudaStream_t st) {
+// Spreads npts points onto the zeroed grid, kNu3Slice points at a time (their
+// records take nufft3_rec_bytes each).
+cudaError_t nufft3_boxes_dev(const NuLaunch3& L, const NuTileLaunch& TL, const double* pos, const void* val,
+                             long long npts, void* grid, cudaStream_t st) {
   const NuGeom3 g = geom3(L);
   const int nty = (int)(L.my / 8), ntz = (int)(L.mz / 8), ntiles = (int)(L.mx / 8) * nty * ntz;
   const size_t smem = nufft3_box_smem(L.w);
-  auto k = spread ? nu3_boxes<true> : nu3_boxes<false>;
-  cudaError_t e = kernel_smem_grant(reinterpret_cast<const void*>(k), smem);
+  cudaError_t e = kernel_smem_grant(reinterpret_cast<const void*>(nu3_boxes), smem);
   if (e != cudaSuccess) return e;
-  if (!spread && npts > 0) {
-    e = cudaMemsetAsync(out, 0, (size_t)npts * 16, st);
-    if (e != cudaSuccess) return e;
-  }
   const int boxes = (int)(L.mx / 16) * (int)(L.my / 8) * (int)(L.mz / 16);
   for (long long p0 = 0; p0 < npts; p0 += kNu3Slice) {
     const long long n = std::min<long long>(kNu3Slice, npts - p0);
@@ -1209,14 +1162,14 @@ cudaError_t nufft3_boxes_dev(const NuLaunch3& L, const NuTileLaunch& TL, bool sp
       default: return cudaErrorInvalidValue;
     }
     points<<<(unsigned)((n + kNuPts - 1) / kNuPts), 3 * kNuPts, 0, st>>>(
-        g, TL.idx, ps, spread ? static_cast<const double2*>(val) + p0 : nullptr, (int)n, TL.rec);
+        g, TL.idx, ps, static_cast<const double2*>(val) + p0, (int)n, TL.rec);
     // a box's chunks are dealt to `split` CTAs: about 4096 CTAs in all, so a
     // grid of few boxes, or points crowded into some of them, still fills the chip
     const long long chunks = (n + kNuBoxChunk - 1) / kNuBoxChunk;
     const int split = (int)std::max<long long>(1, std::min<long long>(chunks, std::min(32, 4096 / boxes)));
-    k<<<dim3((unsigned)boxes, (unsigned)split), kNuBoxThreads, smem, st>>>(
+    nu3_boxes<<<dim3((unsigned)boxes, (unsigned)split), kNuBoxThreads, smem, st>>>(
         (int)L.mx, (int)L.my, (int)L.mz, L.w, TL.off, TL.rec, static_cast<double2*>(grid),
-        spread ? nullptr : static_cast<double2*>(out) + p0, split > 1 || npts > kNu3Slice);
+        split > 1 || npts > kNu3Slice);
     count_launch(5);
   }
   return cudaGetLastError();

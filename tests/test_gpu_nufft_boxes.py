@@ -2,7 +2,7 @@
 rows, its candidate runs and the polynomial kernel can go wrong: every kernel
 width, grids one box wide and up, crowded points (a box's points split over
 CTAs), points on cell boundaries, against the reference algorithm restated in
-numpy."""
+numpy; interpolation repeats bit for bit."""
 import numpy as np
 import pytest
 import torch
@@ -131,3 +131,21 @@ def test_3d_position_not_finite(afc, cuda, bad, shape, w):
     assert np.isnan(y2[100])
     keep = np.arange(npts) != 100
     assert rel_l2(y2[keep], good[keep]) < 1e-13
+
+
+@pytest.mark.parametrize("shape,w,npts", [((16, 16, 16), 6, 20000), ((20, 16, 12), 9, 3000), ((8, 8, 8), 6, 3000),
+                                          ((4, 4, 4), 10, 500)])
+def test_3d_interpolation_repeats(afc, cuda, shape, w, npts):
+    # each value is summed by one warp in one order, whatever the order the points
+    # were sorted in
+    from apollofft_b200.nufft import NufftPlan3D
+    g = torch.Generator(device="cuda").manual_seed(npts)
+    pos = torch.rand(npts, 3, dtype=torch.float64, device="cuda", generator=g)
+    pos = (pos * torch.tensor(shape, dtype=torch.float64, device="cuda")).contiguous()
+    modes = torch.randn(shape, dtype=torch.complex128, device="cuda", generator=g)
+    plan = NufftPlan3D(shape, (1.0, 1.0, 1.0), 2, w)
+    first = plan.type2(modes, pos)
+    for _ in range(5):
+        assert torch.equal(torch.view_as_real(plan.type2(modes, pos)), torch.view_as_real(first))
+    swap = torch.randperm(npts, device="cuda", generator=g)
+    assert torch.equal(torch.view_as_real(plan.type2(modes, pos[swap].contiguous())), torch.view_as_real(first[swap]))
