@@ -1386,6 +1386,13 @@ struct afc_nufft_plan_s {
 // 3D NUFFT plan (apollo-nufft NufftPlan3D, transform/dimension_3d.rs:193-230):
 // per axis m = next_pow2(max(sigma n, 2w + 1)), one C2C f64 plan of
 // (mx, my, mz) over the plan-owned grid, deconvolution factors per axis.
+// A buffer of a 3D NUFFT plan with so much per point.
+struct NuPointBuf {
+  void* p = nullptr;
+  int64_t cap = 0;        // points it holds
+  bool captured = false;  // a captured graph has its address
+};
+
 struct afc_nufft3d_plan_s {
   int64_t n[3] = {0, 0, 0}, m[3] = {0, 0, 0};
   double d[3] = {0, 0, 0};
@@ -1397,8 +1404,8 @@ struct afc_nufft3d_plan_s {
   double* deconv = nullptr;  // nx + ny + nz factors, axis after axis
   void* grid = nullptr;      // mx my mz complex128, C order
   afc::NuTileLaunch tiles;   // B = 0: per-point kernels
-  int64_t pts_cap = 0;       // points the tile / rank / index buffers hold
-  int64_t rec_cap = 0;       // points the record buffer holds
+  NuPointBuf buckets, records;
+  std::vector<void*> retired;  // outgrown buffers that captured graphs still use
   std::mutex mu;             // one caller enqueues on the grid at a time
   afc::Fence fence;          // the grid's (and tile buffers') last use on the GPU
   ~afc_nufft3d_plan_s();
@@ -2396,9 +2403,11 @@ afc_nufft_plan_s::~afc_nufft_plan_s() {
 }
 
 afc_nufft3d_plan_s::~afc_nufft3d_plan_s() {
-  for (int* b : {tiles.cnt, tiles.off, tiles.tile})
+  for (int* b : {tiles.cnt, tiles.off})
     if (b) cudaFree(b);
-  if (tiles.rec) cudaFree(tiles.rec);
+  for (void* b : {buckets.p, records.p})
+    if (b) cudaFree(b);
+  for (void* b : retired) cudaFree(b);
   if (fft) afc_plan_destroy(fft);
   if (deconv) cudaFree(deconv);
   if (grid) cudaFree(grid);
@@ -3201,28 +3210,39 @@ afc_status afc_nufft3d_plan_create(afc_nufft3d_plan* out, int64_t nx, int64_t ny
   return AFC_OK;
 }
 
-// Grows the per-point tile buffers (synchronous allocation) when a call brings
-// more points than any call before it; false -> the per-point kernels run.
-static afc_status nu3_reserve_records(afc_nufft3d_plan_s& p, int64_t npts) {
-  const int64_t n = std::min<int64_t>(npts, kNu3Slice);
-  if (n <= p.rec_cap) return AFC_OK;
-  if (p.tiles.rec) cudaFree(p.tiles.rec);
-  p.tiles.rec = nullptr;
-  p.rec_cap = 0;
-  AFC_CUDA(dev_alloc((void**)&p.tiles.rec, (size_t)n * nufft3_rec_bytes(p.w)), "NUFFT point records");
-  p.rec_cap = n;
+// Makes b hold npts points.  A buffer whose address a captured graph has lives
+// as long as the plan; it is outgrown by twice its size, so the buffers set aside
+// add up to less than the one in use.
+static afc_status nu3_grow(afc_nufft3d_plan_s& p, NuPointBuf& b, int64_t npts, int64_t most, size_t per_point,
+                           const char* what) {
+  if (npts <= b.cap) return AFC_OK;
+  NuPointBuf nb;
+  nb.cap = b.captured ? std::min(most, std::max(npts, 2 * b.cap)) : npts;
+  if (b.captured) p.retired.push_back(b.p);
+  else if (b.p) cudaFree(b.p);
+  b = NuPointBuf{};
+  AFC_CUDA(dev_alloc(&nb.p, (size_t)nb.cap * per_point), what);
+  b = nb;
   return AFC_OK;
 }
-static afc_status nu3_reserve(afc_nufft3d_plan_s& p, int64_t npts, bool* tiled) {
+// The per-point buffers of a call, grown (synchronous allocation) when it brings
+// more points than any call before it.  *tiled false: the per-point kernels run,
+// which need none -- a captured call cannot allocate.
+static afc_status nu3_reserve(afc_nufft3d_plan_s& p, int64_t npts, bool boxes, bool cap, bool* tiled) {
+  const int64_t slice = std::min<int64_t>(npts, kNu3Slice);
   *tiled = p.tiles.B != 0 && npts > 0 && npts <= INT32_MAX;
-  if (!*tiled || npts <= p.pts_cap) return AFC_OK;
-  if (p.tiles.tile) cudaFree(p.tiles.tile);  // tile, rank and idx are one allocation
-  p.tiles.tile = p.tiles.rank = p.tiles.idx = nullptr;
-  p.pts_cap = 0;
-  AFC_CUDA(dev_alloc((void**)&p.tiles.tile, 3 * (size_t)npts * sizeof(int)), "NUFFT point buckets");
-  p.tiles.rank = p.tiles.tile + npts;
-  p.tiles.idx = p.tiles.rank + npts;
-  p.pts_cap = npts;
+  if (cap && (npts > p.buckets.cap || (boxes && slice > p.records.cap))) *tiled = false;
+  if (!*tiled) return AFC_OK;
+  afc_status s = nu3_grow(p, p.buckets, npts, INT32_MAX, 3 * sizeof(int), "NUFFT point buckets");
+  if (s == AFC_OK && boxes)
+    s = nu3_grow(p, p.records, slice, kNu3Slice, nufft3_rec_bytes(p.w), "NUFFT point records");
+  if (s != AFC_OK) return s;
+  if (cap) p.buckets.captured = true;
+  if (cap && boxes) p.records.captured = true;
+  p.tiles.tile = static_cast<int*>(p.buckets.p);
+  p.tiles.rank = p.tiles.tile + p.buckets.cap;
+  p.tiles.idx = p.tiles.rank + p.buckets.cap;
+  p.tiles.rec = static_cast<double*>(p.records.p);
   return AFC_OK;
 }
 
@@ -3258,15 +3278,14 @@ afc_status afc_nufft3d_type1(afc_nufft3d_plan plan, const double* positions, con
   const bool cap = stream_capturing(st);
   AFC_CUDA(plan->fence.before(st, cap), "NUFFT ordering");
   const NuLaunch3 L = nu_launch3(*plan);
-  AFC_CUDA(cudaMemsetAsync(plan->grid, 0, (size_t)(L.mx * L.my * L.mz) * 16, st), "NUFFT grid");
+  const bool boxes = nufft3_boxes(L);
   bool tiled = false;
-  afc_status r = nu3_reserve(*plan, npts, &tiled);
+  afc_status r = nu3_reserve(*plan, npts, boxes, cap, &tiled);
   if (r != AFC_OK) return r;
-  if (tiled && nufft3_boxes(L)) {
-    r = nu3_reserve_records(*plan, npts);
-    if (r != AFC_OK) return r;
+  AFC_CUDA(cudaMemsetAsync(plan->grid, 0, (size_t)(L.mx * L.my * L.mz) * 16, st), "NUFFT grid");
+  if (tiled && boxes)
     AFC_CUDA(nufft3_boxes_dev(L, plan->tiles, positions, values, npts, plan->grid, st), "NUFFT spread");
-  } else if (tiled)
+  else if (tiled)
     AFC_CUDA(nufft3_tiled_dev(L, plan->tiles, true, positions, values, npts, plan->grid, st), "NUFFT spread");
   else
     AFC_CUDA(nufft3_spread_dev(L, positions, values, npts, plan->grid, st), "NUFFT spread");
@@ -3290,14 +3309,14 @@ afc_status afc_nufft3d_type2(afc_nufft3d_plan plan, const void* modes, const dou
   const bool cap = stream_capturing(st);
   AFC_CUDA(plan->fence.before(st, cap), "NUFFT ordering");
   const NuLaunch3 L = nu_launch3(*plan);
+  bool tiled = false;
+  afc_status s = nu3_reserve(*plan, npts, false, cap, &tiled);
+  if (s != AFC_OK) return s;
   AFC_CUDA(cudaMemsetAsync(plan->grid, 0, (size_t)(L.mx * L.my * L.mz) * 16, st), "NUFFT grid");
   const double* dc = plan->deconv;
   AFC_CUDA(nufft3_modes_dev(L, dc, dc + L.nx, dc + L.nx + L.ny, modes, plan->grid, true, st), "NUFFT modes");
   // the reference's three normalized inverse axis passes: scale 1/(mx my mz)
-  afc_status s = afc_execute(plan->fft, plan->grid, plan->grid, AFC_INVERSE, stream);
-  if (s != AFC_OK) return s;
-  bool tiled = false;
-  s = nu3_reserve(*plan, npts, &tiled);
+  s = afc_execute(plan->fft, plan->grid, plan->grid, AFC_INVERSE, stream);
   if (s != AFC_OK) return s;
   if (tiled)
     AFC_CUDA(nufft3_tiled_dev(L, plan->tiles, false, positions, plan->grid, npts, out, st), "NUFFT interpolation");

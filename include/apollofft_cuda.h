@@ -292,9 +292,9 @@ AFC_API afc_status afc_hilbert_plan_destroy(afc_hilbert_plan plan);
  * spreading, the FFT of this library and the deconvolution follow the
  * reference step by step (type 1 spreads with atomic adds instead of the
  * reference's bucket sort, so sums differ in rounding only).  Calls on one plan
- * share its grid: calls on the same stream are ordered, overlapping calls on
- * different streams race.  Invalid n, dx, sigma < 2 or width outside 2..32 ->
- * AFC_ERR_VALIDATION. */
+ * share its grid: overlapping calls on different streams are ordered on the GPU
+ * by events, which calls captured into a graph skip.  Invalid n, dx, sigma < 2
+ * or width outside 2..32 -> AFC_ERR_VALIDATION. */
 typedef struct afc_nufft_plan_s* afc_nufft_plan;
 AFC_API afc_status afc_nufft1d_plan_create(afc_nufft_plan* out, int64_t n, double dx, int64_t sigma,
                                            int64_t kernel_width, int device);
@@ -316,7 +316,11 @@ AFC_API afc_status afc_nufft_plan_destroy(afc_nufft_plan plan);
  * the reference's normalized inverse axis passes (dimension_3d.rs:548-551):
  * out[j] ~ sum_k modes_k exp(+2 pi i (...)) / (mx my mz).  Spreading uses
  * atomic adds instead of the reference's bucket sort (rounding differs only).
- * One grid per plan: overlapping calls on different streams race.
+ * One grid per plan: overlapping calls on different streams are ordered on
+ * the GPU by events, which calls captured into a graph skip.  Per-point buffers
+ * grow, with a synchronous allocation, when a call brings more points than any
+ * before it; a captured call that would have to grow them takes the per-point
+ * kernels, and buffers a captured call used live as long as the plan.
  * afc_nufft3d_grid_dims writes (mx, my, mz). */
 typedef struct afc_nufft3d_plan_s* afc_nufft3d_plan;
 AFC_API afc_status afc_nufft3d_plan_create(afc_nufft3d_plan* out, int64_t nx, int64_t ny, int64_t nz, double dx,

@@ -149,3 +149,44 @@ def test_3d_interpolation_repeats(afc, cuda, shape, w, npts):
         assert torch.equal(torch.view_as_real(plan.type2(modes, pos)), torch.view_as_real(first))
     swap = torch.randperm(npts, device="cuda", generator=g)
     assert torch.equal(torch.view_as_real(plan.type2(modes, pos[swap].contiguous())), torch.view_as_real(first[swap]))
+
+
+@pytest.mark.parametrize("first", ["captured", "before"])
+@pytest.mark.parametrize("shape,w", [((16, 16, 16), 6), ((8, 8, 8), 6), ((4, 4, 4), 10)])
+def test_3d_captured_buffers_stay(afc, cuda, shape, w, first):
+    # Both types captured, on a plan that has never run (per-point kernels: a
+    # capture allocates nothing) or has run with as many points (its buffers'
+    # addresses are in the graph); then larger calls, which grow the buffers
+    # twice, and others' allocations in between.
+    from apollofft_b200.nufft import NufftPlan3D
+    npts = 1500
+    g = torch.Generator(device="cuda").manual_seed(w)
+    dims = torch.tensor(shape, dtype=torch.float64, device="cuda")
+    pos = [(torch.rand(k * npts, 3, dtype=torch.float64, device="cuda", generator=g) * dims).contiguous()
+           for k in (1, 3, 20)]
+    val = [torch.randn(k * npts, dtype=torch.complex128, device="cuda", generator=g) for k in (1, 3, 20)]
+    modes = torch.randn(shape, dtype=torch.complex128, device="cuda", generator=g)
+    plan, other = (NufftPlan3D(shape, (1.0, 1.0, 1.0), 2, w) for _ in range(2))
+    big = NufftPlan3D((4, 4, 4), (1.0, 1.0, 1.0), 2, 10)  # loads the per-point kernels outside a capture
+    big.type2(big.type1(pos[0], val[0]), pos[0])
+    want1, want2 = other.type1(pos[0], val[0]), other.type2(modes, pos[0])
+    if first == "before":
+        plan.type2(plan.type1(pos[0], val[0]), pos[0])
+    out1, out2 = torch.zeros_like(want1), torch.zeros_like(want2)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        plan.type1(pos[0], val[0], out=out1)
+        plan.type2(modes, pos[0], out=out2)
+    for k in (1, 2):
+        got1, got2 = plan.type1(pos[k], val[k]), plan.type2(modes, pos[k])
+        other.type1(pos[k], val[k])
+        out1.zero_()
+        out2.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        # sums of the same products in another order
+        assert rel_l2(out1.cpu().numpy(), want1.cpu().numpy()) < 1e-13
+        assert rel_l2(out2.cpu().numpy(), want2.cpu().numpy()) < 1e-13
+        assert rel_l2(plan.type1(pos[k], val[k]).cpu().numpy(), got1.cpu().numpy()) < 1e-13
+        assert torch.equal(torch.view_as_real(plan.type2(modes, pos[k])), torch.view_as_real(got2))
