@@ -1404,7 +1404,7 @@ struct afc_nufft3d_plan_s {
   double* deconv = nullptr;  // nx + ny + nz factors, axis after axis
   void* grid = nullptr;      // mx my mz complex128, C order
   afc::NuTileLaunch tiles;   // B = 0: per-point kernels
-  NuPointBuf buckets, records;
+  NuPointBuf buckets, records, slots;
   std::vector<void*> retired;  // outgrown buffers that captured graphs still use
   std::mutex mu;             // one caller enqueues on the grid at a time
   afc::Fence fence;          // the grid's (and tile buffers') last use on the GPU
@@ -2405,7 +2405,7 @@ afc_nufft_plan_s::~afc_nufft_plan_s() {
 afc_nufft3d_plan_s::~afc_nufft3d_plan_s() {
   for (int* b : {tiles.cnt, tiles.off})
     if (b) cudaFree(b);
-  for (void* b : {buckets.p, records.p})
+  for (void* b : {buckets.p, records.p, slots.p})
     if (b) cudaFree(b);
   for (void* b : retired) cudaFree(b);
   if (fft) afc_plan_destroy(fft);
@@ -3228,21 +3228,31 @@ static afc_status nu3_grow(afc_nufft3d_plan_s& p, NuPointBuf& b, int64_t npts, i
 // The per-point buffers of a call, grown (synchronous allocation) when it brings
 // more points than any call before it.  *tiled false: the per-point kernels run,
 // which need none -- a captured call cannot allocate.
-static afc_status nu3_reserve(afc_nufft3d_plan_s& p, int64_t npts, bool boxes, bool cap, bool* tiled) {
-  const int64_t slice = std::min<int64_t>(npts, kNu3Slice);
+static afc_status nu3_reserve(afc_nufft3d_plan_s& p, int64_t npts, bool boxes, bool interp, bool cap, bool* tiled) {
+  struct Need {
+    NuPointBuf* b;
+    int64_t n, most;
+    size_t per_point;
+    const char* what;
+  } need[3] = {{&p.buckets, npts, INT32_MAX, 3 * sizeof(int), "NUFFT point buckets"},
+               {&p.records, std::min<int64_t>(npts, kNu3Slice), kNu3Slice, nufft3_rec_bytes(p.w), "NUFFT point records"},
+               {&p.slots, std::min<int64_t>(npts, kNu3Slice), kNu3Slice, nufft3_slot_bytes(p.w), "NUFFT point sums"}};
+  const int cnt = !boxes ? 1 : interp ? 3 : 2;
   *tiled = p.tiles.B != 0 && npts > 0 && npts <= INT32_MAX;
-  if (cap && (npts > p.buckets.cap || (boxes && slice > p.records.cap))) *tiled = false;
+  for (int i = 0; i < cnt; ++i)
+    if (cap && need[i].n > need[i].b->cap) *tiled = false;
   if (!*tiled) return AFC_OK;
-  afc_status s = nu3_grow(p, p.buckets, npts, INT32_MAX, 3 * sizeof(int), "NUFFT point buckets");
-  if (s == AFC_OK && boxes)
-    s = nu3_grow(p, p.records, slice, kNu3Slice, nufft3_rec_bytes(p.w), "NUFFT point records");
-  if (s != AFC_OK) return s;
-  if (cap) p.buckets.captured = true;
-  if (cap && boxes) p.records.captured = true;
+  for (int i = 0; i < cnt; ++i) {
+    const Need& d = need[i];
+    afc_status s = nu3_grow(p, *d.b, d.n, d.most, d.per_point, d.what);
+    if (s != AFC_OK) return s;
+    if (cap) d.b->captured = true;
+  }
   p.tiles.tile = static_cast<int*>(p.buckets.p);
   p.tiles.rank = p.tiles.tile + p.buckets.cap;
   p.tiles.idx = p.tiles.rank + p.buckets.cap;
   p.tiles.rec = static_cast<double*>(p.records.p);
+  p.tiles.slots = static_cast<double2*>(p.slots.p);
   return AFC_OK;
 }
 
@@ -3280,11 +3290,11 @@ afc_status afc_nufft3d_type1(afc_nufft3d_plan plan, const double* positions, con
   const NuLaunch3 L = nu_launch3(*plan);
   const bool boxes = nufft3_boxes(L);
   bool tiled = false;
-  afc_status r = nu3_reserve(*plan, npts, boxes, cap, &tiled);
+  afc_status r = nu3_reserve(*plan, npts, boxes, false, cap, &tiled);
   if (r != AFC_OK) return r;
   AFC_CUDA(cudaMemsetAsync(plan->grid, 0, (size_t)(L.mx * L.my * L.mz) * 16, st), "NUFFT grid");
   if (tiled && boxes)
-    AFC_CUDA(nufft3_boxes_dev(L, plan->tiles, positions, values, npts, plan->grid, st), "NUFFT spread");
+    AFC_CUDA(nufft3_boxes_dev(L, plan->tiles, true, positions, values, npts, plan->grid, nullptr, st), "NUFFT spread");
   else if (tiled)
     AFC_CUDA(nufft3_tiled_dev(L, plan->tiles, true, positions, values, npts, plan->grid, st), "NUFFT spread");
   else
@@ -3309,8 +3319,9 @@ afc_status afc_nufft3d_type2(afc_nufft3d_plan plan, const void* modes, const dou
   const bool cap = stream_capturing(st);
   AFC_CUDA(plan->fence.before(st, cap), "NUFFT ordering");
   const NuLaunch3 L = nu_launch3(*plan);
+  const bool boxes = nufft3_boxes(L);
   bool tiled = false;
-  afc_status s = nu3_reserve(*plan, npts, false, cap, &tiled);
+  afc_status s = nu3_reserve(*plan, npts, boxes, true, cap, &tiled);
   if (s != AFC_OK) return s;
   AFC_CUDA(cudaMemsetAsync(plan->grid, 0, (size_t)(L.mx * L.my * L.mz) * 16, st), "NUFFT grid");
   const double* dc = plan->deconv;
@@ -3318,7 +3329,10 @@ afc_status afc_nufft3d_type2(afc_nufft3d_plan plan, const void* modes, const dou
   // the reference's three normalized inverse axis passes: scale 1/(mx my mz)
   s = afc_execute(plan->fft, plan->grid, plan->grid, AFC_INVERSE, stream);
   if (s != AFC_OK) return s;
-  if (tiled)
+  if (tiled && boxes)
+    AFC_CUDA(nufft3_boxes_dev(L, plan->tiles, false, positions, nullptr, npts, plan->grid, out, st),
+             "NUFFT interpolation");
+  else if (tiled)
     AFC_CUDA(nufft3_tiled_dev(L, plan->tiles, false, positions, plan->grid, npts, out, st), "NUFFT interpolation");
   else
     AFC_CUDA(nufft3_interp_dev(L, plan->grid, positions, npts, out, st), "NUFFT interpolation");

@@ -242,15 +242,17 @@ struct NuTileLaunch {
   int* tile = nullptr;  // npts
   int* rank = nullptr;  // npts
   int* idx = nullptr;   // npts
-  double* rec = nullptr;  // box kernel: a record per point of a slice
+  double* rec = nullptr;  // box kernels: a record per point of a slice
+  double2* slots = nullptr;  // box interpolation: the CTAs' sums for each point of a slice
 };
-// Points the box kernel takes at a time (bounds its record buffer).
+// Points the box kernels take at a time (bounds their record and slot buffers).
 constexpr long long kNu3Slice = 1 << 18;
 bool nufft3_boxes(const NuLaunch3& L);
-size_t nufft3_box_smem(int w);
+size_t nufft3_box_smem(int w, bool spread);
+size_t nufft3_slot_bytes(int w);
 size_t nufft3_rec_bytes(int w);
-cudaError_t nufft3_boxes_dev(const NuLaunch3& L, const NuTileLaunch& TL, const double* pos, const void* val,
-                             long long npts, void* grid, cudaStream_t st);
+cudaError_t nufft3_boxes_dev(const NuLaunch3& L, const NuTileLaunch& TL, bool spread, const double* pos,
+                             const void* val, long long npts, void* grid, void* out, cudaStream_t st);
 int nufft3_tile_size(int w);
 size_t nufft3_tile_smem(int B, int w);
 cudaError_t nufft3_tiled_dev(const NuLaunch3& L, const NuTileLaunch& TL, bool spread, const double* pos,

@@ -654,44 +654,53 @@ __global__ void __launch_bounds__(kNuTileThreads) nu3_spread_tiles(const __grid_
   }
 }
 
-// ─── 3D spreading by boxes of cells ───
-// The tile kernel is bound by shared memory (a 16-byte cell per tap, read and
-// written back) and adds every tile's halo to the grid with atomics, 15 times
-// the cells at w = 6.  Here the cells stay in registers and the points move: a
-// warp owns a box of 8 x 4 x 8 cells and meets every point whose taps reach it
-// (25 boxes per point at w = 6).  Per box the sums are small FP64 matrix products
-// (mma m8n8k4), C[x][z] += wx[point][x] (v wy wz)[point][z], 4 points at a time,
-// for each y and for both parts of v.  One operand element per lane feeds 8 FMAs.
-// Measured at 2^18 points on 128^3 cells, w = 6 (kernel alone): tiles 1650 us;
-// boxes with scalar FMAs, bound by the broadcast weight loads, 1095 us; these 612
-// us, bound by the shared-memory loads and chunk barriers ahead of each group
-// (FP64 pipe 6-8 % busy).
-// Interpolation keeps the tile kernel: a point's boxes would have to add their
-// parts to its value in whatever order they finish, and 711 us of box kernel and
-// 54 us of records are no gain on its 784 us that would be worth values that
-// change in the last bit from call to call.
-//  nu3_points: one record per point in tile order: value, centre, and the axis
-//              weights between runs of seven zeros, so no tap is range-checked;
+// ─── 3D spreading and interpolation by boxes of cells ───
+// The tile kernels are bound by shared memory (a 16-byte cell per tap, read and
+// for spreading written back) and spreading adds every tile's halo to the grid
+// with atomics, 15 times the cells at w = 6.  Here the cells stay in registers
+// and the points move: a warp owns a box of 8 x 4 x 8 cells and meets every
+// point whose taps reach it (25 boxes per point at w = 6).  Per box the sums are
+// small FP64 matrix products (mma m8n8k4):
+//   spreading      C[x][z] += wx[point][x] (v wy wz)[point][z], 4 points at a
+//                  time, for each y and for both parts of v;
+//   interpolation  D[point][z] = sum_x wx[point][x] cell[x][z], 8 points at a
+//                  time, then summed over y and z with their weights.
+// One operand element per lane feeds 8 FMAs.
+//  nu3_points: one record per point in tile order: value, centre, index, and the
+//              axis weights between runs of seven zeros, so no tap is range-checked;
 //  nu3_boxes:  a CTA of 8 warps owns 16 x 8 x 16 cells and streams the records of
 //              the tiles within w cells of it through shared memory, the next chunk
 //              in flight while one is worked on.  Each warp lists the records that
 //              meet its box and takes them in groups.
-// Boxes partition the grid: each cell is written once, without atomics unless a
-// box's points are split over CTAs.
+//  nu3_collect: interpolation only.  A CTA adds up its eight boxes' parts of a
+//              point in one order and stores the sum in a slot of the point that
+//              its place relative to the point's first tap determines (7.7 CTAs
+//              per point on average at w = 6); this adds the slots in order.  So a
+//              value is the same bits whatever the order the CTAs ran in.
+// Boxes partition the grid: spreading writes each cell once, without atomics
+// unless a box's points are split over CTAs.
 constexpr int kNuBoxThreads = 256;
-// chunk and CTAs per SM measured at 2^18 points on 128^3 cells, w = 6: 32 points,
-// three CTAs 798 us for the whole call, 64 points, two CTAs 845, 32 points, two
-// CTAs 917
+// chunk and CTAs per SM measured at 2^18 points on 128^3 cells, w = 6 (spreading /
+// interpolation with atomics): 32 points, three CTAs 798 / 900 us for the whole
+// call, 64 points, two CTAs 845 / 927, 32 points, two CTAs 917 / 1027
 constexpr int kNuBoxChunk = 32;
 constexpr int kNuBoxRuns = 64;  // contiguous runs of candidate points per CTA
 
-// Record: v.x, v.y, centre cells (three of four ints), then x, y and z weights.
+// Record: v.x, v.y, centre cells and index (four ints), then x, y and z weights.
 __host__ __device__ constexpr int nu_xo(int) { return 11; }
 __host__ __device__ constexpr int nu_yo(int T) { return 18 + T; }
 __host__ __device__ constexpr int nu_zo(int T) { return 25 + 2 * T; }
 __host__ __device__ constexpr int nu_rec(int T) { return (32 + 3 * T + 1) / 2 * 2; }
 constexpr int kNuZeros = 16;  // a block of zeros: the record of the slots that fill up a group
-__host__ __device__ constexpr int nu_list() { return (kNuBoxChunk + 8) * 4; }  // ints per warp
+__host__ __device__ constexpr int nu_list() { return (kNuBoxChunk + 16) * 4; }  // ints per warp
+// The CTA blocks of 16 x 8 x 16 cells that the taps of a point with centre cell c
+// reach along an axis of nb blocks of 2^sh cells: the first (c - w) >> sh, then
+// upward, wrapping.
+__host__ __device__ constexpr int nu_slots(int w, int sh) { return ((2 * w + (1 << sh) - 1) >> sh) + 1; }  // at most
+__host__ __device__ constexpr int nu_slots3(int w) { return nu_slots(w, 4) * nu_slots(w, 3) * nu_slots(w, 4); }
+__device__ __forceinline__ int nu_blocks(int c, int w, int sh, int nb) {
+  return min(nb, ((c + w) >> sh) - ((c - w) >> sh) + 1);
+}
 
 __device__ __forceinline__ void nu_cp16(void* smem, const void* gmem) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem)
@@ -701,7 +710,7 @@ __device__ __forceinline__ void nu_cp16(void* smem, const void* gmem) {
 // Block of kNuPts points, three threads each (one per axis): the records are put
 // together in shared memory and stored whole (rows written straight to global
 // memory were 13 eight-byte stores per thread to 32 places each: 97 us at 2^18
-// points).
+// points).  val null (interpolation): no value in the record.
 constexpr int kNuPts = 64;
 template <int T>
 __global__ void __launch_bounds__(3 * kNuPts) nu3_points(const __grid_constant__ NuGeom3 g, const int* __restrict__ idx,
@@ -729,9 +738,10 @@ __global__ void __launch_bounds__(3 * kNuPts) nu3_points(const __grid_constant__
       int* c = reinterpret_cast<int*>(r + 2);
       c[a] = (int)((long long)rt & (m - 1));
       if (a == 0) {
-        const double2 v = val[j];
+        const double2 v = val ? val[j] : make_double2(0.0, 0.0);
         r[0] = v.x;
         r[1] = v.y;
+        c[3] = j;
       }
     }
     __syncthreads();
@@ -749,12 +759,15 @@ __device__ __forceinline__ void nu_mma(double2& d, double a, double b) {
                : "d"(a), "d"(b));
 }
 
-// Records -> cells (add: the cells may be shared with other CTAs).
+// SPREAD: records -> cells (add: the cells may be shared with other CTAs);
+// else: cells -> a slot of `out` per point and CTA that its taps reach.
+template <bool SPREAD>
 __global__ void __launch_bounds__(kNuBoxThreads, 3)
     nu3_boxes(int mx, int my, int mz, int w, const int* __restrict__ off, const double* __restrict__ rec,
-              double2* __restrict__ grid, int add) {
+              double2* __restrict__ grid, double2* __restrict__ out, int add) {
   extern __shared__ __align__(16) double nu_sm[];
   __shared__ int run_start[kNuBoxRuns], run_pre[kNuBoxRuns + 1];
+  __shared__ int s_dst[2][kNuBoxChunk];  // !SPREAD: where the CTA's sum of each point goes, by chunk parity
   const int T = 2 * w + 1, S = nu_rec(T);
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int nby = my / 8, nbz = mz / 16;
@@ -775,7 +788,7 @@ __global__ void __launch_bounds__(kNuBoxThreads, 3)
   }
   const int ZB = 2 * kNuBoxChunk * S;  // the zero block
   if (tid < kNuZeros) nu_sm[ZB + tid] = 0.0;
-  int4* const list = reinterpret_cast<int4*>(nu_sm + ZB + kNuZeros) + wid * (kNuBoxChunk + 8);
+  int4* const list = reinterpret_cast<int4*>(nu_sm + ZB + kNuZeros) + wid * (kNuBoxChunk + 16);
   __syncthreads();
   if (tid == 0) {
     run_pre[0] = 0;
@@ -810,26 +823,54 @@ __global__ void __launch_bounds__(kNuBoxThreads, 3)
   const int x0 = gx0 + (wid >> 2) * 8, y0 = gy0 + ((wid >> 1) & 1) * 4, z0 = gz0 + (wid & 1) * 8;
   const int lr = lane >> 2, lk = lane & 3;
   stage(c, 0);
-  double2 acc[4][2];  // C[x = lr][z = 2 lk, 2 lk + 1] of row y, real and imaginary
+  double2 acc[4][2];     // SPREAD: C[x = lr][z = 2 lk, 2 lk + 1] of row y, real and imaginary
+  double cell[4][2][2];  // else: B[x = lk + 4 s][z = lr] of row y, real and imaginary
+  // else: the boxes' parts of a chunk's points, by chunk parity, box and point
+  double2* const part = reinterpret_cast<double2*>(nu_sm + ZB + kNuZeros + (kNuBoxThreads / 32) * nu_list() / 2);
   const long long sx = (long long)my * mz;
+  if constexpr (SPREAD) {
 #pragma unroll
-  for (int j = 0; j < 4; ++j) acc[j][0] = acc[j][1] = make_double2(0.0, 0.0);
-  bool any = false;
-  for (int k = 0; c < nchunk; ++k, c += gridDim.y) {
-    const int slot = k & 1;
-    if (c + (int)gridDim.y < nchunk) {
-      stage(c + gridDim.y, slot ^ 1);
-      asm volatile("cp.async.wait_group 1;\n" ::: "memory");
-    } else {
-      asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    for (int j = 0; j < 4; ++j) acc[j][0] = acc[j][1] = make_double2(0.0, 0.0);
+  } else {
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int s = 0; s < 2; ++s) {
+        const double2 v = grid[(x0 + 4 * s + lk) * sx + (long long)(y0 + j) * mz + z0 + lr];
+        cell[j][s][0] = v.x;
+        cell[j][s][1] = v.y;
+      }
+  }
+  // the parts of the chunk of this parity, by one warp, a lane per point; they are
+  // next written two chunks on
+  auto sum_parts = [&](int slot) {
+    const int dst = s_dst[slot][lane];
+    if (dst < 0) return;
+    const double2* q = part + slot * 8 * kNuBoxChunk + lane;
+    double2 v = q[0];
+#pragma unroll
+    for (int b8 = 1; b8 < 8; ++b8) {
+      v.x += q[b8 * kNuBoxChunk].x;
+      v.y += q[b8 * kNuBoxChunk].y;
     }
-    __syncthreads();
+    out[dst] = v;
+  };
+  static_assert(kNuBoxThreads == 256 && kNuBoxChunk == 32, "8 boxes of a warp each, a lane per point of the chunk");
+  bool any = false;
+  int k = 0;
+  for (; c < nchunk; ++k, c += gridDim.y) {
+    const int slot = k & 1;
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    __syncthreads();  // this chunk is here, the one before it done by every warp
+    if (c + (int)gridDim.y < nchunk) stage(c + gridDim.y, slot ^ 1);
+    if (!SPREAD && k > 0 && wid == (k & 7)) sum_parts(slot ^ 1);
     // the chunk's records that meet this box: offsets of its first weights (in
     // doubles from nu_sm; a box may start up to seven zeros before a row)
+    double2* const mine = part + (slot * 8 + wid) * kNuBoxChunk;
+    const bool slots = !SPREAD && wid == (k + 4 & 7);  // this warp works out the points' slots
     int n = 0;
-#pragma unroll
-    for (int h = 0; h < kNuBoxChunk / 32; ++h) {
-      const int p = lane + 32 * h, rp = (slot * kNuBoxChunk + p) * S;
+    {
+      const int p = lane, rp = (slot * kNuBoxChunk + p) * S;
       bool hit = false;
       int4 e = make_int4(0, 0, 0, 0);
       if (p * nchunk + c < total) {
@@ -837,48 +878,115 @@ __global__ void __launch_bounds__(kNuBoxThreads, 3)
         const int dx = (x0 - cc.x + w) & (mx - 1), dy = (y0 - cc.y + w) & (my - 1), dz = (z0 - cc.z + w) & (mz - 1);
         hit = (dx < T || dx > mx - 8) && (dy < T || dy > my - 4) && (dz < T || dz > mz - 8);
         e = make_int4(rp + nu_xo(T) + (dx < T ? dx : dx - mx), rp + nu_yo(T) + (dy < T ? dy : dy - my),
-                      rp + nu_zo(T) + (dz < T ? dz : dz - mz), rp);
+                      rp + nu_zo(T) + (dz < T ? dz : dz - mz), SPREAD ? rp : p);
+        if (slots) {
+          int dst = -1;
+          const int nbx = mx / 16;
+          const int bxr = (gx0 / 16 - ((cc.x - w) >> 4)) & (nbx - 1), byr = (gy0 / 8 - ((cc.y - w) >> 3)) & (nby - 1);
+          const int bzr = (gz0 / 16 - ((cc.z - w) >> 4)) & (nbz - 1);
+          if (bxr < nu_blocks(cc.x, w, 4, nbx) && byr < nu_blocks(cc.y, w, 3, nby) && bzr < nu_blocks(cc.z, w, 4, nbz))
+            dst = cc.w * nu_slots3(w) + (bxr * nu_slots(w, 3) + byr) * nu_slots(w, 4) + bzr;
+          s_dst[slot][p] = dst;
+        }
+      } else if (slots) {
+        s_dst[slot][p] = -1;
       }
       const unsigned mask = __ballot_sync(0xffffffffu, hit);
-      if (hit) list[n + __popc(mask & ((1u << lane) - 1))] = e;
-      n += __popc(mask);
+      if (hit) list[__popc(mask & ((1u << lane) - 1))] = e;
+      else if (!SPREAD) mine[p] = make_double2(0.0, 0.0);
+      n = __popc(mask);
     }
-    any = any || n;
     // fills up the last group, and one group past it for the loop's look-ahead
-    if (lane < 8) list[n + lane] = make_int4(ZB, ZB, ZB, ZB);
+    if (lane < 16) list[n + lane] = make_int4(ZB, ZB, ZB, SPREAD ? ZB : -1);
     __syncwarp();
-    int4 e = list[lk];
+    constexpr int G = SPREAD ? 4 : 8;
+    int4 e = list[SPREAD ? lk : lr];
 #pragma unroll 2
-    for (int i = 0; i < n; i += 4) {
-      const int4 e_next = list[i + 4 + lk];
-      const double2 v = *reinterpret_cast<const double2*>(nu_sm + e.w);
-      const double wz = nu_sm[e.z + lr], ax = nu_sm[e.x + lr];
-      const double vr = v.x * wz, vi = v.y * wz;
+    for (int i = 0; i < n; i += G) {
+      const int4 e_next = list[i + G + (SPREAD ? lk : lr)];
+      if constexpr (SPREAD) {
+        const double2 v = *reinterpret_cast<const double2*>(nu_sm + e.w);
+        const double wz = nu_sm[e.z + lr], ax = nu_sm[e.x + lr];
+        const double vr = v.x * wz, vi = v.y * wz;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const double wy = nu_sm[e.y + j];
-        nu_mma(acc[j][0], ax, vr * wy);
-        nu_mma(acc[j][1], ax, vi * wy);
+        for (int j = 0; j < 4; ++j) {
+          const double wy = nu_sm[e.y + j];
+          nu_mma(acc[j][0], ax, vr * wy);
+          nu_mma(acc[j][1], ax, vi * wy);
+        }
+      } else {
+        const double a0 = nu_sm[e.x + lk], a1 = nu_sm[e.x + 4 + lk];
+        const double w0 = nu_sm[e.z + 2 * lk], w1 = nu_sm[e.z + 2 * lk + 1];
+        double re = 0.0, im = 0.0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          double2 dr = make_double2(0.0, 0.0), di = dr;
+          nu_mma(dr, a0, cell[j][0][0]);
+          nu_mma(di, a0, cell[j][0][1]);
+          nu_mma(dr, a1, cell[j][1][0]);
+          nu_mma(di, a1, cell[j][1][1]);
+          const double wy = nu_sm[e.y + j];
+          re = fma(wy, fma(w1, dr.y, w0 * dr.x), re);
+          im = fma(wy, fma(w1, di.y, w0 * di.x), im);
+        }
+#pragma unroll
+        for (int o = 1; o < 4; o <<= 1) {
+          re += __shfl_xor_sync(0xffffffffu, re, o);
+          im += __shfl_xor_sync(0xffffffffu, im, o);
+        }
+        if (lk == 0 && e.w >= 0) mine[e.w] = make_double2(re, im);
       }
       e = e_next;
     }
-    __syncthreads();  // the slot is refilled
+    any = any || n;
   }
-  if (!any) return;
+  if constexpr (!SPREAD) {
+    __syncthreads();
+    if (wid == 0) sum_parts(k & 1 ^ 1);
+  }
+  if constexpr (SPREAD) {
+    if (!any) return;
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    double2* o = grid + (x0 + lr) * sx + (long long)(y0 + j) * mz + z0 + 2 * lk;
-    const double2 c0 = make_double2(acc[j][0].x, acc[j][1].x), c1 = make_double2(acc[j][0].y, acc[j][1].y);
-    if (add) {
-      atomicAdd(&o[0].x, c0.x);
-      atomicAdd(&o[0].y, c0.y);
-      atomicAdd(&o[1].x, c1.x);
-      atomicAdd(&o[1].y, c1.y);
-    } else {
-      o[0] = c0;
-      o[1] = c1;
+    for (int j = 0; j < 4; ++j) {
+      double2* o = grid + (x0 + lr) * sx + (long long)(y0 + j) * mz + z0 + 2 * lk;
+      const double2 c0 = make_double2(acc[j][0].x, acc[j][1].x), c1 = make_double2(acc[j][0].y, acc[j][1].y);
+      if (add) {
+        atomicAdd(&o[0].x, c0.x);
+        atomicAdd(&o[0].y, c0.y);
+        atomicAdd(&o[1].x, c1.x);
+        atomicAdd(&o[1].y, c1.y);
+      } else {
+        o[0] = c0;
+        o[1] = c1;
+      }
     }
   }
+}
+
+// The slots of each point: four lanes take its x and y blocks in turn, then add up
+// in one order.  Centre and index come from the record (three fmod per point
+// otherwise).
+__global__ void nu3_collect(int mx, int my, int mz, int w, const double* __restrict__ rec,
+                            const double2* __restrict__ slots, int npts, double2* __restrict__ out) {
+  const int ny = nu_slots(w, 3), nz = nu_slots(w, 4);
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, i0 = min(t >> 2, npts - 1), l = t & 3;
+  const int4 cc = *reinterpret_cast<const int4*>(rec + (long long)i0 * nu_rec(2 * w + 1) + 2);
+  const int bx = nu_blocks(cc.x, w, 4, mx / 16), by = nu_blocks(cc.y, w, 3, my / 8), bz = nu_blocks(cc.z, w, 4, mz / 16);
+  const double2* q = slots + (long long)cc.w * nu_slots3(w);
+  double2 v = make_double2(0.0, 0.0);
+  for (int i = l; i < bx * by; i += 4) {
+    const double2* r = q + (i / by * ny + i % by) * nz;
+    for (int z = 0; z < bz; ++z) {
+      v.x += r[z].x;
+      v.y += r[z].y;
+    }
+  }
+#pragma unroll
+  for (int o = 1; o < 4; o <<= 1) {
+    v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
+    v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
+  }
+  if (l == 0 && t >> 2 < npts) out[cc.w] = v;
 }
 
 // T: taps per axis at compile time.  A lane holds the point's x-weights in
@@ -1123,22 +1231,26 @@ bool nufft3_boxes(const NuLaunch3& L) {
   const long long lo = std::min(L.mx, std::min(L.my, L.mz)), hi = std::max(L.mx, std::max(L.my, L.mz));
   const int T = 2 * L.w + 1, wt = (L.w + 7) / 8;
   return lo >= 16 && lo >= T + 8 && hi < (1 << 20) && (2 + 2 * wt) * (1 + 2 * wt) * 2 <= kNuBoxRuns &&
-         nufft3_box_smem(L.w) <= 112 * 1024;
+         nufft3_box_smem(L.w, false) <= 112 * 1024;
 }
-size_t nufft3_box_smem(int w) {
+size_t nufft3_box_smem(int w, bool spread) {
   return ((size_t)2 * kNuBoxChunk * nu_rec(2 * w + 1) + kNuZeros) * sizeof(double) +
-         (size_t)(kNuBoxThreads / 32) * nu_list() * sizeof(int);
+         (size_t)(kNuBoxThreads / 32) * nu_list() * sizeof(int) +
+         (spread ? 0 : (size_t)2 * (kNuBoxThreads / 32) * kNuBoxChunk * sizeof(double2));
 }
+size_t nufft3_slot_bytes(int w) { return (size_t)nu_slots3(w) * sizeof(double2); }
 size_t nufft3_rec_bytes(int w) { return (size_t)nu_rec(2 * w + 1) * sizeof(double); }
 
-// Spreads npts points onto the zeroed grid, kNu3Slice points at a time (their
-// records take nufft3_rec_bytes each).
-cudaError_t nufft3_boxes_dev(const NuLaunch3& L, const NuTileLaunch& TL, const double* pos, const void* val,
-                             long long npts, void* grid, cudaStream_t st) {
+// Spreads npts points onto the zeroed grid, or interpolates the grid at them
+// into out; kNu3Slice points at a time (their records take nufft3_rec_bytes each
+// and, interpolating, their slots nufft3_slot_bytes).
+cudaError_t nufft3_boxes_dev(const NuLaunch3& L, const NuTileLaunch& TL, bool spread, const double* pos,
+                             const void* val, long long npts, void* grid, void* out, cudaStream_t st) {
   const NuGeom3 g = geom3(L);
   const int nty = (int)(L.my / 8), ntz = (int)(L.mz / 8), ntiles = (int)(L.mx / 8) * nty * ntz;
-  const size_t smem = nufft3_box_smem(L.w);
-  cudaError_t e = kernel_smem_grant(reinterpret_cast<const void*>(nu3_boxes), smem);
+  const size_t smem = nufft3_box_smem(L.w, spread);
+  auto k = spread ? nu3_boxes<true> : nu3_boxes<false>;
+  cudaError_t e = kernel_smem_grant(reinterpret_cast<const void*>(k), smem);
   if (e != cudaSuccess) return e;
   const int boxes = (int)(L.mx / 16) * (int)(L.my / 8) * (int)(L.mz / 16);
   for (long long p0 = 0; p0 < npts; p0 += kNu3Slice) {
@@ -1162,15 +1274,18 @@ cudaError_t nufft3_boxes_dev(const NuLaunch3& L, const NuTileLaunch& TL, const d
       default: return cudaErrorInvalidValue;
     }
     points<<<(unsigned)((n + kNuPts - 1) / kNuPts), 3 * kNuPts, 0, st>>>(
-        g, TL.idx, ps, static_cast<const double2*>(val) + p0, (int)n, TL.rec);
+        g, TL.idx, ps, spread ? static_cast<const double2*>(val) + p0 : nullptr, (int)n, TL.rec);
     // a box's chunks are dealt to `split` CTAs: about 4096 CTAs in all, so a
     // grid of few boxes, or points crowded into some of them, still fills the chip
     const long long chunks = (n + kNuBoxChunk - 1) / kNuBoxChunk;
     const int split = (int)std::max<long long>(1, std::min<long long>(chunks, std::min(32, 4096 / boxes)));
-    nu3_boxes<<<dim3((unsigned)boxes, (unsigned)split), kNuBoxThreads, smem, st>>>(
-        (int)L.mx, (int)L.my, (int)L.mz, L.w, TL.off, TL.rec, static_cast<double2*>(grid),
+    k<<<dim3((unsigned)boxes, (unsigned)split), kNuBoxThreads, smem, st>>>(
+        (int)L.mx, (int)L.my, (int)L.mz, L.w, TL.off, TL.rec, static_cast<double2*>(grid), TL.slots,
         split > 1 || npts > kNu3Slice);
-    count_launch(5);
+    if (!spread)
+      nu3_collect<<<(unsigned)((4 * n + 255) / 256), 256, 0, st>>>((int)L.mx, (int)L.my, (int)L.mz, L.w, TL.rec, TL.slots,
+                                                                   (int)n, static_cast<double2*>(out) + p0);
+    count_launch(spread ? 5 : 6);
   }
   return cudaGetLastError();
 }

@@ -43,6 +43,25 @@ def test_3d_boxes(afc, oracle, cuda, shape, w, npts, layout):
     assert rel_l2(y2, ref.type2(modes, pos, oracle)) < 1e-12
 
 
+@pytest.mark.parametrize("shape,w", [((16, 16, 16), 2), ((8, 10, 13), 3)])
+def test_3d_slices(afc, oracle, cuda, shape, w):
+    # more points than the box kernels take at a time: their buffers are used again,
+    # every slice adds to the grid, the second slice's values go behind the first's
+    from apollofft_b200.nufft import NufftPlan3D
+    npts = (1 << 18) + 7
+    rng = np.random.default_rng(w)
+    ref = RefPlan3(shape, (1.0, 1.0, 1.0), 2, w)
+    pos = np.ascontiguousarray(rng.uniform(0, 1, (npts, 3)) * np.array(shape))
+    val = rng.standard_normal(npts) + 1j * rng.standard_normal(npts)
+    modes = rng.standard_normal(shape) + 1j * rng.standard_normal(shape)
+    plan = NufftPlan3D(shape, (1.0, 1.0, 1.0), 2, w)
+    p_t = torch.from_numpy(pos).cuda()
+    y1 = plan.type1(p_t, torch.from_numpy(val).cuda()).cpu().numpy()
+    y2 = plan.type2(torch.from_numpy(modes).cuda(), p_t).cpu().numpy()
+    assert rel_l2(y1, ref.type1(pos, val, oracle)) < 1e-12
+    assert rel_l2(y2, ref.type2(modes, pos, oracle)) < 1e-12
+
+
 @pytest.mark.parametrize("n,w,npts", [(1, 2, 5), (3, 6, 40), (64, 4, 1000), (257, 6, 3001), (1000, 8, 500), (50, 13, 64),
                                       (40, 20, 64)])
 def test_1d_widths(afc, oracle, cuda, n, w, npts):
@@ -136,8 +155,7 @@ def test_3d_position_not_finite(afc, cuda, bad, shape, w):
 @pytest.mark.parametrize("shape,w,npts", [((16, 16, 16), 6, 20000), ((20, 16, 12), 9, 3000), ((8, 8, 8), 6, 3000),
                                           ((4, 4, 4), 10, 500)])
 def test_3d_interpolation_repeats(afc, cuda, shape, w, npts):
-    # each value is summed by one warp in one order, whatever the order the points
-    # were sorted in
+    # whatever order the boxes run in and the points were sorted in
     from apollofft_b200.nufft import NufftPlan3D
     g = torch.Generator(device="cuda").manual_seed(npts)
     pos = torch.rand(npts, 3, dtype=torch.float64, device="cuda", generator=g)
