@@ -1099,13 +1099,23 @@ static unsigned nu_grid(long long work) {
   return (unsigned)b;
 }
 
-// Sorting costs three passes over the points (about 60 us per million); below
-// about a million taps, or when the window of 32 cells leaves few centre cells,
-// the direct atomics are faster unless the points crowd the grid.
+// Sorting costs three passes over the points (about 60 us per million) and three
+// launches, and saves atomics: about 20 per window of 32 cells and 32 points
+// instead of 2 T per point, and the contention of crowded points.  Measured at
+// uniform / crowded points (the middle sampled most), us unsorted -> sorted:
+//  * from two million taps on, w = 4, n = 4096, 2^20 points 160 -> 195 / 978 -> 312,
+//    n = 65536 156 -> 146 / 328 -> 210, w = 6 219 -> 166 / 479 -> 233;
+//  * from 16 points a cell on, w = 4, n = 1024, 2^16 points 35 -> 51 / 136 -> 52;
+//  * below six taps a cell the windows hold a point or two: w = 4, n = 2^22, 2^22
+//    points 1112 -> 1116 / 1101 -> 1345: unsorted;
+//  * w <= 3, n = 1024, 2^20 points: w = 2 136 -> 357 / 917 -> 371, w = 3 286 -> 365:
+//    unsorted, but for the few cells whose atomics serialize (w = 2, n = 128, 2^18
+//    points 183 -> 116 / 562 -> 164).
 bool nufft_sorted(const NuLaunch& L, long long npts) {
   const long long T = 2 * L.w + 1;
-  return T <= 25 && L.m >= 64 && L.m < (1ll << 31) - 64 && npts <= INT32_MAX &&
-         (npts * T >= (1 << 21) || (npts >= 16 * L.m && npts >= 4096));
+  if (T > 25 || L.m < 64 || L.m >= (1ll << 31) - 64 || npts > INT32_MAX) return false;
+  if (T < 9) return L.m <= 256 && npts >= 256 * L.m;
+  return npts * T >= 6 * L.m && (npts * T >= (1 << 21) || (npts >= 16 * L.m && npts >= 4096));
 }
 
 cudaError_t nufft_spread_dev(const NuLaunch& L, const NuTileLaunch& TL, const double* pos, const void* val,

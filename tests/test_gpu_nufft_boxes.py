@@ -8,7 +8,7 @@ import pytest
 import torch
 
 from conftest import rel_l2
-from oracle.nufft import RefPlan, RefPlan3
+from oracle.nufft import RefPlan, RefPlan3, c_type1_1d, c_type1_3d, c_type2_3d
 
 pytestmark = pytest.mark.gpu
 
@@ -43,23 +43,23 @@ def test_3d_boxes(afc, oracle, cuda, shape, w, npts, layout):
     assert rel_l2(y2, ref.type2(modes, pos, oracle)) < 1e-12
 
 
-@pytest.mark.parametrize("shape,w", [((16, 16, 16), 2), ((8, 10, 13), 3)])
+@pytest.mark.parametrize("shape,w", [((16, 16, 16), 4), ((16, 10, 13), 5)])
 def test_3d_slices(afc, oracle, cuda, shape, w):
     # more points than the box kernels take at a time: their buffers are used again,
     # every slice adds to the grid, the second slice's values go behind the first's
     from apollofft_b200.nufft import NufftPlan3D
     npts = (1 << 18) + 7
     rng = np.random.default_rng(w)
-    ref = RefPlan3(shape, (1.0, 1.0, 1.0), 2, w)
+    dx = (1.0, 1.0, 1.0)
     pos = np.ascontiguousarray(rng.uniform(0, 1, (npts, 3)) * np.array(shape))
     val = rng.standard_normal(npts) + 1j * rng.standard_normal(npts)
     modes = rng.standard_normal(shape) + 1j * rng.standard_normal(shape)
-    plan = NufftPlan3D(shape, (1.0, 1.0, 1.0), 2, w)
+    plan = NufftPlan3D(shape, dx, 2, w)
     p_t = torch.from_numpy(pos).cuda()
     y1 = plan.type1(p_t, torch.from_numpy(val).cuda()).cpu().numpy()
     y2 = plan.type2(torch.from_numpy(modes).cuda(), p_t).cpu().numpy()
-    assert rel_l2(y1, ref.type1(pos, val, oracle)) < 1e-12
-    assert rel_l2(y2, ref.type2(modes, pos, oracle)) < 1e-12
+    assert rel_l2(y1, c_type1_3d(shape, dx, 2, w, pos, val)) < 1e-12
+    assert rel_l2(y2, c_type2_3d(shape, dx, 2, w, modes, pos)) < 1e-12
 
 
 @pytest.mark.parametrize("n,w,npts", [(1, 2, 5), (3, 6, 40), (64, 4, 1000), (257, 6, 3001), (1000, 8, 500), (50, 13, 64),
@@ -78,6 +78,43 @@ def test_1d_widths(afc, oracle, cuda, n, w, npts):
     y2 = plan.type2(torch.from_numpy(coef).cuda(), p_t).cpu().numpy()
     assert rel_l2(y1, ref.type1(pos, val, oracle)) < 1e-12
     assert rel_l2(y2, ref.type2(coef, pos, oracle)) < 1e-12
+
+
+@pytest.mark.parametrize("n,w,npts", [(32, 2, 16384), (32, 3, 16384), (32, 4, 4096), (33, 5, 4096), (40, 6, 5001),
+                                      (64, 7, 8192), (36, 8, 4097), (32, 9, 4099), (48, 12, 5000), (32, 12, 131),
+                                      (70000, 8, 430_000)])
+def test_1d_sorted(afc, oracle, cuda, n, w, npts):
+    # the widths with kernels of their own (4 .. 8) and any other, a window that
+    # wraps a grid of two windows, a partly filled warp, bins of more than eight
+    # cells (the last case); the case of 131 points is spread unsorted
+    from apollofft_b200.nufft import NufftPlan1D
+    rng = np.random.default_rng(n + w)
+    length = 0.3 * n
+    pos = rng.uniform(-0.2, 1.2, npts) * length
+    pos[: npts // 4] = 0.01 * length * rng.standard_normal(npts // 4)  # crowded about the wrap
+    val = rng.standard_normal(npts) + 1j * rng.standard_normal(npts)
+    y = NufftPlan1D(n, 0.3, 2, w).type1(torch.from_numpy(pos).cuda(), torch.from_numpy(val).cuda()).cpu().numpy()
+    assert rel_l2(y, c_type1_1d(n, 0.3, 2, w, pos, val)) < 1e-12
+
+
+@pytest.mark.parametrize("n,w,npts,sort", [
+    (1024, 2, 1 << 20, False), (1024, 3, 1 << 20, False), (128, 2, 1 << 16, True), (128, 3, (1 << 16) - 1, False),
+    (1024, 4, 1 << 15, True), (1024, 4, (1 << 15) - 1, False), (65536, 6, 1 << 18, True), (1 << 20, 4, 1 << 20, False)])
+def test_1d_sorted_line(afc, cuda, n, w, npts, sort):
+    # which spreads sort first: three more launches (bins, offsets, indices)
+    from apollofft_b200.nufft import NufftPlan1D
+    plan = NufftPlan1D(n, 1.0, 2, w)
+    g = torch.Generator(device="cuda").manual_seed(n)
+    pos = torch.rand(npts, dtype=torch.float64, device="cuda", generator=g) * n
+    val = torch.randn(npts, dtype=torch.complex128, device="cuda", generator=g)
+
+    def launches(k):
+        before = afc.kernel_launch_count()
+        plan.type1(pos[:k], val[:k])
+        return afc.kernel_launch_count() - before
+
+    plan.type1(pos, val)
+    assert launches(npts) - launches(1) == (3 if sort else 0)
 
 
 def test_1d_first_call_captured(afc, cuda):
