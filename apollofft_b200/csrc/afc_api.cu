@@ -3319,7 +3319,7 @@ afc_status afc_nufft3d_type2(afc_nufft3d_plan plan, const void* modes, const dou
   const bool cap = stream_capturing(st);
   AFC_CUDA(plan->fence.before(st, cap), "NUFFT ordering");
   const NuLaunch3 L = nu_launch3(*plan);
-  const bool boxes = nufft3_boxes(L);
+  const bool boxes = nufft3_boxes_interp(L, npts);
   bool tiled = false;
   afc_status s = nu3_reserve(*plan, npts, boxes, true, cap, &tiled);
   if (s != AFC_OK) return s;

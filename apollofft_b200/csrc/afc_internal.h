@@ -248,6 +248,7 @@ struct NuTileLaunch {
 // Points the box kernels take at a time (bounds their record and slot buffers).
 constexpr long long kNu3Slice = 1 << 18;
 bool nufft3_boxes(const NuLaunch3& L);
+bool nufft3_boxes_interp(const NuLaunch3& L, long long npts);
 size_t nufft3_box_smem(int w, bool spread);
 size_t nufft3_slot_bytes(int w);
 size_t nufft3_rec_bytes(int w);

@@ -1243,6 +1243,16 @@ bool nufft3_boxes(const NuLaunch3& L) {
   return lo >= 16 && lo >= T + 8 && hi < (1 << 20) && (2 + 2 * wt) * (1 + 2 * wt) * 2 <= kNuBoxRuns &&
          nufft3_box_smem(L.w, false) <= 112 * 1024;
 }
+// Interpolation with few taps costs the tile kernel less than the boxes' records
+// and sums: from a point per 32 cells on, w <= 3 takes the tiles.  Measured at
+// uniform / crowded points, us tiles -> boxes: w = 2, 2^20 points on 128^3 cells
+// 491 / 3818 -> 2310 / 6525, w = 3, 2^17 on 64^3 182 / 1599 -> 366 / 507 (a tile is
+// one CTA, so crowded points on a small grid would prefer boxes); w = 2, 2^15
+// on 256^3 767 / 571 -> 537 / 739; w = 4, 2^17 on 128^3 325 / 1249 -> 408 / 1088, w = 6
+// 518 / 2353 -> 489 / 1347: boxes.
+bool nufft3_boxes_interp(const NuLaunch3& L, long long npts) {
+  return nufft3_boxes(L) && (L.w > 3 || 32 * npts < L.mx * L.my * L.mz);
+}
 size_t nufft3_box_smem(int w, bool spread) {
   return ((size_t)2 * kNuBoxChunk * nu_rec(2 * w + 1) + kNuZeros) * sizeof(double) +
          (size_t)(kNuBoxThreads / 32) * nu_list() * sizeof(int) +

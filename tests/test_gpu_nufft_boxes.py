@@ -62,6 +62,25 @@ def test_3d_slices(afc, oracle, cuda, shape, w):
     assert rel_l2(y2, c_type2_3d(shape, dx, 2, w, modes, pos)) < 1e-12
 
 
+@pytest.mark.parametrize("shape,w,npts,boxes", [((16, 16, 16), 2, 1024, False), ((16, 16, 16), 2, 1023, True),
+                                                ((16, 20, 16), 3, 3000, False), ((16, 16, 16), 4, 3000, True)])
+def test_3d_interpolation_line(afc, cuda, shape, w, npts, boxes):
+    # boxes take two launches more than tiles (records, sums)
+    from apollofft_b200.nufft import NufftPlan3D
+    rng = np.random.default_rng(w)
+    dx = (1.0, 1.0, 1.0)
+    pos = np.ascontiguousarray(rng.uniform(0, 1, (npts, 3)) * np.array(shape))
+    modes = rng.standard_normal(shape) + 1j * rng.standard_normal(shape)
+    plan = NufftPlan3D(shape, dx, 2, w)
+    m_t, p_t = torch.from_numpy(modes).cuda(), torch.from_numpy(pos).cuda()
+    plan.type2(m_t, p_t)
+    before = afc.kernel_launch_count()
+    y = plan.type2(m_t, p_t).cpu().numpy()
+    # placement and three axis passes, bins, offsets, indices, interpolation
+    assert afc.kernel_launch_count() - before == (10 if boxes else 8)
+    assert rel_l2(y, c_type2_3d(shape, dx, 2, w, modes, pos)) < 1e-12
+
+
 @pytest.mark.parametrize("n,w,npts", [(1, 2, 5), (3, 6, 40), (64, 4, 1000), (257, 6, 3001), (1000, 8, 500), (50, 13, 64),
                                       (40, 20, 64)])
 def test_1d_widths(afc, oracle, cuda, n, w, npts):
