@@ -2115,11 +2115,17 @@ static void tune_group(BatchGroup& g, bool dbl, void* scratch, cudaStream_t st) 
 }
 
 // The tile list of the compile-time batch kernel.  Transforms of several passes
-// come first, largest first, pass k of a transform about k kLag tiles after its
+// come first, largest first, pass k of a transform about k lag tiles after its
 // first one: far enough that the tiles in flight rarely wait, close enough that
 // the intermediates stay in L2.  Single-tile transforms fill the drain.
 struct FxAcc {
-  static constexpr double kLag = 1800;  // three tiles for each CTA in flight (600 / 1800 / 4000: 1345 / 1287 / 1288 us)
+  // Three tiles for each CTA in flight (148 SMs, four complex64 or two complex128
+  // CTAs each).  Lags of 300 / 900 / 1800 / 3600 tiles, us: 4096 transforms of 64 ..
+  // 65536 points complex64 1682 / 1080 / 1073 / 1076, complex128 2504 / 2219 / 2243 /
+  // 2248; 1024 of 8192 .. 65536 points 1241 / 799 / 787 / 793 and 1653 / 1447 / 1469 /
+  // 1473; batches of at most 512 do not care past 900.
+  const double lag;
+  explicit FxAcc(bool dbl) : lag(3.0 * 148 * (dbl ? 2 : 4)) {}
   struct Multi {
     long long tiles;  // all passes of one transform
     std::vector<FxBatchItem> items;
@@ -2178,10 +2184,10 @@ struct FxAcc {
     std::vector<std::pair<double, FxBatchItem>> all;
     double at = 0;
     for (const auto& m : multi) {
-      for (size_t j = 0; j < m.items.size(); ++j) all.emplace_back(at + m.pass[j] * kLag, m.items[j]);
+      for (size_t j = 0; j < m.items.size(); ++j) all.emplace_back(at + m.pass[j] * lag, m.items[j]);
       at += (double)m.tiles;
     }
-    const double span = multi.empty() ? 1.0 : 2 * kLag;
+    const double span = multi.empty() ? 1.0 : 2 * lag;
     for (size_t j = 0; j < single.size(); ++j)
       all.emplace_back(at + span * (double)j / (double)single.size(), single[j].second);
     std::stable_sort(all.begin(), all.end(), [](auto& a, auto& b) { return a.first < b.first; });
@@ -2213,7 +2219,7 @@ static afc_status build_phases(afc_batch_plan_s& bp, bool inv, cudaStream_t st) 
     size_t smem = 0;
   };
   std::vector<PhaseAcc> acc;
-  FxAcc fxa;
+  FxAcc fxa(bp.dbl);
   for (auto& g : bp.groups) {
     Recorder rec;
     rec.fx = true;
