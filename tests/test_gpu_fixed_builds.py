@@ -1,20 +1,17 @@
-"""The fixed-address axis builds (every shared-memory offset a compile-time
-constant) against the general build and the oracle: 256 points as radix
-16 x 16 for contiguous lanes (1D batches, the last axis of a 3D volume) and
-strided lanes (the middle and first axes), alone and inside the pass pair, and
-4096 points as radix 16 x 16 x 16 on contiguous lanes, and the compile-time
-stage lists of the smooth odd lengths 343 = 7 7 7, 243 = 9 9 3 and
-250 = 10 5 5 on contiguous and strided lanes; forward and inverse with 1/N, in
-and out of place.
+"""The compile-time builds of the axis kernels (every shared-memory offset a
+constant) against the general kernels and the oracle: 256 and 4096 points, 2048
+points, and the odd lengths 343 = 7 7 7, 243 = 9 9 3 and 250 = 10 5 5, on
+contiguous lanes (1D batches, the last axis of a volume) and strided lanes (the
+other axes); forward and inverse with 1/N, in and out of place, and beside the
+pass pair.
 
-AFC_TMA_N256 / AFC_TMA_N4096 (read by the library at every plan): 0 general
-build, 1 the fixed build for complex64, 2 for complex128 as well (N256 default
-1, N4096 default 2).  AFC_TMA_FIXED: 0 general build, 1 the stage lists
-(default).  Results against the
-oracle's FftPlan1D/3D (crates/apollo-fft/src/application/execution/plan/fft/
-dimension_{1,3}d.rs) at f64 <= 1e-12 and f32 <= 1e-5; both builds compute the
-same butterflies with the same twiddles in the same order, so their outputs
-agree bit for bit.
+AFC_FX=0 when a plan is made keeps the general kernels, so the plans here are
+not the cached ones.  Lengths and strides that have no compile-time build
+(4096-point columns, complex128 columns of 2048 points) run the general kernel on
+both sides.  Results against the oracle's FftPlan1D/3D
+(crates/apollo-fft/src/application/execution/plan/fft/dimension_{1,3}d.rs) at
+f64 <= 1e-12 and f32 <= 1e-5; both kernels compute the same stages, so their
+outputs differ by rounding only.
 """
 import numpy as np
 import pytest
@@ -33,11 +30,8 @@ def cplx(rng, shape):
 
 
 def run(afc, cuda, monkeypatch, mode, shape, prec, x, inverse=False, batch=1):
-    monkeypatch.setenv("AFC_TMA_N256", str(mode))
-    monkeypatch.setenv("AFC_TMA_N4096", str(mode))
-    monkeypatch.setenv("AFC_TMA_FIXED", "1" if mode else "0")
-    monkeypatch.setenv("AFC_TMA_L4", "1" if mode else "0")
-    p = afc.CudaPlan(list(shape), precision=prec, batch=batch)
+    monkeypatch.setenv("AFC_FX", str(mode))
+    p = afc.CudaPlan(list(shape), precision=prec, batch=batch, cached=False)
     return p.execute(torch.from_numpy(x).to(cuda, DT[prec]), inverse=inverse).cpu().numpy()
 
 
@@ -59,11 +53,11 @@ def test_fixed_build_matches_oracle_and_general(afc, oracle, cuda, monkeypatch, 
         ref = np.stack([oracle.fft3d(v) for v in x3])
         ref_inv = np.stack([oracle.fft3d(v, inverse=True) for v in x3])
     ref, ref_inv = ref.reshape(full), ref_inv.reshape(full)
-    fixed = run(afc, cuda, monkeypatch, 2, shape, prec, x, batch=batch)
+    fixed = run(afc, cuda, monkeypatch, 1, shape, prec, x, batch=batch)
     general = run(afc, cuda, monkeypatch, 0, shape, prec, x, batch=batch)
     assert rel_l2(fixed, ref) < TOL[prec]
     assert rel_l2(fixed, general) < SAME[prec]
-    fixed_i = run(afc, cuda, monkeypatch, 2, shape, prec, x, inverse=True, batch=batch)
+    fixed_i = run(afc, cuda, monkeypatch, 1, shape, prec, x, inverse=True, batch=batch)
     assert rel_l2(fixed_i, ref_inv) < TOL[prec]
     assert rel_l2(fixed_i, run(afc, cuda, monkeypatch, 0, shape, prec, x, inverse=True, batch=batch)) < SAME[prec]
 
@@ -74,7 +68,6 @@ def test_fixed_build_in_place_and_in_the_pair(afc, oracle, cuda, monkeypatch, pr
     shape = (5, 256, 256)
     x = cplx(rng, shape)
     ref = oracle.fft3d(x)
-    monkeypatch.setenv("AFC_TMA_N256", "2")
     p = afc.CudaPlan(list(shape), precision=prec)
     t = torch.from_numpy(x).to(cuda, DT[prec])
     p.execute(t, out=t)
@@ -92,9 +85,8 @@ def test_fixed_build_in_place_and_in_the_pair(afc, oracle, cuda, monkeypatch, pr
 @pytest.mark.parametrize("kind", ["r2c_full", "r2c_half"])
 @pytest.mark.parametrize("shape,batch", [((2048,), 6), ((2, 2048), 3), ((2048, 2048), 1)])
 def test_fixed_real_lanes_2048(afc, cuda, monkeypatch, kind, shape, batch):
-    """Real input rows widened in the first stage and real parts stored by the
-    last stage of the in-place 2048-point build, against numpy (f32 <= 1e-5)
-    and against the general build."""
+    """Real input rows widened on load and real parts stored by the 2048-point
+    build, against numpy (f32 <= 1e-5) and against the general kernels."""
     rng = np.random.default_rng(2048 + batch)
     x = rng.standard_normal((batch,) + shape).astype(np.float32)
     axes = tuple(range(1, len(shape) + 1))
@@ -103,9 +95,8 @@ def test_fixed_real_lanes_2048(afc, cuda, monkeypatch, kind, shape, batch):
         ref = np.fft.rfftn(x.astype(np.float64), axes=axes)
     outs = {}
     for mode in ("0", "1"):
-        monkeypatch.setenv("AFC_TMA_FIXED", mode)
-        monkeypatch.setenv("AFC_TMA_L4", mode)
-        p = afc.CudaPlan(list(shape), precision="f32", kind=kind, batch=batch)
+        monkeypatch.setenv("AFC_FX", mode)
+        p = afc.CudaPlan(list(shape), precision="f32", kind=kind, batch=batch, cached=False)
         y = p.execute(torch.from_numpy(x).to(cuda))
         back = p.execute(y, inverse=True)
         outs[mode] = (y.cpu().numpy().reshape(ref.shape), back.cpu().numpy().reshape(x.shape))
