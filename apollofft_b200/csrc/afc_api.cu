@@ -311,8 +311,8 @@ static int env_int(const char* name, int dflt) {
 struct LenPlan {
   StageList sl{};
   void* tw = nullptr;
-  // stage twiddles of the compile-time engine (powers of two 64 .. 4096;
-  // AFC_FX=0 at plan creation keeps the general engine), behind tw's entries in
+  // stage twiddles of the compile-time engine (powers of two 64 .. 4096, 243, 250
+  // and 343; AFC_FX=0 at plan creation keeps the general engine), behind tw's entries in
   // the same allocation; null when the length has no compile-time build
   void* fx_tw = nullptr;
   int P = 0, ld = 0;
@@ -769,8 +769,9 @@ static cudaError_t exec_axis(const AxisPlan& ap, bool dbl, bool inv, const AxisI
       // 1024 and 256 points complex64 119 and 52 against 81 and 49 us,
       // complex128 165 and 98 against 126 and 87 us.  The TMA tile spends a
       // barrier and a shared-memory round trip on each side of the stages and
-      // keeps one tile per CTA in flight; here a dozen CTAs per SM load, compute
-      // and store independently.
+      // keeps one tile per CTA in flight; here two to eight CTAs per SM (complex64
+      // rows 8, complex128 rows and convolutions 4 to 6, columns 2 or 3) load,
+      // compute and store independently.
       if ((!tl_rec || tl_rec->fx) && ap.lp.fx_tw) {
         LaunchDesc f = d;
         if (io.im.es == 1 && io.om.es == 1) {
@@ -1056,7 +1057,8 @@ static int plan_stages_uncached(int64_t m, size_t csz) {
   return best;
 }
 
-// Whether a Bluestein convolution of M points runs on the compile-time engine.
+// Whether a Bluestein convolution of M points runs on the compile-time engine:
+// both factors of its two passes within the 1024-point columns.
 static bool fx_conv_length(int64_t M) {
   return env_int("AFC_FX", 1) != 0 && (M & (M - 1)) == 0 && M >= 64 && M <= (1 << 20);
 }
@@ -1068,10 +1070,13 @@ static int64_t conv_length(int64_t need, size_t csz, bool bluestein) {
   int64_t p2 = 1;
   while (p2 < need) p2 <<= 1;
   // Bluestein convolutions of 64 .. 2^20 points run on the compile-time engine
-  // at powers of two, three to four times as fast per point as a 7-smooth length
-  // on the general one (complex64, 2^22 convolution points: 50 against 183 us
-  // in one tile, 78 against 280 us in three passes), so a smooth length at
-  // least half as long never pays
+  // at powers of two, two to four times as fast per point as a 7-smooth length on
+  // the general one, so a smooth length at least half as long never paid.  2^22
+  // points in all, us engine / general, complex64 and complex128: 1031 points
+  // (4096 against 2100) 75 / 237 and 169 / 356, 2053 (8192 in three passes against
+  // 4116 in one tile, the closest) 193 / 252 and 323 / 366, 4099 (16384 against
+  // 8232) 179 / 213 and 299 / 612, 40009 166 / 458 and 292 / 762.  Past 2^20 the engine
+  // has no build: 524287 points take 130 us (8 lanes), 524309 511 (7 lanes).
   if (bluestein && fx_conv_length(p2)) return p2;
   int64_t best = p2;
   static const int mode = env_int("AFC_CONV_LEN", 0);  // 0 cost model, 1 powers of two only

@@ -11,8 +11,10 @@ namespace afc {
 // CTAs per SM a kernel is built for.  16 points are 32 (complex64) or 64
 // (complex128) registers; 1024 threads leave 64 registers, 768 80, 512 128.
 // Complex64 rows fit 64 without spills (16384 x 4096 both ways 391 -> 369 us);
-// the columns' strides and the convolution's second network do not (8 x 2^20
-// 151 -> 164 us) and keep 80.  The odd lengths hold at most 10 points.
+// the strides of columns of up to 512 points and the convolution's second network
+// do not (8 x 2^20 151 -> 164 us) and keep 80.  Columns of 1024 and 2048 points run
+// 512 threads, two CTAs of 64 registers and 16 to 24 bytes of spills (one CTA of
+// 128: 8 x 2^20 183 us against 148).  The odd lengths hold at most 10 points.
 template <class T, int N, int FORM, int MODE> constexpr int fx_min_ctas(int threads) {
   if (!fx_pow2(N)) return (sizeof(T) == 4 ? 1024 : 512) / ((threads + 31) / 32 * 32);
   if (threads > 256) return sizeof(T) == 4 ? 2 : 1;
@@ -43,7 +45,9 @@ template <class T, int N, int FORM, int MODE, int IN, int OUT, bool HALF> static
 }
 
 // Lane-minor forms stop at 1024 points: rows of 64 bytes at 2048 would need a
-// CTA of 1024 threads (64 registers each).
+// CTA of 1024 threads (64 registers each).  Plain complex64 columns of 2048 points
+// have a build with rows of 32 bytes (the 2048^2 images: 128 us a pass against 150 on
+// the TMA kernel).
 template <class T, int FORM, int MODE, int IN, int OUT, bool HALF = false> static FxEntry fx_by_length(long long n) {
   switch (n) {
     case 64: return fx_entry<T, 64, FORM, MODE, IN, OUT, HALF>();

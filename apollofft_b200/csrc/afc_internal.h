@@ -202,7 +202,7 @@ cudaError_t launch_tc_fft(const TcLaunch& d, bool fp16, cudaStream_t st);
 // 1D NUFFT spreading / interpolation (afc_nufft.cu), complex128 grids
 // Coefficients of phi in s = w^2 - x^2 (K = 0: none, the series is evaluated).
 struct NuPoly {
-  static constexpr int max = 80;  // terms for w <= 12 at sigma = 2
+  static constexpr int max = 80;  // terms for w <= 15 at sigma = 2
   int K = 0;
   double c[max] = {};
 };

@@ -58,9 +58,10 @@ __device__ __forceinline__ double nu_kb(double x, double w, double beta, double 
 // phi as a polynomial: I0's series in (z/2)^2 = (beta / 2w)^2 s, s = w^2 - x^2,
 // divided by I0(beta), has the fixed positive coefficients NuPoly::c, so Horner
 // needs one FMA per term instead of the running product's three operations, no
-// division and no square root; s = (w - x)(w + x) does not cancel at the edge.  The first dropped term is below 2^-60 of phi(0) = 1.  Measured
-// on B200 at w = 6 (46 terms): the weights were about half of a 1D call.  K = 0
-// (kernels too wide for the table): the series.
+// division and no square root; s = (w - x)(w + x) does not cancel at the edge.  The
+// first dropped term is below 2^-60 of phi(0) = 1.  At w = 6 (44 terms) the series'
+// weights were about half of a 1D call.  K = 0 (kernels too wide for the table): the
+// series.
 __device__ __forceinline__ double nu_phi(const NuPoly& f, double x, double w, double beta, double i0b) {
   if (f.K == 0) return nu_kb(x, w, beta, i0b);
   const double s = (w - x) * (w + x);
@@ -665,7 +666,13 @@ __global__ void __launch_bounds__(kNuTileThreads) nu3_spread_tiles(const __grid_
 //                  time, for each y and for both parts of v;
 //   interpolation  D[point][z] = sum_x wx[point][x] cell[x][z], 8 points at a
 //                  time, then summed over y and z with their weights.
-// One operand element per lane feeds 8 FMAs.
+// One operand element per lane feeds 8 FMAs.  Measured at 2^18 uniform points on
+// 128^3 cells, w = 6 (kernel alone): spreading by tiles 1650 us, by boxes with scalar
+// FMAs, bound by the broadcast weight loads, 1095, by these 612; interpolation by
+// tiles 784 us, by boxes 713 and 23 for the sums, bound by the shared-memory loads
+// ahead of each group (the FP64 pipe is 6-8 % busy).  Tiles are one CTA each, so for
+// crowded points the boxes are up to 40 times as fast at spreading and 14 at
+// interpolation (16^3 modes, w = 6, 2^17 points).
 //  nu3_points: one record per point in tile order: value, centre, index, and the
 //              axis weights between runs of seven zeros, so no tap is range-checked;
 //  nu3_boxes:  a CTA of 8 warps owns 16 x 8 x 16 cells and streams the records of
@@ -1296,7 +1303,11 @@ cudaError_t nufft3_boxes_dev(const NuLaunch3& L, const NuTileLaunch& TL, bool sp
     points<<<(unsigned)((n + kNuPts - 1) / kNuPts), 3 * kNuPts, 0, st>>>(
         g, TL.idx, ps, spread ? static_cast<const double2*>(val) + p0 : nullptr, (int)n, TL.rec);
     // a box's chunks are dealt to `split` CTAs: about 4096 CTAs in all, so a
-    // grid of few boxes, or points crowded into some of them, still fills the chip
+    // grid of few boxes, or points crowded into some of them, still fills the chip.
+    // Type 1 at w = 6, us with 1 / 2 / 4 / 8 / 32 CTAs a box: 2^18 points on 64^3 modes
+    // (1024 boxes) uniform 716 / 705 / 728 / 789 / 1189, crowded about the middle 15388 /
+    // 8781 / 5017 / 2910 / 1273; 2^15 on 32^3 (128 boxes) 199 / 154 / 154 / 145 / 191 and
+    // 2031 / 1129 / 639 / 422 / 202; 2^18 on 16^3 (16 boxes) 8863 / 4564 / 2367 / 1269 / 874
     const long long chunks = (n + kNuBoxChunk - 1) / kNuBoxChunk;
     const int split = (int)std::max<long long>(1, std::min<long long>(chunks, std::min(32, 4096 / boxes)));
     k<<<dim3((unsigned)boxes, (unsigned)split), kNuBoxThreads, smem, st>>>(

@@ -19,8 +19,8 @@ CASES = [((4, 4, 4), (0.1, 0.1, 0.1), 2, 6, 3),
          ((8, 6, 5), (0.25, 0.5, 0.2), 2, 6, 150),
          ((16, 12, 10), (1.0, 0.1, 0.3), 2, 4, 300),
          ((3, 2, 2), (0.5, 0.75, 1.0), 3, 6, 40),
-         ((16, 16, 16), (0.0625, 0.0625, 0.0625), 2, 6, 2000),   # shared-memory tiles, B = 8
-         ((6, 5, 4), (1.0, 1.0, 1.0), 2, 8, 60),                 # B = 4 tiles
+         ((16, 16, 16), (0.0625, 0.0625, 0.0625), 2, 6, 2000),   # boxes, as most grids
+         ((6, 5, 4), (1.0, 1.0, 1.0), 2, 8, 60),                 # 32 cells a side: boxes at w = 8 too
          ((4, 4, 4), (1.0, 1.0, 1.0), 2, 10, 30)]                # too wide for a tile: per-point kernels
 
 
