@@ -1391,7 +1391,7 @@ struct afc_nufft_plan_s {
 // 3D NUFFT plan (apollo-nufft NufftPlan3D, transform/dimension_3d.rs:193-230):
 // per axis m = next_pow2(max(sigma n, 2w + 1)), one C2C f64 plan of
 // (mx, my, mz) over the plan-owned grid, deconvolution factors per axis.
-// A buffer of a 3D NUFFT plan with so much per point.
+// The per-point buffer of a 3D NUFFT plan.
 struct NuPointBuf {
   void* p = nullptr;
   int64_t cap = 0;        // points it holds
@@ -1409,7 +1409,7 @@ struct afc_nufft3d_plan_s {
   double* deconv = nullptr;  // nx + ny + nz factors, axis after axis
   void* grid = nullptr;      // mx my mz complex128, C order
   afc::NuTileLaunch tiles;   // B = 0: per-point kernels
-  NuPointBuf buckets, records, slots;
+  NuPointBuf points;
   std::vector<void*> retired;  // outgrown buffers that captured graphs still use
   std::mutex mu;             // one caller enqueues on the grid at a time
   afc::Fence fence;          // the grid's (and tile buffers') last use on the GPU
@@ -2416,8 +2416,7 @@ afc_nufft_plan_s::~afc_nufft_plan_s() {
 afc_nufft3d_plan_s::~afc_nufft3d_plan_s() {
   for (int* b : {tiles.cnt, tiles.off})
     if (b) cudaFree(b);
-  for (void* b : {buckets.p, records.p, slots.p})
-    if (b) cudaFree(b);
+  if (points.p) cudaFree(points.p);
   for (void* b : retired) cudaFree(b);
   if (fft) afc_plan_destroy(fft);
   if (deconv) cudaFree(deconv);
@@ -3221,49 +3220,35 @@ afc_status afc_nufft3d_plan_create(afc_nufft3d_plan* out, int64_t nx, int64_t ny
   return AFC_OK;
 }
 
-// Makes b hold npts points.  A buffer whose address a captured graph has lives
-// as long as the plan; it is outgrown by twice its size, so the buffers set aside
-// add up to less than the one in use.
-static afc_status nu3_grow(afc_nufft3d_plan_s& p, NuPointBuf& b, int64_t npts, int64_t most, size_t per_point,
-                           const char* what) {
-  if (npts <= b.cap) return AFC_OK;
-  NuPointBuf nb;
-  nb.cap = b.captured ? std::min(most, std::max(npts, 2 * b.cap)) : npts;
-  if (b.captured) p.retired.push_back(b.p);
-  else if (b.p) cudaFree(b.p);
-  b = NuPointBuf{};
-  AFC_CUDA(dev_alloc(&nb.p, (size_t)nb.cap * per_point), what);
-  b = nb;
-  return AFC_OK;
-}
-// The per-point buffers of a call, grown (synchronous allocation) when it brings
-// more points than any call before it.  *tiled false: the per-point kernels run,
-// which need none -- a captured call cannot allocate.
-static afc_status nu3_reserve(afc_nufft3d_plan_s& p, int64_t npts, bool boxes, bool interp, bool cap, bool* tiled) {
-  struct Need {
-    NuPointBuf* b;
-    int64_t n, most;
-    size_t per_point;
-    const char* what;
-  } need[3] = {{&p.buckets, npts, INT32_MAX, 3 * sizeof(int), "NUFFT point buckets"},
-               {&p.records, std::min<int64_t>(npts, kNu3Slice), kNu3Slice, nufft3_rec_bytes(p.w), "NUFFT point records"},
-               {&p.slots, std::min<int64_t>(npts, kNu3Slice), kNu3Slice, nufft3_slot_bytes(p.w), "NUFFT point sums"}};
-  const int cnt = !boxes ? 1 : interp ? 3 : 2;
-  *tiled = p.tiles.B != 0 && npts > 0 && npts <= INT32_MAX;
-  for (int i = 0; i < cnt; ++i)
-    if (cap && need[i].n > need[i].b->cap) *tiled = false;
+// The per-point buffer of a call: tile, rank and index of every point and, for
+// the box kernels, record and slots of every point of a slice, in one allocation
+// (a first call pays about 300 us for each).  It grows when a call brings more
+// points than any call before it.  One whose address a captured graph has lives as
+// long as the plan and is outgrown by twice its size, so the buffers set aside add
+// up to less than the one in use.  *tiled false: the per-point kernels run, which
+// need none -- a captured call cannot allocate.
+static afc_status nu3_reserve(afc_nufft3d_plan_s& p, int64_t npts, bool boxes, bool cap, bool* tiled) {
+  NuPointBuf& b = p.points;
+  *tiled = p.tiles.B != 0 && npts > 0 && npts <= INT32_MAX && !(cap && npts > b.cap);
   if (!*tiled) return AFC_OK;
-  for (int i = 0; i < cnt; ++i) {
-    const Need& d = need[i];
-    afc_status s = nu3_grow(p, *d.b, d.n, d.most, d.per_point, d.what);
-    if (s != AFC_OK) return s;
-    if (cap) d.b->captured = true;
+  if (npts > b.cap) {
+    const int64_t n = b.captured ? std::min<int64_t>(INT32_MAX, std::max(npts, 2 * b.cap)) : npts;
+    const size_t slice = (size_t)std::min<int64_t>(n, kNu3Slice);
+    const size_t lists = ((size_t)n * 3 * sizeof(int) + 255) / 256 * 256;
+    const size_t recs = boxes ? (slice * nufft3_rec_bytes(p.w) + 255) / 256 * 256 : 0;
+    const size_t slots = boxes ? slice * nufft3_slot_bytes(p.w) : 0;
+    if (b.captured) p.retired.push_back(b.p);
+    else if (b.p) cudaFree(b.p);
+    b = NuPointBuf{};
+    AFC_CUDA(dev_alloc(&b.p, lists + recs + slots), "NUFFT point buffer");
+    b.cap = n;
+    p.tiles.tile = static_cast<int*>(b.p);
+    p.tiles.rank = p.tiles.tile + n;
+    p.tiles.idx = p.tiles.rank + n;
+    p.tiles.rec = reinterpret_cast<double*>(static_cast<char*>(b.p) + lists);
+    p.tiles.slots = reinterpret_cast<double2*>(static_cast<char*>(b.p) + lists + recs);
   }
-  p.tiles.tile = static_cast<int*>(p.buckets.p);
-  p.tiles.rank = p.tiles.tile + p.buckets.cap;
-  p.tiles.idx = p.tiles.rank + p.buckets.cap;
-  p.tiles.rec = static_cast<double*>(p.records.p);
-  p.tiles.slots = static_cast<double2*>(p.slots.p);
+  if (cap) b.captured = true;
   return AFC_OK;
 }
 
@@ -3301,7 +3286,7 @@ afc_status afc_nufft3d_type1(afc_nufft3d_plan plan, const double* positions, con
   const NuLaunch3 L = nu_launch3(*plan);
   const bool boxes = nufft3_boxes(L);
   bool tiled = false;
-  afc_status r = nu3_reserve(*plan, npts, boxes, false, cap, &tiled);
+  afc_status r = nu3_reserve(*plan, npts, boxes, cap, &tiled);
   if (r != AFC_OK) return r;
   AFC_CUDA(cudaMemsetAsync(plan->grid, 0, (size_t)(L.mx * L.my * L.mz) * 16, st), "NUFFT grid");
   if (tiled && boxes)
@@ -3332,7 +3317,7 @@ afc_status afc_nufft3d_type2(afc_nufft3d_plan plan, const void* modes, const dou
   const NuLaunch3 L = nu_launch3(*plan);
   const bool boxes = nufft3_boxes_interp(L, npts);
   bool tiled = false;
-  afc_status s = nu3_reserve(*plan, npts, boxes, true, cap, &tiled);
+  afc_status s = nu3_reserve(*plan, npts, nufft3_boxes(L), cap, &tiled);
   if (s != AFC_OK) return s;
   AFC_CUDA(cudaMemsetAsync(plan->grid, 0, (size_t)(L.mx * L.my * L.mz) * 16, st), "NUFFT grid");
   const double* dc = plan->deconv;

@@ -317,10 +317,10 @@ AFC_API afc_status afc_nufft_plan_destroy(afc_nufft_plan plan);
  * out[j] ~ sum_k modes_k exp(+2 pi i (...)) / (mx my mz).  Spreading uses
  * atomic adds instead of the reference's bucket sort (rounding differs only).
  * One grid per plan: overlapping calls on different streams are ordered on
- * the GPU by events, which calls captured into a graph skip.  Per-point buffers
- * grow, with a synchronous allocation, when a call brings more points than any
- * before it; a captured call that would have to grow them takes the per-point
- * kernels, and buffers a captured call used live as long as the plan.
+ * the GPU by events, which calls captured into a graph skip.  A per-point buffer
+ * grows, with a synchronous allocation, when a call brings more points than any
+ * before it; a captured call that would have to grow it takes the per-point
+ * kernels, and a buffer that a captured call used lives as long as the plan.
  * afc_nufft3d_grid_dims writes (mx, my, mz). */
 typedef struct afc_nufft3d_plan_s* afc_nufft3d_plan;
 AFC_API afc_status afc_nufft3d_plan_create(afc_nufft3d_plan* out, int64_t nx, int64_t ny, int64_t nz, double dx,
