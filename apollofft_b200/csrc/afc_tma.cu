@@ -101,17 +101,17 @@ template <class C> struct TView {
   }
 };
 
-// PAD: the power-of-two lists' padded views; the others are linear in r.  Forward
-// stages of the others run the inverse butterfly on values with real and imaginary
+// PAD: the power-of-two lists' padded views; the others are linear in r.
+// EXCH: forward stages run the inverse butterfly on values with real and imaginary
 // part exchanged (exchanging z is i conj(z), so both directions are one set of
-// instructions): written out, the forward code of the 7-smooth complex128 build
-// spilled 104 bytes (356 of reloads) at its 128 registers, the inverse none.
+// instructions).  The 7-smooth build does: written out, its complex128 forward code
+// spilled 104 bytes (356 of reloads) at 128 registers, the inverse none.
 // 2^23 points forward, us written out / exchanged: complex128 rows of 7 points 63 / 48,
 // 360 108 / 83, 1000 127 / 88, 2187 148 / 118, complex64 rows of 1000 60 / 56.
-template <int R, bool INV, bool PAD, class C, class S>
+template <int R, bool INV, bool PAD, bool EXCH, class C, class S>
 __device__ __forceinline__ void tma_stage(TView<C> src, TView<C> dst, int l, int n, const StageDesc& sd,
                                           const C* __restrict__ tw, int t, int P, S sc) {
-  constexpr bool SW = !INV && !PAD;
+  constexpr bool SW = !INV && EXCH;
   const int nb = n / R;
   for (int j = t; j < nb; j += P) {
     const int Ns = stage_stride(sd.Ns), d0 = stage_stride(PAD ? nb : nb * src.is);
@@ -353,7 +353,7 @@ __device__ __forceinline__ typename CT<T>::type* tma_stages(const TmaArgs<T>& a,
     const TView<C> dst = last ? olin : ((s & 1) ? cpad : wv);
     const C* twi = twb + sd.twoff;
     const T sc = last ? a.scale : (T)1;
-#define AFC_TM(R) tma_stage<R, INV, P2>(src, dst, l, n, sd, twi, t, P, sc)
+#define AFC_TM(R) tma_stage<R, INV, P2, S7>(src, dst, l, n, sd, twi, t, P, sc)
     if constexpr (P2) {
       switch (sd.R) {
         case 2: AFC_TM(2); break;
