@@ -2225,19 +2225,20 @@ static afc_status build_phases(afc_batch_plan_s& bp, bool inv, cudaStream_t st) 
   };
   std::vector<PhaseAcc> acc;
   FxAcc fxa(bp.dbl);
-  for (auto& g : bp.groups) {
-    Recorder rec;
-    rec.fx = true;
+  // a group's launches, on the compile-time engine where it serves them (fx)
+  auto record_group = [&](const BatchGroup& g, bool fx, Recorder& rec) {
+    rec.launches.clear();
+    rec.fx = fx;
     tl_rec = &rec;
     AxisIO io;
     io.in = tag_ptr(1, 0);
     io.out = tag_ptr(2, 0);
-    io.lanes = g->lanes;
-    io.im = LaneMap{1, 1, 0, 0, 1, 1, g->d_off};
+    io.lanes = g.lanes;
+    io.im = LaneMap{1, 1, 0, 0, 1, 1, g.d_off};
     io.om = io.im;
-    io.scale = inv ? 1.0 / (double)g->n : 1.0;
+    io.scale = inv ? 1.0 / (double)g.n : 1.0;
     cudaError_t e = cudaSuccess;
-    if (g->ap->algo == ALGO_NOOP) {
+    if (g.ap->algo == ALGO_NOOP) {
       LaunchDesc d;
       d.sl.n = 1;
       d.sl.nst = 0;
@@ -2252,23 +2253,40 @@ static afc_status build_phases(afc_batch_plan_s& bp, bool inv, cudaStream_t st) 
       d.L = (int)std::min<long long>(64, std::max(1LL, io.lanes));
       e = do_lanes(d, bp.dbl, inv, st);
     } else {
-      e = exec_axis(*g->ap, bp.dbl, inv, io, tag_ptr(3, g->ws_off), st);
+      e = exec_axis(*g.ap, bp.dbl, inv, io, tag_ptr(3, g.ws_off), st);
     }
+    tl_rec = nullptr;
+    return e;
+  };
+  auto on_engine = [](const RecLaunch& r) { return r.d.fx_form >= 0; };
+  // Short batches run in the phases alone: with a general length among them, rows of
+  // at most 1024 points in a launch of their own cost it about 9 us and save less up to
+  // 2^20 points (4096 would not: the phases' tiles of one CTA each take longer).  us with
+  // both lists / phases alone, lengths 64 .. 1024: 8 transforms complex64 25 / 17, complex128
+  // 27 / 19, 600 of them 37 / 26 and 42 / 30, 2500 47 / 39 and 70 / 65, 5000 59 / 54 and 111 / 113;
+  // 32 of 64 .. 4096 points 54 / 71 and 68 / 72.
+  bool general = false, short_rows = true;
+  long long points = 0;
+  for (auto& g : bp.groups) {
+    Recorder rec;
+    cudaError_t e = record_group(*g, true, rec);
+    if (e != cudaSuccess) return cuda_fail(e, "batch record");
+    points += g->n * g->lanes;
+    if (!std::all_of(rec.launches.begin(), rec.launches.end(), on_engine)) general = true;
+    else if (rec.launches.size() != 1 || rec.launches[0].d.fx_mode == FX_CONV || g->n > 1024) short_rows = false;
+  }
+  const bool fx = !(general && short_rows && points <= (1 << 20));
+  for (auto& g : bp.groups) {
+    Recorder rec;
+    cudaError_t e = record_group(*g, fx, rec);
     // a group goes to the compile-time list only as a whole: its passes are
     // ordered there by its own counters
-    if (e == cudaSuccess && std::all_of(rec.launches.begin(), rec.launches.end(),
-                                        [](const RecLaunch& r) { return r.d.fx_form >= 0; })) {
-      tl_rec = nullptr;
+    if (e == cudaSuccess && std::all_of(rec.launches.begin(), rec.launches.end(), on_engine)) {
       fxa.add(rec.launches, g->off, bp.dbl);
       continue;
     }
-    if (e == cudaSuccess && std::any_of(rec.launches.begin(), rec.launches.end(),
-                                        [](const RecLaunch& r) { return r.d.fx_form >= 0; })) {
-      rec.launches.clear();
-      rec.fx = false;
-      e = exec_axis(*g->ap, bp.dbl, inv, io, tag_ptr(3, g->ws_off), st);
-    }
-    tl_rec = nullptr;
+    if (e == cudaSuccess && std::any_of(rec.launches.begin(), rec.launches.end(), on_engine))
+      e = record_group(*g, false, rec);
     if (e != cudaSuccess) return cuda_fail(e, "batch record");
     for (size_t k = 0; k < rec.launches.size(); ++k) {
       if (acc.size() <= k) acc.resize(k + 1);

@@ -77,3 +77,26 @@ def test_plan_creation_leaves_no_stale_error(afc, cuda):
         y = bp.execute(xt, mode=mode).cpu().numpy()
         for got, src in zip(lanes_of(y, lens), lanes_of(x, lens)):
             assert rel_l2(got, np.fft.fft(src.astype(np.complex128))) < 1e-5
+
+
+@pytest.mark.parametrize("prec", ["f32", "f64"])
+@pytest.mark.parametrize("lengths,launches", [
+    ([64, 128, 1024, 512], 1),                 # the compile-time engine alone
+    ([64, 100, 1024, 97, 1, 7], 1),            # short rows beside general lengths: the phases alone
+    ([64, 100, 2048, 97], 2), ([64, 2053, 100], 2),
+    ([1024] * 1024 + [100], 2),                # more than 2^20 points
+    ([1024] * 1023 + [100], 1)])
+def test_launches_of_short_batches(afc, cuda, prec, lengths, launches):
+    rng = np.random.default_rng(len(lengths))
+    cdt = np.complex64 if prec == "f32" else np.complex128
+    xs = [(rng.standard_normal(n) + 1j * rng.standard_normal(n)).astype(cdt) for n in lengths]
+    b = afc.BatchPlan(lengths, precision=prec)
+    t = torch.from_numpy(np.concatenate(xs)).to(cuda)
+    b.execute(t, mode=2)
+    before = afc.kernel_launch_count()
+    y = b.execute(t, mode=2)
+    assert afc.kernel_launch_count() - before == launches
+    back = b.execute(y, inverse=True, mode=2).cpu().numpy()
+    tol = 1e-5 if prec == "f32" else 1e-12
+    assert rel_l2(y.cpu().numpy(), np.concatenate([np.fft.fft(x) for x in xs])) < tol
+    assert rel_l2(back, np.concatenate(xs)) < tol
