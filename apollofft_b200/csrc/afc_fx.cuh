@@ -41,7 +41,7 @@ template <> struct FxRad<4096> { static constexpr int n = 3, r0 = 16, r1 = 16, r
 // Three odd lengths, plain rows and columns only: e points per thread, a multiple
 // of every radix.  They took the place of TMA builds for the same lengths; other
 // smooth lengths have none (complex64 volumes both ways, of the copy rate over six
-// passes: 243 x 250 x 343 0.61; 240 x 252 x 350 0.46, 225 x 240 x 245 0.34, 288^3 0.44).
+// passes: 243 x 250 x 343 0.61; 240 x 252 x 350 0.47, 225 x 240 x 245 0.34, 288^3 0.45).
 template <> struct FxRad<243> { static constexpr int n = 3, r0 = 9, r1 = 9, r2 = 3, e = 9; };
 template <> struct FxRad<250> { static constexpr int n = 3, r0 = 10, r1 = 5, r2 = 5, e = 10; };
 template <> struct FxRad<343> { static constexpr int n = 3, r0 = 7, r1 = 7, r2 = 7, e = 7; };
