@@ -1115,14 +1115,17 @@ static unsigned nu_grid(long long work) {
 //  * from 16 points a cell on, w = 4, n = 1024, 2^16 points 35 -> 51 / 136 -> 52;
 //  * below six taps a cell the windows hold a point or two: w = 4, n = 2^22, 2^22
 //    points 1112 -> 1116 / 1101 -> 1345: unsorted;
-//  * w <= 3, n = 1024, 2^20 points: w = 2 136 -> 357 / 917 -> 371, w = 3 286 -> 365:
-//    unsorted, but for the few cells whose atomics serialize (w = 2, n = 128, 2^18
-//    points 183 -> 116 / 562 -> 164).
+//  * w = 3 from 16 points a cell on only: n = 1024, 2^20 points 286 -> 365 / 1366 -> 388,
+//    n = 4096 139 -> 197 / 744 -> 307; n = 65536 (8 a cell) 122 -> 146 / 267 -> 206;
+//  * w = 2: n = 1024, 2^20 points 136 -> 357 / 917 -> 371: unsorted, but for the few
+//    cells whose atomics serialize (n = 128, 2^18 points 183 -> 116 / 562 -> 164).
 bool nufft_sorted(const NuLaunch& L, long long npts) {
   const long long T = 2 * L.w + 1;
   if (T > 25 || L.m < 64 || L.m >= (1ll << 31) - 64 || npts > INT32_MAX) return false;
-  if (T < 9) return L.m <= 256 && npts >= 256 * L.m;
-  return npts * T >= 6 * L.m && (npts * T >= (1 << 21) || (npts >= 16 * L.m && npts >= 4096));
+  const bool crowd = npts >= 16 * L.m && npts >= 4096;
+  if (T < 7) return L.m <= 256 && npts >= 256 * L.m;
+  if (T < 9) return crowd;
+  return crowd || (npts * T >= 6 * L.m && npts * T >= (1 << 21));
 }
 
 cudaError_t nufft_spread_dev(const NuLaunch& L, const NuTileLaunch& TL, const double* pos, const void* val,
@@ -1251,14 +1254,15 @@ bool nufft3_boxes(const NuLaunch3& L) {
          nufft3_box_smem(L.w, false) <= 112 * 1024;
 }
 // Interpolation with few taps costs the tile kernel less than the boxes' records
-// and sums: from a point per 32 cells on, w <= 3 takes the tiles.  Measured at
+// and sums: from a point per 32 cells on, w = 2 takes the tiles.  Measured at
 // uniform / crowded points, us tiles -> boxes: w = 2, 2^20 points on 128^3 cells
-// 491 / 3818 -> 2310 / 6525, w = 3, 2^17 on 64^3 182 / 1599 -> 366 / 507 (a tile is
-// one CTA, so crowded points on a small grid would prefer boxes); w = 2, 2^15
-// on 256^3 767 / 571 -> 537 / 739; w = 4, 2^17 on 128^3 325 / 1249 -> 408 / 1088, w = 6
-// 518 / 2353 -> 489 / 1347: boxes.
+// 491 / 3818 -> 2310 / 6525, 2^17 on 64^3 123 / 1019 -> 346 / 469 (a tile is one CTA, so
+// crowded points on a small grid would prefer boxes); 2^15 on 256^3 767 / 571 -> 537 /
+// 739: boxes.  Wider kernels gain less from tiles and lose more: w = 3, 2^17 on 64^3
+// 182 / 1599 -> 366 / 507, w = 4, 2^17 on 128^3 325 / 1249 -> 408 / 1088, w = 6 518 / 2353 ->
+// 489 / 1347: boxes.
 bool nufft3_boxes_interp(const NuLaunch3& L, long long npts) {
-  return nufft3_boxes(L) && (L.w > 3 || 32 * npts < L.mx * L.my * L.mz);
+  return nufft3_boxes(L) && (L.w > 2 || 32 * npts < L.mx * L.my * L.mz);
 }
 size_t nufft3_box_smem(int w, bool spread) {
   return ((size_t)2 * kNuBoxChunk * nu_rec(2 * w + 1) + kNuZeros) * sizeof(double) +

@@ -63,7 +63,7 @@ def test_3d_slices(afc, oracle, cuda, shape, w):
 
 
 @pytest.mark.parametrize("shape,w,npts,boxes", [((16, 16, 16), 2, 1024, False), ((16, 16, 16), 2, 1023, True),
-                                                ((16, 20, 16), 3, 3000, False), ((16, 16, 16), 4, 3000, True)])
+                                                ((16, 20, 16), 2, 9000, False), ((16, 16, 16), 3, 3000, True)])
 def test_3d_interpolation_line(afc, cuda, shape, w, npts, boxes):
     # boxes take two launches more than tiles (records, sums)
     from apollofft_b200.nufft import NufftPlan3D
@@ -117,7 +117,8 @@ def test_1d_sorted(afc, oracle, cuda, n, w, npts):
 
 
 @pytest.mark.parametrize("n,w,npts,sort", [
-    (1024, 2, 1 << 20, False), (1024, 3, 1 << 20, False), (128, 2, 1 << 16, True), (128, 3, (1 << 16) - 1, False),
+    (1024, 2, 1 << 20, False), (128, 2, 1 << 16, True), (128, 2, (1 << 16) - 1, False), (1024, 3, 1 << 15, True),
+    (65536, 3, 1 << 20, False),
     (1024, 4, 1 << 15, True), (1024, 4, (1 << 15) - 1, False), (65536, 6, 1 << 18, True), (1 << 20, 4, 1 << 20, False)])
 def test_1d_sorted_line(afc, cuda, n, w, npts, sort):
     # which spreads sort first: three more launches (bins, offsets, indices)
